@@ -35,7 +35,7 @@ EXPORTS = [
     "gmes_graph_destroy", "gmes_rasterize", "gmes_batch_step_noalloc",
     "gmes_tmz_sizes", "gmes_tmz_check", "gmes_tmz_set_design", "gmes_tmz_reset",
     "gmes_tmz_forward", "gmes_tmz_objective", "gmes_tmz_adjoint", "gmes_points_update",
-    "gmes_copy_async", "gmes_nonfinite",
+    "gmes_copy_async", "gmes_nonfinite", "gmes_step_launches",
 ]
 NOALLOC_MAX_GRIDS = 64
 
@@ -163,6 +163,7 @@ def load():
                                          P(C.c_double), C.c_void_p]
     lib.gmes_reset.argtypes = [P(GridDescC), C.c_void_p]
     lib.gmes_step.argtypes = [P(GridDescC), C.c_int32, C.c_void_p]
+    lib.gmes_step_launches.argtypes = [P(GridDescC), C.c_int32, P(C.c_int64)]
     lib.gmes_half_step.argtypes = [P(GridDescC), C.c_int32, C.c_int32, C.c_void_p]
     lib.gmes_read_field.argtypes = [P(GridDescC), C.c_int32, P(C.c_double), C.c_void_p]
     lib.gmes_write_field.argtypes = [P(GridDescC), C.c_int32, P(C.c_double), C.c_void_p]

@@ -213,7 +213,8 @@ class Batch:
                 N.check(self.lib.gmes_graph_launch(C.c_void_p(e._graph(s)), sst))
             else:
                 N.check(self.lib.gmes_step(C.byref(e.desc), s, sst))
-            launched += s * self._solo_launches_per_step(i)
+            launched += (e.step_launches(s) if hasattr(e, "step_launches")
+                         else s * self._solo_launches_per_step(i))
         for ss in side:
             self.stream.wait_stream(ss)
         return launched

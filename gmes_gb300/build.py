@@ -28,7 +28,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relax
 # that their one-step and temporally blocked forms round alike.
 EXTRA = {"gmes_coef.cu": ["--fmad=false"], "gmes_raster.cu": ["--fmad=false"],
          "gmes_adjoint.cu": ["--fmad=false"]}
-SOURCES = ["gmes_capi.cu", "gmes_coef.cu", "gmes_step.cu", "gmes_raster.cu", "gmes_adjoint.cu",
+SOURCES = ["gmes_capi.cu", "gmes_coef.cu", "gmes_step.cu", "gmes_persist.cu", "gmes_raster.cu", "gmes_adjoint.cu",
            "gmes_points.cu"]
 
 

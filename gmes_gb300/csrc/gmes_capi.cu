@@ -2,13 +2,16 @@
 // coefficient-block layout, host<->device staging and error reporting.
 // Status codes follow the reference binding's exception classes
 // (src/pw_material.i:23-33): ValueError, IndexError, RuntimeError.
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <deque>
 #include <functional>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "gmes_internal.cuh"
@@ -43,6 +46,32 @@ int elem_size(int32_t precision) {
     default:
       return 0;
   }
+}
+
+// The word that kernels set when a wait ran past its limit: pinned, allocated
+// once per process outside any stream capture (gmes_build_coefficients).
+std::atomic<int*> g_wait_error{nullptr};
+
+cudaError_t ensure_wait_error() {
+  static std::mutex m;
+  std::lock_guard<std::mutex> lock(m);
+  if (g_wait_error.load() != nullptr) return cudaSuccess;
+  void* p = nullptr;
+  const cudaError_t e =
+      cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+  if (e != cudaSuccess) return e;
+  *static_cast<int*>(p) = 0;
+  g_wait_error.store(static_cast<int*>(p));
+  return cudaSuccess;
+}
+
+// GMES_ERR_CUDA once a kernel has given up waiting.
+gmes_status check_wait_error() {
+  const int* w = g_wait_error.load();
+  if (w != nullptr && *static_cast<const volatile int*>(w) != 0)
+    return fail(GMES_ERR_CUDA, "a step kernel gave up waiting for its other blocks: the fields "
+                               "it was stepping are not valid");
+  return GMES_OK;
 }
 
 // Validate everything that can be checked without touching device memory.
@@ -118,6 +147,15 @@ gmes_status check_aux(const gmes_grid_desc* g) {
 
 }  // namespace
 
+int* wait_error_word() { return g_wait_error.load(); }
+
+int sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 1;
+  return n;
+}
+
 GridDev make_grid_dev(const gmes_grid_desc& g) {
   GridDev d;
   std::memset(&d, 0, sizeof(d));
@@ -129,6 +167,7 @@ GridDev make_grid_dev(const gmes_grid_desc& g) {
   d.dt = g.dt;
   d.active = g.active;
   d.nsrc = g.nsrc;
+  d.npml = g.npml;
   d.pointwise = (g.flags & GMES_FLAG_POINTWISE) ? 1 : 0;
   const CoefLayout L = coef_layout(g);
   char* base = static_cast<char*>(g.coef);
@@ -231,6 +270,45 @@ BatchView batch_view(const gmes_batch& b) {
   return v;
 }
 
+// Barrier words of the persistent kernel (gmes_persist.cu).  A direct launch
+// takes the next word of a ring far longer than the launches that can be in
+// flight; a graph captured here keeps a word until it is destroyed, and the
+// word then goes to the back of the queue, so that it is dealt again only
+// thousands of captures after its graph's last launch.  A capture begun by the
+// caller gets none: its graph's lifetime is not known here.
+std::mutex g_word_mutex;
+std::deque<int> g_free_words;                    // of destroyed graphs
+int g_next_word = kRingWords;                    // never used yet
+std::unordered_map<void*, int> g_graph_words;    // graph -> its word
+std::atomic<unsigned> g_ring_word{0};
+struct Capture {
+  int word = -1;
+};
+thread_local Capture* g_capture = nullptr;       // the capture this thread runs
+
+int take_word(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) return -1;
+  if (st == cudaStreamCaptureStatusNone) return (int)(g_ring_word++ % kRingWords);
+  if (g_capture == nullptr) return -1;
+  if (g_capture->word < 0) {
+    std::lock_guard<std::mutex> lock(g_word_mutex);
+    if (g_next_word < kRingWords + kGraphWords) {
+      g_capture->word = g_next_word++;
+    } else if (!g_free_words.empty()) {
+      g_capture->word = g_free_words.front();
+      g_free_words.pop_front();
+    }
+  }
+  return g_capture->word;
+}
+
+void give_word(int word) {
+  if (word < 0) return;
+  std::lock_guard<std::mutex> lock(g_word_mutex);
+  g_free_words.push_back(word);
+}
+
 // Host copies of the descriptors of the last kHostBatches prepared batches,
 // keyed by workspace address: gmes_batch_step passes them to the multi-grid
 // cell kernel as launch arguments (batches of at most kParamJobs grids).
@@ -297,6 +375,8 @@ Plan make_plan(const gmes_grid_desc& g, Plan* inc) {
   p.cplx = (g.flags & GMES_FLAG_COMPLEX) != 0;
   p.disp = (g.flags & GMES_FLAG_DISPERSIVE) != 0;
   p.im = p.cplx ? make_im_view(p.re, g) : p.re;
+  p.precision = g.precision;
+  p.word = -1;
   p.incident = nullptr;
   if (g.ntfsf > 0 && g.incident != nullptr && inc != nullptr) {
     *inc = make_plan(*g.incident, nullptr);
@@ -408,8 +488,8 @@ gmes_status gmes_build_coefficients(const gmes_grid_desc* g, const gmes_class_de
   const CoefLayout L = coef_layout(*g);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   char* base = static_cast<char*>(g->coef);
-  cudaError_t e = cudaSuccess;
-  if (ncls > 0)
+  cudaError_t e = ensure_wait_error();
+  if (e == cudaSuccess && ncls > 0)
     e = cudaMemcpyAsync(base + L.raw_classes, classes, ncls * sizeof(gmes_class_desc),
                         cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess && g->nparam > 0)
@@ -530,10 +610,36 @@ gmes_status gmes_step(const gmes_grid_desc* g, int32_t nsteps, void* stream) {
     return fail(GMES_ERR_VALUE, "nsteps = %d exceeds the incident grid's source capacity %d",
                 nsteps, g->incident->src_steps);
   if (nsteps == 0) return GMES_OK;
+  st = check_wait_error();
+  if (st != GMES_OK) return st;
   Plan inc;
-  const Plan p = make_plan(*g, &inc);
+  Plan p = make_plan(*g, &inc);
+  if (persist_takes(p) || (p.incident != nullptr && persist_takes(inc)))
+    p.word = inc.word = take_word(static_cast<cudaStream_t>(stream));
   cudaError_t e = launch_step(*g, p, nsteps, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "launching step kernels");
+  return GMES_OK;
+}
+
+gmes_status gmes_step_launches(const gmes_grid_desc* g, int32_t nsteps, int64_t* launches) {
+  gmes_status st = check_desc(g, true);
+  if (st != GMES_OK) return st;
+  if (launches == nullptr) return fail(GMES_ERR_VALUE, "launches is NULL");
+  if (nsteps < 0) return fail(GMES_ERR_VALUE, "nsteps = %d must be >= 0", nsteps);
+  Plan inc;
+  const Plan p = make_plan(*g, &inc);
+  auto per_half = [](const Plan& q) {
+    const int planes = q.cplx ? 2 : 1;
+    return 1 + planes * (1 + (q.re.nsrc > 0) + (q.re.ntfsf > 0) + (q.re.nprobe > 0));
+  };
+  if (nsteps == 0)
+    *launches = 0;
+  else if (persist_takes(p))
+    *launches = 1;
+  else
+    *launches = (int64_t)nsteps * (2 * per_half(p) + (p.incident == nullptr ? 0
+                                                      : persist_takes(inc)  ? 1
+                                                                            : 2 * per_half(inc)));
   return GMES_OK;
 }
 
@@ -551,6 +657,8 @@ gmes_status gmes_half_step(const gmes_grid_desc* g, int32_t side, int32_t step, 
   if (st != GMES_OK) return st;
   if (g->ntfsf > 0 && g->incident->nsrc > 0 && step >= g->incident->src_steps)
     return fail(GMES_ERR_INDEX, "step %d outside the incident grid's source-value buffer", step);
+  st = check_wait_error();
+  if (st != GMES_OK) return st;
   Plan inc;
   const Plan p = make_plan(*g, &inc);
   cudaError_t e = launch_half(*g, p, side, step, static_cast<cudaStream_t>(stream));
@@ -662,18 +770,32 @@ static gmes_status capture(cudaStream_t s, void** exec_out,
   if (exec_out == nullptr) return fail(GMES_ERR_VALUE, "graph_exec is NULL");
   cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return cuda_fail(e, "beginning stream capture");
+  Capture cap;
+  g_capture = &cap;
   gmes_status st = body();
+  g_capture = nullptr;
   cudaGraph_t graph = nullptr;
   e = cudaStreamEndCapture(s, &graph);
   if (st != GMES_OK) {
     if (graph) cudaGraphDestroy(graph);
+    give_word(cap.word);
     return st;
   }
-  if (e != cudaSuccess) return cuda_fail(e, "ending stream capture");
+  if (e != cudaSuccess) {
+    give_word(cap.word);
+    return cuda_fail(e, "ending stream capture");
+  }
   cudaGraphExec_t exec = nullptr;
   e = cudaGraphInstantiate(&exec, graph, 0);
   cudaGraphDestroy(graph);
-  if (e != cudaSuccess) return cuda_fail(e, "instantiating graph");
+  if (e != cudaSuccess) {
+    give_word(cap.word);
+    return cuda_fail(e, "instantiating graph");
+  }
+  if (cap.word >= 0) {
+    std::lock_guard<std::mutex> lock(g_word_mutex);
+    g_graph_words[exec] = cap.word;
+  }
   *exec_out = exec;
   return GMES_OK;
 }
@@ -692,6 +814,8 @@ gmes_status gmes_graph_capture_batch(const gmes_batch* b, int32_t nsteps, int32_
 
 gmes_status gmes_graph_launch(void* graph_exec, void* stream) {
   if (graph_exec == nullptr) return fail(GMES_ERR_VALUE, "graph_exec is NULL");
+  const gmes_status st = check_wait_error();
+  if (st != GMES_OK) return st;
   cudaError_t e = cudaGraphLaunch(static_cast<cudaGraphExec_t>(graph_exec),
                                   static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "launching graph");
@@ -700,7 +824,17 @@ gmes_status gmes_graph_launch(void* graph_exec, void* stream) {
 
 gmes_status gmes_graph_destroy(void* graph_exec) {
   if (graph_exec == nullptr) return GMES_OK;
+  int word = -1;
+  {
+    std::lock_guard<std::mutex> lock(g_word_mutex);
+    const auto it = g_graph_words.find(graph_exec);
+    if (it != g_graph_words.end()) {
+      word = it->second;
+      g_graph_words.erase(it);
+    }
+  }
   cudaError_t e = cudaGraphExecDestroy(static_cast<cudaGraphExec_t>(graph_exec));
+  give_word(word);
   if (e != cudaSuccess) return cuda_fail(e, "destroying graph");
   return GMES_OK;
 }
@@ -768,7 +902,7 @@ gmes_status gmes_read_field(const gmes_grid_desc* g, int32_t comp, double* host_
       host_out[i] = (double)tmp[2 * i] + (double)tmp[2 * i + 1];
   }
   if (e != cudaSuccess) return cuda_fail(e, "reading field");
-  return GMES_OK;
+  return check_wait_error();
 }
 
 gmes_status gmes_write_field(const gmes_grid_desc* g, int32_t comp, const double* host_in,

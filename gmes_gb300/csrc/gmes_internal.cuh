@@ -187,7 +187,7 @@ struct GridDev {
   // arrays they sample (the aux grid's Hy for the E side, Ex for the H side)
   const gmes_transparent* tfsf;
   int32_t ntfsf;
-  int32_t pad2;
+  int32_t npml;           // PML layers (profile sets) of the grid
   const void* tf_field[2];
   int64_t tf_npts[2];
   // probes: values recorded per step of a call
@@ -210,6 +210,8 @@ struct Plan {
   GridDev re, im;
   bool cplx, disp;
   const Plan* incident;
+  int precision;
+  int word;  // barrier word of the persistent kernel, -1: none to be had
 };
 
 // ---------------------------------------------------------------------------
@@ -452,6 +454,18 @@ cudaError_t launch_points(const gmes_points& g, void* inplace, const void* in1, 
 
 // Host-side helpers implemented in gmes_capi.cu.
 GridDev make_grid_dev(const gmes_grid_desc& g);
+// Pinned word that a kernel sets when a wait ran past its limit (NULL until
+// the first gmes_build_coefficients), and the SMs of the current device.
+int* wait_error_word();
+int sm_count();
+
+// Whole chunks of steps of a small grid in one launch (gmes_persist.cu).
+// Its grid-wide barrier counts in a word of its own per launch in flight:
+// kRingWords are dealt in turn to direct launches, the others belong to
+// captured graphs.
+constexpr int kRingWords = 1024, kGraphWords = 4096;
+bool persist_takes(const Plan& p);
+cudaError_t launch_persist(const Plan& p, int nsteps, int st0, cudaStream_t s);
 
 // Launchers implemented per precision in gmes_step.cu.
 cudaError_t launch_step(const gmes_grid_desc& g, const Plan& p, int nsteps, cudaStream_t s);

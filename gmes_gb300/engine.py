@@ -389,6 +389,12 @@ class GridEngine:
             done += k
         self._leave()
 
+    def step_launches(self, nsteps):
+        """Kernels one chunk of ``nsteps`` steps launches."""
+        out = C.c_int64()
+        N.check(self.lib.gmes_step_launches(C.byref(self.desc), int(nsteps), C.byref(out)))
+        return out.value
+
     def half_step(self, side, slot=0):
         """Enqueue one half-step (0: E, 1: H) reading staged source slot ``slot``."""
         N.check(self.lib.gmes_half_step(C.byref(self.desc), int(side), int(slot),

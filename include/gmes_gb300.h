@@ -308,6 +308,12 @@ gmes_status gmes_reset(const gmes_grid_desc* g, void* stream);
 gmes_status gmes_step(const gmes_grid_desc* g, int32_t nsteps, void* stream);
 
 /*
+ * The kernels that gmes_step(g, nsteps) launches, in *launches: a small grid's
+ * steps run as one launch, the others' as a few per half-step.
+ */
+gmes_status gmes_step_launches(const gmes_grid_desc* g, int32_t nsteps, int64_t* launches);
+
+/*
  * One half of step `step` (0-based index into src_val, < src_steps when
  * there are sources): side 0 = H ghost copy, E update, E sources; side 1 =
  * E ghost copy, H update, H sources.  gmes_step(g, n) is n pairs of these.
