@@ -2,10 +2,25 @@
 //
 // A small grid's step is bound by its launches: six dependent kernels (ghost
 // copy, cell update and sources of each half) of 2-3 us each, whatever they
-// compute.  Here the whole chunk is one cooperative launch.  Every block owns
-// a contiguous range of cells and walks the steps with one grid-wide barrier
-// after each half; the thread that updates a point also writes its ghost
-// images and applies its point sources, so a half needs no further phase.
+// compute.  Here the whole chunk is one cooperative launch that walks the steps
+// with one grid-wide barrier after each half; the thread that updates a point
+// also writes its ghost images, and its block applies its point sources, so a
+// half needs no further phase.  What then bounds a half-step, measured on GB300
+// (200^2 TMz, FP64, us per step): two barriers 2.8 (1.4 each: the stores reach
+// L2, one atomic, one poll), and in between the longest chain of dependent
+// loads and the FP64 pipe of the SM with most work:
+//   six launches per step                                  15.4
+//   one launch, k_cell's cell body, blocks of contiguous
+//   cells                                                   8.4
+//   tables in shared memory for class ids, coefficients
+//   and profiles                                            7.8
+//   the same number of cells on every SM                    7.1
+//   cells dealt to the blocks in groups of 32 (absorbing
+//   layer and media spread over the SMs)                    6.9
+//   one component per warp and group instead of three       6.1
+// (48x40x44 cells in 3-D: 22.9, 22.1, 24.0, 20.6, 18.9, 13.0.)  Blocks of 256
+// threads (4 per SM) ran 6.6 / 15.0, 1024 threads (1 per SM) 6.5 / 13.5, three
+// blocks of 512 (40 registers) 6.6 / 13.4.
 //
 // The ghost planes are left as FDTD.step leaves them (gmes/fdtd.py:1099-1122):
 // E's hold the present values, H's those from before the last E half.  A point
