@@ -598,44 +598,41 @@ __global__ void k_tmz_adj_src(const TmzDev t, int side) {
 // ---------------------------------------------------------------------------
 // Temporally blocked kernels (FP32).
 // ---------------------------------------------------------------------------
-// A block owns a TI x TJ tile of one design's lattice and keeps the region
-// of RI x RJ = (TI + 2 H) x (TJ + 2 H) points around it in shared memory
-// (region point (a, c) is lattice point (ri0 + a, rj0 + c) taken periodically,
-// so tiles at the lattice edge see its periodic images).  An E update reads
+// A block owns a TI x TJ tile of one design's lattice and advances the region
+// of RI x RJ = (TI + 2 H) x (TJ + 2 H) points around it (region point (a, c) is
+// lattice point (ri0 + a, rj0 + c) taken periodically, so tiles at the lattice
+// edge see its periodic images) by up to H steps per launch.  An E update reads
 // its low-side neighbours (i-1, j-1) and an H update its high-side ones
-// (i+1, j+1); updating every region point that has its neighbours in the
-// region, each half-step leaves the values exact on the region shrunk by
-// one more row and column on one side.  After s <= H steps the values are
-// exact on [s, RI-1-s] (H fields) and [s, RI-s] (E), which contain the tile,
-// so the tile is written back and the next launch reloads fresh halos.
-// DRAM traffic per step falls from a read and write of every field per
-// half-step to one read of the region and one write of the tile per H
-// steps.  Sources, monitors, design increments and gradients are applied
-// as in the one-step kernels: sources to every copy of their point in the
-// region, records and gradients only from tile points.
+// (i+1, j+1), so each half-step leaves the values exact on the region shrunk by
+// one more row and column on one side; after s <= H steps they are exact on
+// [s, RI-1-s] (H fields) and [s, RI-s] (E), which contain the tile.  What the
+// region's edge points hold meanwhile is never stored.  DRAM traffic per step
+// falls from a read and write of every field per half-step to one read of the
+// region and one write of the tile per H steps.
 //
-// Each launch reads every region point's flags and plain-form
-// coefficients from the resolved map once and keeps them in registers, so
-// a sub-step of a plain point is a few shared-memory operations; CPML
-// points inside a profile go through the per-point functions above.
+// The region lives in registers: a warp holds Q whole rows, a lane columns 2 l
+// and 2 l + 1 of each.  The neighbour along j is in the lane or one shuffle
+// away (one per two points), the neighbour along i in the lane, or, for the
+// warp's first or last row, in the row that the next warp left in shared
+// memory (two rows per warp and half-step, one barrier).  Measured on GB300
+// (512^2, 64 designs, 200 steps, ms forward / adjoint), against the form with
+// every field in shared memory (13 accesses per point-step forward, 21
+// adjoint; 113 instructions), which general tiles still take: 27.6 / 31.7 ->
+// 12.4 / 16.1.  The plain tiles alone (121 of 220) take 4.3 / 5.0 of it, near
+// the time of reading their regions and writing their tiles (5 TB/s); the
+// absorbing ones are bound by instruction issue at 32 warps per SM.
 //
-// Threads: RJ = 64 columns x 8 rows; a thread owns column c of rows
-// ty, ty + 8, ...; psi (and psi adjoint) values are loaded and stored only
-// on CPML points inside a profile.
+// What a tile's points are is settled once per design set (k_tmz_tiles), so
+// that the loops carry no per-point look-ups: plain tiles, most of them with
+// one set of coefficients; tiles with absorbing rows or absorbing columns,
+// whose psi stay in registers; and general tiles (TbTile), which take a
+// per-point loop over fields in shared memory.
 constexpr int kTbHalo = GMES_TMZ_MAX_BLOCK_STEPS;  // most steps per launch
-constexpr int kTbRJ = 64;    // region columns (j)
-constexpr int kTbRows = 8;   // thread rows
-constexpr int kTbThreads = kTbRJ * kTbRows;
-
-template <bool B>
-struct PsiTag {
-  static constexpr bool value = B;
-};
-constexpr int kTbRI = 32;    // region rows (i)
-#ifndef GMES_TB_MIN_BLOCKS
-#define GMES_TB_MIN_BLOCKS 2
-#endif
-constexpr int kTbMinBlocks = GMES_TB_MIN_BLOCKS;  // resident blocks per SM (register budget)
+constexpr int kTbRJ = 64;                          // region columns (j)
+constexpr int kTbTJ = kTbRJ - 2 * kTbHalo;
+constexpr int kTbWarps = 16;
+constexpr int kTbThreads = 32 * kTbWarps;
+static_assert(kTbHalo % 2 == 0, "a lane's two columns lie in the tile together");
 
 __device__ __forceinline__ int wrap_index(int v, int n) {
   if (v < 0) v += n;
@@ -645,96 +642,736 @@ __device__ __forceinline__ int wrap_index(int v, int n) {
   return v < 0 ? v + n : v;
 }
 
-template <int RI>
+// Q: rows per warp.
+template <class P, int Q>
 struct TbGeom {
-  static constexpr int H = kTbHalo, RJ = kTbRJ, TI = RI - 2 * kTbHalo, TJ = kTbRJ - 2 * kTbHalo;
-  static constexpr int NP = RI * kTbRJ, Q = RI / kTbRows;
-  static_assert(RI % kTbRows == 0 && TI > 0, "region rows");
+  using R = typename P::R;
+  static constexpr int RI = Q * kTbWarps, TI = RI - 2 * kTbHalo, NP = RI * kTbRJ;
+  // shared memory (values): the exchanged rows (one slot more per direction
+  // for the region's edge) and the layer's row and column entries, then, over the same
+  // bytes, a special tile's gradient state (2 FP64 per point, adjoint) and
+  // source map, or a general tile's 7 (forward) or 11 (adjoint) arrays
+  static constexpr int kRows = 2 * (kTbWarps + 1) * kTbRJ;
+  static constexpr int kHead = kRows + 6 * RI + 6 * kTbRJ;
+  static constexpr size_t special = (size_t)NP * (2 * sizeof(double) + sizeof(uint16_t));
+  static constexpr size_t fwd_bytes =
+      (size_t)kHead * sizeof(R) + (7 * NP * sizeof(R) > special ? 7 * NP * sizeof(R) : special);
+  static constexpr size_t adj_bytes =
+      (size_t)kHead * sizeof(R) + (11 * NP * sizeof(R) > special ? 11 * NP * sizeof(R) : special);
+  static_assert((kHead * sizeof(R)) % 16 == 0, "FP64 state is aligned");
+};
+
+// A point in the region's source maps: entry + 1, and whether it is hard.
+constexpr unsigned kTbHard = 0x8000u;
+
+// The block's tile and design: the designs of one tile are neighbours, so
+// that the blocks of an SM mostly run the same form and share the map.
+struct TbBlock {
+  int b, tile, row, col;
+  __device__ __forceinline__ TbBlock(const TmzDev& t) {
+    const unsigned n = (unsigned)t.nb, cols = (unsigned)(t.ny + kTbTJ - 1) / kTbTJ;
+    tile = (int)(blockIdx.x / n);
+    b = (int)(blockIdx.x - (unsigned)tile * n);
+    row = (int)((unsigned)tile / cols);
+    col = (int)((unsigned)tile - (unsigned)row * cols);
+  }
+};
+
+// What every thread of a block knows of its place.
+template <class P, int Q>
+struct TbPlace {
+  using R = typename P::R;
+  using G = TbGeom<P, Q>;
+  int lane, warp, b, ri0, rj0, j0, j1;
+  int64_t base;
+  bool pair, jt0, jt1;  // columns adjacent in memory; columns in the tile
+  int li[Q];
+  __device__ __forceinline__ TbPlace(const TmzDev& t) {
+    lane = threadIdx.x & 31;
+    warp = threadIdx.x >> 5;
+    const TbBlock k(t);
+    b = k.b;
+    ri0 = k.row * G::TI - kTbHalo;
+    rj0 = k.col * kTbTJ - kTbHalo;
+    const int c = 2 * lane;
+    j0 = wrap_index(rj0 + c, t.ny);
+    j1 = wrap_index(rj0 + c + 1, t.ny);
+    pair = (t.ny & 1) == 0;
+    const bool in = c >= kTbHalo && c < kTbHalo + kTbTJ;
+    jt0 = in && rj0 + c < t.ny;
+    jt1 = in && rj0 + c + 1 < t.ny;
+    base = (int64_t)b * t.plane;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) li[q] = wrap_index(ri0 + warp * Q + q, t.nx);
+  }
+  __device__ __forceinline__ bool row_in_tile(const TmzDev& t, int q) const {
+    const int a = warp * Q + q;
+    return a >= kTbHalo && a < kTbHalo + G::TI && ri0 + a < t.nx;
+  }
+  // the lane's two values of row q of an array of the design
+  __device__ __forceinline__ void load(const TmzDev& t, const void* p, int q, R v[2]) const {
+    const R* row = static_cast<const R*>(p) + base + (int64_t)li[q] * t.ny;
+    if (pair) {
+      struct alignas(2 * sizeof(R)) Two {
+        R a, b;
+      };
+      const Two w = *reinterpret_cast<const Two*>(row + j0);
+      v[0] = w.a;
+      v[1] = w.b;
+    } else {
+      v[0] = row[j0];
+      v[1] = row[j1];
+    }
+  }
+  __device__ __forceinline__ void store(const TmzDev& t, void* p, int q, const R v[2]) const {
+    R* row = static_cast<R*>(p) + base + (int64_t)li[q] * t.ny;
+    if (pair && jt0 && jt1) {
+      struct alignas(2 * sizeof(R)) Two {
+        R a, b;
+      };
+      *reinterpret_cast<Two*>(row + j0) = Two{v[0], v[1]};
+    } else {
+      if (jt0) row[j0] = v[0];
+      if (jt1) row[j1] = v[1];
+    }
+  }
+};
+
+// Two neighbouring values of a shared-memory row.
+template <class R>
+struct alignas(2 * sizeof(R)) Row2 {
+  R a, b;
+};
+
+// Entry m (b, c / d, 1 / (kappa d)) of layer pm's profiles: Ez and Hy along x,
+// Ez and Hx along y, at a lattice index.
+__device__ __forceinline__ int tb_entry(int m) { return m == 0 ? 0 : m + 2; }
+template <class P>
+__device__ __forceinline__ typename P::R prof_ex(const GridDev& g, int pm, int m, int i) {
+  return P::cfg(g.prof[pm][2][0] + (int64_t)i * kProfStride + tb_entry(m));
+}
+template <class P>
+__device__ __forceinline__ typename P::R prof_yx(const GridDev& g, int pm, int m, int i) {
+  return P::cfg(g.prof[pm][4][0] + (int64_t)(i + 1) * kProfStride + tb_entry(m));
+}
+template <class P>
+__device__ __forceinline__ typename P::R prof_ey(const GridDev& g, int pm, int m, int j) {
+  return P::cfg(g.prof[pm][2][1] + (int64_t)j * kProfStride + tb_entry(m));
+}
+template <class P>
+__device__ __forceinline__ typename P::R prof_xy(const GridDev& g, int pm, int m, int j) {
+  return P::cfg(g.prof[pm][3][1] + (int64_t)(j + 1) * kProfStride + tb_entry(m));
+}
+
+// A tile's absorbing rows (KIND kTbRows: on along x, Ez and Hy), columns
+// (kTbCols: on along y, Ez and Hx) or both (kTbBoth), with their psi (or psi adjoints) in
+// registers.  The updates are those of e_cpml and its siblings, term for term,
+// with the psi that is off left out (it is zero).  A row's state is
+// warp-uniform and branches; a column's selects.
+template <class P, int Q, int KIND>
+struct TbLayer {};
+
+template <class P, int Q>
+struct TbLayer<P, Q, kTbRows> {
+  using R = typename P::R;
+  using G = TbGeom<P, Q>;
+  bool re[Q], ry[Q];  // row on for Ez / Hy
+  R se[Q][2], sy[Q][2], k2[2];  // k2: the lane's columns' 1 / (kappa d) along y
+  __device__ __forceinline__ void load(const TmzDev& t, const TbPlace<P, Q>& p,
+                                       void* const* src) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const unsigned f = __ldg(t.pflags + (int64_t)p.li[q] * t.ny + p.j0);
+      re[q] = __any_sync(0xffffffffu, f & kTmzOnE1);
+      ry[q] = __any_sync(0xffffffffu, f & kTmzOnY);
+      p.load(t, src[0], q, se[q]);
+      p.load(t, src[3], q, sy[q]);
+    }
+  }
+  // the region rows' entries: Ez's b, c / d, 1 / (kappa d), then Hy's
+  __device__ __forceinline__ void fill(const GridDev& g, const TmzDev& t, const TbPlace<P, Q>& p,
+                                       const TbTile<R>& tile, R* sR) const {
+    for (int k = threadIdx.x; k < G::RI; k += kTbThreads) {
+      const int i = wrap_index(p.ri0 + k, t.nx);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        sR[m * G::RI + k] = prof_ex<P>(g, tile.pm, m, i);
+        sR[(3 + m) * G::RI + k] = prof_yx<P>(g, tile.pm, m, i);
+      }
+    }
+    for (int c = threadIdx.x; c < kTbRJ; c += kTbThreads)
+      sR[6 * G::RI + c] = prof_ey<P>(g, tile.pm, 2, wrap_index(p.rj0 + c, t.ny));
+  }
+  __device__ __forceinline__ void columns(const R* sR, int lane) {
+    k2[0] = sR[6 * G::RI + 2 * lane];
+    k2[1] = sR[6 * G::RI + 2 * lane + 1];
+  }
+  __device__ __forceinline__ void store(const TmzDev& t, const TbPlace<P, Q>& p,
+                                        void* const* dst) const {
+    const R none[2] = {P::zero(), P::zero()};
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      if (!p.row_in_tile(t, q)) continue;
+      if (re[q]) {  // both psi of every absorbing Ez point
+        p.store(t, dst[0], q, se[q]);
+        p.store(t, dst[1], q, none);
+      }
+      if (ry[q]) p.store(t, dst[3], q, sy[q]);
+    }
+  }
+  __device__ __forceinline__ R e_fwd(const R* sR, int a, int q, int h, R e, R c1, R c2n, R cdt,
+                                     R D1, R D2) {
+    if (!re[q]) return fmadd(fmadd(e, c1, D1), c2n, D2);
+    se[q][h] = fmadd(sR[a] * se[q][h], sR[G::RI + a], D1);
+    return fmadd(e, cdt, fmadd(fmadd(se[q][h] - P::zero(), sR[2 * G::RI + a], D1), -k2[h], D2));
+  }
+  __device__ __forceinline__ R x_fwd(int, int, R x, R cxn, R, R D1) { return fmadd(x, cxn, D1); }
+  __device__ __forceinline__ R y_fwd(const R* sR, int a, int q, int h, R y, R cy, R cdt, R D2) {
+    if (!ry[q]) return fmadd(y, cy, D2);
+    sy[q][h] = fmadd(sR[3 * G::RI + a] * sy[q][h], sR[4 * G::RI + a], D2);
+    return fmadd(y, -cdt, fmadd(-sy[q][h], -sR[5 * G::RI + a], D2));
+  }
+  // curl weights; the psi adjoint of an absorbing point advances
+  __device__ __forceinline__ R y_adj(const R* sR, int a, int q, int h, R l, R cy, R cdt) {
+    if (!ry[q]) return cy * l;
+    const R direct = cdt * (sR[5 * G::RI + a] * l);
+    const R t = fmadd(sy[q][h], cdt, l);
+    sy[q][h] = sR[3 * G::RI + a] * t;
+    return fmadd(direct, sR[4 * G::RI + a], t);
+  }
+  __device__ __forceinline__ R x_adj(int, int, R l, R cxn, R) { return cxn * l; }
+  __device__ __forceinline__ void e_adj(const R* sR, int a, int q, int h, R l, R c1, R c2n, R cdt,
+                                        R& v1, R& v2) {
+    if (!re[q]) {
+      v1 = c1 * l;
+      v2 = c2n * l;
+      return;
+    }
+    const R t = fmadd(se[q][h], cdt, l);
+    v1 = fmadd(cdt * (sR[2 * G::RI + a] * l), sR[G::RI + a], t);
+    v2 = -(cdt * (k2[h] * l));
+    se[q][h] = sR[a] * t;
+  }
+};
+
+template <class P, int Q>
+struct TbLayer<P, Q, kTbCols> {
+  using R = typename P::R;
+  using G = TbGeom<P, Q>;
+  bool ce[2], cx[2];  // column on for Ez / Hx
+  R ey[3][2], xy[3][2];
+  R se[Q][2], sx[Q][2];
+  __device__ __forceinline__ void load(const TmzDev& t, const TbPlace<P, Q>& p,
+                                       void* const* src) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const unsigned f = __ldg(t.pflags + (int64_t)p.li[0] * t.ny + (h ? p.j1 : p.j0));
+      ce[h] = f & kTmzOnE2;
+      cx[h] = f & kTmzOnX;
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      p.load(t, src[1], q, se[q]);
+      p.load(t, src[2], q, sx[q]);
+    }
+  }
+  // the region columns' entries (Ez's, then Hx's) and the rows' 1 / (kappa d)
+  __device__ __forceinline__ void fill(const GridDev& g, const TmzDev& t, const TbPlace<P, Q>& p,
+                                       const TbTile<R>& tile, R* sR) const {
+    for (int k = threadIdx.x; k < G::RI; k += kTbThreads)
+      sR[2 * G::RI + k] = prof_ex<P>(g, tile.pm, 2, wrap_index(p.ri0 + k, t.nx));
+    for (int c = threadIdx.x; c < kTbRJ; c += kTbThreads) {
+      const int j = wrap_index(p.rj0 + c, t.ny);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        sR[6 * G::RI + m * kTbRJ + c] = prof_ey<P>(g, tile.pm, m, j);
+        sR[6 * G::RI + (3 + m) * kTbRJ + c] = prof_xy<P>(g, tile.pm, m, j);
+      }
+    }
+  }
+  // the lane's columns' entries (after a barrier); off its slab a column's psi
+  // stays zero: b = c = 0, whatever the buffer holds there
+  __device__ __forceinline__ void columns(const R* sR, int lane) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        ey[m][h] = sR[6 * G::RI + m * kTbRJ + 2 * lane + h];
+        xy[m][h] = sR[6 * G::RI + (3 + m) * kTbRJ + 2 * lane + h];
+      }
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        if (!ce[h]) se[q][h] = P::zero();
+        if (!cx[h]) sx[q][h] = P::zero();
+      }
+    }
+  }
+  __device__ __forceinline__ void store(const TmzDev& t, const TbPlace<P, Q>& p,
+                                        void* const* dst) const {
+    const R none[2] = {P::zero(), P::zero()};
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      if (!p.row_in_tile(t, q)) continue;
+      if (__any_sync(0xffffffffu, ce[0] || ce[1])) {
+        p.store(t, dst[0], q, none);
+        p.store(t, dst[1], q, se[q]);
+      }
+      p.store(t, dst[2], q, sx[q]);
+    }
+  }
+  __device__ __forceinline__ R e_fwd(const R* sR, int a, int q, int h, R e, R c1, R c2n, R cdt,
+                                     R D1, R D2) {
+    const R n = fmadd(ey[0][h] * se[q][h], ey[1][h], D2);
+    const R on = fmadd(e, cdt, fmadd(fmadd(P::zero() - n, sR[2 * G::RI + a], D1), -ey[2][h], D2));
+    const R off = fmadd(fmadd(e, c1, D1), c2n, D2);
+    se[q][h] = ce[h] ? n : se[q][h];
+    return ce[h] ? on : off;
+  }
+  __device__ __forceinline__ R x_fwd(int q, int h, R x, R cxn, R cdt, R D1) {
+    const R n = fmadd(xy[0][h] * sx[q][h], xy[1][h], D1);
+    const R on = fmadd(x, -cdt, fmadd(n, xy[2][h], D1));
+    const R off = fmadd(x, cxn, D1);
+    sx[q][h] = cx[h] ? n : sx[q][h];
+    return cx[h] ? on : off;
+  }
+  __device__ __forceinline__ R y_fwd(const R*, int, int, int, R y, R cy, R, R D2) {
+    return fmadd(y, cy, D2);
+  }
+  __device__ __forceinline__ R y_adj(const R*, int, int, int, R l, R cy, R) { return cy * l; }
+  __device__ __forceinline__ R x_adj(int q, int h, R l, R cxn, R cdt) {
+    const R direct = -(cdt * (xy[2][h] * l));
+    const R t = fmadd(sx[q][h], -cdt, l);
+    const R on = fmadd(direct, xy[1][h], t);
+    sx[q][h] = cx[h] ? xy[0][h] * t : sx[q][h];
+    return cx[h] ? on : cxn * l;
+  }
+  __device__ __forceinline__ void e_adj(const R* sR, int a, int q, int h, R l, R c1, R c2n, R cdt,
+                                        R& v1, R& v2) {
+    const R t = fmadd(se[q][h], -cdt, l);
+    const R n2 = fmadd(-(cdt * (ey[2][h] * l)), ey[1][h], t);
+    v1 = ce[h] ? cdt * (sR[2 * G::RI + a] * l) : c1 * l;
+    v2 = ce[h] ? n2 : c2n * l;
+    se[q][h] = ce[h] ? ey[0][h] * t : se[q][h];
+  }
+};
+
+template <class P, int Q>
+struct TbLayer<P, Q, kTbBoth> {
+  using R = typename P::R;
+  using G = TbGeom<P, Q>;
+  bool re[Q], ry[Q], ce[2], cx[2];
+  R ey[3][2], xy[3][2];
+  R s1[Q][2], s2[Q][2], sx[Q][2], sy[Q][2];
+  __device__ __forceinline__ void load(const TmzDev& t, const TbPlace<P, Q>& p,
+                                       void* const* src) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const unsigned f = __ldg(t.pflags + (int64_t)p.li[0] * t.ny + (h ? p.j1 : p.j0));
+      ce[h] = f & kTmzOnE2;
+      cx[h] = f & kTmzOnX;
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const unsigned f = __ldg(t.pflags + (int64_t)p.li[q] * t.ny + p.j0);
+      re[q] = __any_sync(0xffffffffu, f & kTmzOnE1);
+      ry[q] = __any_sync(0xffffffffu, f & kTmzOnY);
+      p.load(t, src[0], q, s1[q]);
+      p.load(t, src[1], q, s2[q]);
+      p.load(t, src[2], q, sx[q]);
+      p.load(t, src[3], q, sy[q]);
+    }
+  }
+  __device__ __forceinline__ void fill(const GridDev& g, const TmzDev& t, const TbPlace<P, Q>& p,
+                                       const TbTile<R>& tile, R* sR) const {
+    for (int k = threadIdx.x; k < G::RI; k += kTbThreads) {
+      const int i = wrap_index(p.ri0 + k, t.nx);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        sR[m * G::RI + k] = prof_ex<P>(g, tile.pm, m, i);
+        sR[(3 + m) * G::RI + k] = prof_yx<P>(g, tile.pm, m, i);
+      }
+    }
+    for (int c = threadIdx.x; c < kTbRJ; c += kTbThreads) {
+      const int j = wrap_index(p.rj0 + c, t.ny);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        sR[6 * G::RI + m * kTbRJ + c] = prof_ey<P>(g, tile.pm, m, j);
+        sR[6 * G::RI + (3 + m) * kTbRJ + c] = prof_xy<P>(g, tile.pm, m, j);
+      }
+    }
+  }
+  __device__ __forceinline__ void columns(const R* sR, int lane) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        ey[m][h] = sR[6 * G::RI + m * kTbRJ + 2 * lane + h];
+        xy[m][h] = sR[6 * G::RI + (3 + m) * kTbRJ + 2 * lane + h];
+      }
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        if (!re[q]) s1[q][h] = P::zero();
+        if (!ry[q]) sy[q][h] = P::zero();
+        if (!ce[h]) s2[q][h] = P::zero();
+        if (!cx[h]) sx[q][h] = P::zero();
+      }
+    }
+  }
+  __device__ __forceinline__ void store(const TmzDev& t, const TbPlace<P, Q>& p,
+                                        void* const* dst) const {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      if (!p.row_in_tile(t, q)) continue;
+      p.store(t, dst[0], q, s1[q]);
+      p.store(t, dst[1], q, s2[q]);
+      p.store(t, dst[2], q, sx[q]);
+      p.store(t, dst[3], q, sy[q]);
+    }
+  }
+  __device__ __forceinline__ R e_fwd(const R* sR, int a, int q, int h, R e, R c1, R c2n, R cdt,
+                                     R D1, R D2) {
+    if (re[q]) s1[q][h] = fmadd(sR[a] * s1[q][h], sR[G::RI + a], D1);
+    const R n2 = fmadd(ey[0][h] * s2[q][h], ey[1][h], D2);
+    s2[q][h] = ce[h] ? n2 : s2[q][h];
+    const R on =
+        fmadd(e, cdt, fmadd(fmadd(s1[q][h] - s2[q][h], sR[2 * G::RI + a], D1), -ey[2][h], D2));
+    if (re[q]) return on;
+    const R off = fmadd(fmadd(e, c1, D1), c2n, D2);
+    return ce[h] ? on : off;
+  }
+  __device__ __forceinline__ R x_fwd(int q, int h, R x, R cxn, R cdt, R D1) {
+    const R n = fmadd(xy[0][h] * sx[q][h], xy[1][h], D1);
+    const R on = fmadd(x, -cdt, fmadd(n, xy[2][h], D1));
+    const R off = fmadd(x, cxn, D1);
+    sx[q][h] = cx[h] ? n : sx[q][h];
+    return cx[h] ? on : off;
+  }
+  __device__ __forceinline__ R y_fwd(const R* sR, int a, int q, int h, R y, R cy, R cdt, R D2) {
+    if (!ry[q]) return fmadd(y, cy, D2);
+    sy[q][h] = fmadd(sR[3 * G::RI + a] * sy[q][h], sR[4 * G::RI + a], D2);
+    return fmadd(y, -cdt, fmadd(-sy[q][h], -sR[5 * G::RI + a], D2));
+  }
+  __device__ __forceinline__ R y_adj(const R* sR, int a, int q, int h, R l, R cy, R cdt) {
+    if (!ry[q]) return cy * l;
+    const R direct = cdt * (sR[5 * G::RI + a] * l);
+    const R t = fmadd(sy[q][h], cdt, l);
+    sy[q][h] = sR[3 * G::RI + a] * t;
+    return fmadd(direct, sR[4 * G::RI + a], t);
+  }
+  __device__ __forceinline__ R x_adj(int q, int h, R l, R cxn, R cdt) {
+    const R direct = -(cdt * (xy[2][h] * l));
+    const R t = fmadd(sx[q][h], -cdt, l);
+    const R on = fmadd(direct, xy[1][h], t);
+    sx[q][h] = cx[h] ? xy[0][h] * t : sx[q][h];
+    return cx[h] ? on : cxn * l;
+  }
+  __device__ __forceinline__ void e_adj(const R* sR, int a, int q, int h, R l, R c1, R c2n, R cdt,
+                                        R& v1, R& v2) {
+    const R d1 = cdt * (sR[2 * G::RI + a] * l), d2 = -(cdt * (ey[2][h] * l));
+    const R t2 = fmadd(s2[q][h], -cdt, l);
+    const R n2 = fmadd(d2, ey[1][h], t2);
+    s2[q][h] = ce[h] ? ey[0][h] * t2 : s2[q][h];
+    if (re[q]) {
+      const R t1 = fmadd(s1[q][h], cdt, l);
+      s1[q][h] = sR[a] * t1;
+      v1 = fmadd(d1, sR[G::RI + a], t1);
+      v2 = ce[h] ? n2 : d2;
+    } else {
+      v1 = ce[h] ? d1 : c1 * l;
+      v2 = ce[h] ? n2 : c2n * l;
+    }
+  }
+};
+
+// The region's map of Ez sources: every copy of every source's point.
+template <class P, int Q>
+__device__ __forceinline__ void tb_source_map(const TmzDev& t, int ri0, int rj0, uint16_t* map) {
+  using G = TbGeom<P, Q>;
+  static_assert(G::NP % 8 == 0, "cleared as 16-byte words");
+  for (int k = threadIdx.x; k < G::NP / 8; k += kTbThreads)
+    reinterpret_cast<uint4*>(map)[k] = make_uint4(0, 0, 0, 0);
+  __syncthreads();
+  for (int k = threadIdx.x; k < t.nsrc; k += kTbThreads) {
+    const gmes_point_source s = t.src[k];
+    if (s.comp != 2 || s.offset < 0 || s.offset >= t.plane) continue;
+    int li, lj;
+    if (t.plane < (int64_t(1) << 31)) {
+      li = (int)((unsigned)s.offset / (unsigned)t.ny);
+      lj = (int)((unsigned)s.offset - (unsigned)li * (unsigned)t.ny);
+    } else {
+      li = (int)(s.offset / t.ny);
+      lj = (int)(s.offset - (int64_t)li * t.ny);
+    }
+    const uint16_t v = (uint16_t)((k + 1) | (s.mode == 0 ? kTbHard : 0u));
+    for (int a = wrap_index(li - ri0, t.nx); a < G::RI; a += t.nx)
+      for (int c = wrap_index(lj - rj0, t.ny); c < kTbRJ; c += t.ny) map[a * kTbRJ + c] = v;
+  }
+  __syncthreads();
+}
+
+// The value of the E half's source of step n at map entry v (0: none), and a
+// field value after that source.
+template <class P>
+__device__ __forceinline__ typename P::R tb_value(const TmzDev& t, unsigned v, int n) {
+  if (v == 0) return P::zero();
+  const int k = (int)(v & (kTbHard - 1)) - 1;
+  return P::from_double(__ldg(t.src_val + (int64_t)(n - 1) * 2 * t.nsrc + k));
+}
+template <class R>
+__device__ __forceinline__ R tb_source(unsigned v, R f, R s) {
+  return v == 0 ? f : ((v & kTbHard) ? s : f - s);
+}
+
+// A special tile: the flags that each of the lane's rows holds (warp-uniform),
+// so that a row without any takes the bare update, and per point what its
+// source, monitor and design pixel need.
+template <class P, int Q>
+struct TbSpecial {
+  using R = typename P::R;
+  using T = typename P::T;
+  using G = TbGeom<P, Q>;
+  unsigned row[Q];
+  uint16_t* map;   // Ez sources
+  double* acc;     // gradient of the launch, then -1 / eps, per region point
+  R v[Q][2];       // source values (forward) or design increments (adjoint)
+  __device__ __forceinline__ void init(unsigned char* smem) {
+    acc = reinterpret_cast<double*>(smem + G::kHead * sizeof(R));
+    map = reinterpret_cast<uint16_t*>(acc + 2 * G::NP);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) row[q] = 0;
+  }
+  __device__ __forceinline__ unsigned flags(const TmzDev& t, const TbPlace<P, Q>& p, int q,
+                                            int h) const {
+    return __ldg(t.pflags + (int64_t)p.li[q] * t.ny + (h ? p.j1 : p.j0));
+  }
+  __device__ __forceinline__ bool owned(const TmzDev& t, const TbPlace<P, Q>& p, int q,
+                                        int h) const {
+    return p.row_in_tile(t, q) && (h ? p.jt1 : p.jt0);
+  }
+  __device__ __forceinline__ int64_t pixel(const TmzDev& t, const TbPlace<P, Q>& p, int q,
+                                           int h) const {
+    return design_index(t, p.li[q], h ? p.j1 : p.j0);
+  }
+  __device__ __forceinline__ int at(const TbPlace<P, Q>& p, int q, int h) const {
+    return (p.warp * Q + q) * kTbRJ + 2 * p.lane + h;
+  }
+  __device__ __forceinline__ void load(const TmzDev& t, const TbPlace<P, Q>& p,
+                                       const TbTile<R>& tile) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      row[q] = __reduce_or_sync(0xffffffffu, flags(t, p, q, 0) | flags(t, p, q, 1));
+    if (tile.any & kTmzSrcE) tb_source_map<P, Q>(t, p.ri0, p.rj0, map);
+  }
+  // forward: the sources' values of step n, fetched a step ahead
+  __device__ __forceinline__ void fetch(const TmzDev& t, const TbPlace<P, Q>& p, int n) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      if (row[q] & kTmzSrcE) {
+        v[q][0] = tb_value<P>(t, map[at(p, q, 0)], n);
+        v[q][1] = tb_value<P>(t, map[at(p, q, 1)], n);
+      }
+  }
+  __device__ __forceinline__ void source(const TbPlace<P, Q>& p, int q, R e[2]) const {
+    if (!(row[q] & kTmzSrcE)) return;
+    e[0] = tb_source((unsigned)map[at(p, q, 0)], e[0], v[q][0]);
+    e[1] = tb_source((unsigned)map[at(p, q, 1)], e[1], v[q][1]);
+  }
+  // forward: the design increment of a point of step slot
+  __device__ __forceinline__ void record(const TmzDev& t, const TbPlace<P, Q>& p, int q, int h,
+                                         int slot, R c1, R c2n, R D1, R D2) const {
+    if ((flags(t, p, q, h) & kTmzDesign) && owned(t, p, q, h))
+      static_cast<T*>(t.hist)[((int64_t)slot * t.nb + p.b) * t.dn[0] * t.dn[1] +
+                              pixel(t, p, q, h)] = fmadd(c2n * D2, c1, D1);
+  }
+  __device__ __forceinline__ void monitor(const TmzDev& t, const TbPlace<P, Q>& p, int q, int n,
+                                          const R e[2]) const {
+    if (!(row[q] & kTmzMonitor)) return;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if ((flags(t, p, q, h) & kTmzMonitor) && owned(t, p, q, h))
+        t.mon[((int64_t)p.b * t.total_steps + (n - 1)) * t.mn[0] * t.mn[1] +
+              monitor_index(t, p.li[q], h ? p.j1 : p.j0)] = to_double(e[h]);
+  }
+  // adjoint: the objective's seed, hard sources, and the design gradient,
+  // which accumulates in shared memory over the launch
+  __device__ __forceinline__ void seed(const GridDev& g, const TmzDev& t, const TbPlace<P, Q>& p,
+                                       int q, int n, R e[2]) const {
+    if (!(row[q] & kTmzMonitor)) return;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (flags(t, p, q, h) & kTmzMonitor) {
+        bool has;
+        e[h] = e[h] + P::from_double(seed_of(g, t, p.b, p.li[q], h ? p.j1 : p.j0, n, &has));
+      }
+  }
+  __device__ __forceinline__ void zero(const TbPlace<P, Q>& p, int q, R e[2]) const {
+    if (!(row[q] & kTmzSrcE)) return;
+    if (map[at(p, q, 0)] & kTbHard) e[0] = P::zero();
+    if (map[at(p, q, 1)] & kTbHard) e[1] = P::zero();
+  }
+  template <class F>
+  __device__ __forceinline__ void pixels(const TmzDev& t, const TbPlace<P, Q>& p, F f) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      if (row[q] & kTmzDesign) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if ((flags(t, p, q, h) & kTmzDesign) && owned(t, p, q, h)) f(q, h, pixel(t, p, q, h));
+      }
+  }
+  __device__ __forceinline__ void grad_load(const TmzDev& t, const TbPlace<P, Q>& p) {
+    const int64_t b = (int64_t)p.b * t.dn[0] * t.dn[1];
+    pixels(t, p, [&](int q, int h, int64_t dp) {
+      acc[at(p, q, h)] = t.grad[b + dp];
+      acc[G::NP + at(p, q, h)] = t.dc[b + dp].neg_reps;
+    });
+  }
+  __device__ __forceinline__ void grad_fetch(const TmzDev& t, const TbPlace<P, Q>& p, int slot) {
+    const int64_t b = ((int64_t)slot * t.nb + p.b) * t.dn[0] * t.dn[1];
+    pixels(t, p, [&](int q, int h, int64_t dp) {
+      v[q][h] = P::ld(static_cast<const T*>(t.hist) + b + dp);
+    });
+  }
+  __device__ __forceinline__ void grad_add(const TmzDev& t, const TbPlace<P, Q>& p, int q,
+                                           const R e[2]) {
+    if (!(row[q] & kTmzDesign)) return;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if ((flags(t, p, q, h) & kTmzDesign) && owned(t, p, q, h)) {
+        const int k = at(p, q, h);
+        acc[k] += to_double(e[h]) * to_double(v[q][h]) * acc[G::NP + k];
+      }
+  }
+  __device__ __forceinline__ void grad_store(const TmzDev& t, const TbPlace<P, Q>& p) {
+    const int64_t b = (int64_t)p.b * t.dn[0] * t.dn[1];
+    pixels(t, p, [&](int q, int h, int64_t dp) { t.grad[b + dp] = acc[at(p, q, h)]; });
+  }
+};
+
+// Ez's coefficients of the lane's two points of row q: the tile's, or, where
+// they vary, those that load() took (c1 and c2n; an absorbing point's cdt is
+// its c1).
+template <class P, int Q, bool VARY>
+struct TbCoef {
+  using R = typename P::R;
+  R c1[Q][2], c2n[Q][2];
+  __device__ __forceinline__ void load(const TmzDev& t, const TbPlace<P, Q>& p) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int j = h ? p.j1 : p.j0;
+        const int64_t ll = (int64_t)p.li[q] * t.ny + j;
+        e_coef<P>(t, p.b, p.li[q], j, ll, __ldg(t.pflags + ll), c1[q][h], c2n[q][h]);
+      }
+  }
+  __device__ __forceinline__ void get(const TbTile<R>&, int q, int h, R& a, R& b) const {
+    a = c1[q][h];
+    b = c2n[q][h];
+  }
+};
+template <class P, int Q>
+struct TbCoef<P, Q, false> {
+  using R = typename P::R;
+  __device__ __forceinline__ void load(const TmzDev&, const TbPlace<P, Q>&) {}
+  __device__ __forceinline__ void get(const TbTile<R>& tile, int, int, R& a, R& b) const {
+    a = tile.c[0];
+    b = tile.c[1];
+  }
+};
+
+template <bool B>
+struct BoolTag {
+  static constexpr bool value = B;
 };
 
 // Plain-form coefficients of one region point.
+template <class R>
 struct TbPoint {
-  float c1, c2n;  // Ez: c1, -c2
-  float cxn, cy;  // Hx: -c1, Hy: c2
+  R c1, c2n;  // Ez: c1, -c2
+  R cxn, cy;  // Hx: -c1, Hy: c2
 };
 
 // Flags and plain-form coefficients of lattice point (i, j) of design b,
 // from the resolved map.
-__device__ __forceinline__ unsigned tb_point(const TmzDev& t, int b, int i, int j, TbPoint& p) {
-  using P = PolF32;
+template <class P>
+__device__ __forceinline__ unsigned tb_point(const TmzDev& t, int b, int i, int j,
+                                             TbPoint<typename P::R>& p) {
   const int64_t ll = (int64_t)i * t.ny + j;
   const unsigned f = __ldg(t.pflags + ll);
   e_coef<P>(t, b, i, j, ll, f, p.c1, p.c2n);
-  p.cxn = __ldg(map_coef<P>(t, 2) + ll);
-  p.cy = __ldg(map_coef<P>(t, 3) + ll);
+  p.cxn = P::ld(map_coef<P>(t, 2) + ll);
+  p.cy = P::ld(map_coef<P>(t, 3) + ll);
   return f;
 }
 
 // Apply this half's sources of step n to every copy of their point in the
 // region: the forward (ADJ false: hard sources set the value, current
 // sources subtract theirs) or the adjoint (ADJ true: hard sources zero it).
-template <bool ADJ>
+template <class P, bool ADJ>
 __device__ __forceinline__ void tb_sources(const TmzDev& t, int side, int n, int ri0, int rj0,
-                                           int RI, int RJ, float* fE, float* fX, float* fY) {
-  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+                                           int RI, int RJ, typename P::R* fE,
+                                           typename P::R* fX, typename P::R* fY) {
+  using R = typename P::R;
+  const int tid = threadIdx.x;
   for (int k = tid; k < t.nsrc; k += kTbThreads) {
     const gmes_point_source s = t.src[k];
     if (s.comp < 2 || s.comp > 4 || (s.comp == 2) != (side == 0)) continue;
     if (s.offset < 0 || s.offset >= t.plane) continue;
     if (ADJ && s.mode != 0) continue;
     const int li = (int)(s.offset / t.ny), lj = (int)(s.offset - (int64_t)li * t.ny);
-    float* f = s.comp == 2 ? fE : (s.comp == 3 ? fX : fY);
-    const float v =
-        ADJ ? 0.f
-            : PolF32::from_double(t.src_val[((int64_t)(n - 1) * 2 + side) * t.nsrc + k]);
+    R* f = s.comp == 2 ? fE : (s.comp == 3 ? fX : fY);
+    const R v =
+        ADJ ? P::zero()
+            : P::from_double(t.src_val[((int64_t)(n - 1) * 2 + side) * t.nsrc + k]);
     for (int a = wrap_index(li - ri0, t.nx); a < RI; a += t.nx)
       for (int c = wrap_index(lj - rj0, t.ny); c < RJ; c += t.ny) {
-        float* q = f + a * RJ + c;
+        R* q = f + a * RJ + c;
         *q = (ADJ || s.mode == 0) ? v : *q - v;
       }
   }
 }
 
-// Forward steps n0+1 .. n0+nsub (nsub <= kTbHalo) of one tile, from the
-// state in t.f to the state in t.tmp (the launch's other blocks still read
-// t.f for their halos, so the result must not overwrite it).  slot0 >= 0:
-// record the design increments of step n0+1+s at hist slot slot0+s;
-// rec_mon: record monitor row n-1 of every step n.
-template <int RI>
-__global__ void __launch_bounds__(kTbThreads, kTbMinBlocks)
-    k_tmz_tb_fwd(const GridDev g, const TmzDev t, int n0, int nsub, int slot0, int rec_mon) {
-  using P = PolF32;
-  using G = TbGeom<RI>;
-  constexpr int H = G::H, RJ = G::RJ, TI = G::TI, TJ = G::TJ, NP = G::NP, Q = G::Q;
-  extern __shared__ float4 tb_smem[];
-  float* sE = reinterpret_cast<float*>(tb_smem);
-  float* sX = sE + NP;
-  float* sY = sX + NP;
-  float* sS = sY + NP;  // psi of Ez (x, y), Hx, Hy: sS + k * NP
-  const int c = threadIdx.x, ty = threadIdx.y, b = blockIdx.z;
-  const int ri0 = (int)blockIdx.y * TI - H, rj0 = (int)blockIdx.x * TJ - H;
+// The forward steps of a general tile: every field in shared memory, a thread
+// the points of one column a few rows apart, per-point updates (e_cpml and its
+// siblings) where the flags ask for them.
+template <class P, int QW>
+__device__ void tb_general_fwd(const GridDev& g, const TmzDev& t, int n0, int nsub, int slot0,
+                               int rec_mon, unsigned char* smem) {
+  using R = typename P::R;
+  using T = typename P::T;
+  using G = TbGeom<P, QW>;
+  constexpr int H = kTbHalo, RJ = kTbRJ, RI = G::RI, TI = G::TI, TJ = kTbTJ, NP = G::NP;
+  constexpr int kRowsAtOnce = kTbThreads / RJ, Q = RI / kRowsAtOnce;
+  R* sE = reinterpret_cast<R*>(smem) + G::kHead;
+  R* sX = sE + NP;
+  R* sY = sX + NP;
+  R* sS = sY + NP;  // psi of Ez (x, y), Hx, Hy: sS + k * NP
+  const TbBlock blk(t);
+  const int c = threadIdx.x % RJ, ty = threadIdx.x / RJ, b = blk.b;
+  const int ri0 = blk.row * TI - H, rj0 = blk.col * TJ - H;
   const int j = wrap_index(rj0 + c, t.ny);
   const bool jtile = c >= H && c < H + TJ && rj0 + c < t.ny;
   const int64_t base = (int64_t)b * t.plane;
   int li[Q];
-  TbPoint pt[Q];
+  TbPoint<R> pt[Q];
   unsigned fl[Q];
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
-    const int a = ty + kTbRows * q, k = a * RJ + c;
+    const int a = ty + kRowsAtOnce * q, k = a * RJ + c;
     li[q] = wrap_index(ri0 + a, t.nx);
-    fl[q] = tb_point(t, b, li[q], j, pt[q]);
+    fl[q] = tb_point<P>(t, b, li[q], j, pt[q]);
     if (jtile && a >= H && a < H + TI && ri0 + a < t.nx) fl[q] |= 1u << 31;  // tile point
     const int64_t lin = base + (int64_t)li[q] * t.ny + j;
-    sE[k] = __ldg(static_cast<const float*>(t.f[0]) + lin);
-    sX[k] = __ldg(static_cast<const float*>(t.f[1]) + lin);
-    sY[k] = __ldg(static_cast<const float*>(t.f[2]) + lin);
+    sE[k] = __ldg(static_cast<const T*>(t.f[0]) + lin);
+    sX[k] = __ldg(static_cast<const T*>(t.f[1]) + lin);
+    sY[k] = __ldg(static_cast<const T*>(t.f[2]) + lin);
     if (fl[q] & kTmzPsiE) {
-      sS[k] = __ldg(static_cast<const float*>(t.f[3]) + lin);
-      sS[NP + k] = __ldg(static_cast<const float*>(t.f[4]) + lin);
+      sS[k] = __ldg(static_cast<const T*>(t.f[3]) + lin);
+      sS[NP + k] = __ldg(static_cast<const T*>(t.f[4]) + lin);
     }
-    if (fl[q] & kTmzPsiX) sS[2 * NP + k] = __ldg(static_cast<const float*>(t.f[5]) + lin);
-    if (fl[q] & kTmzPsiY) sS[3 * NP + k] = __ldg(static_cast<const float*>(t.f[6]) + lin);
+    if (fl[q] & kTmzPsiX) sS[2 * NP + k] = __ldg(static_cast<const T*>(t.f[5]) + lin);
+    if (fl[q] & kTmzPsiY) sS[3 * NP + k] = __ldg(static_cast<const T*>(t.f[6]) + lin);
   }
   unsigned any = 0;
 #pragma unroll
@@ -753,13 +1390,13 @@ __global__ void __launch_bounds__(kTbThreads, kTbMinBlocks)
       const int n = n0 + s + 1;
   #pragma unroll
       for (int q = 0; q < Q; ++q) {
-        const int a = ty + kTbRows * q, k = a * RJ + c;
+        const int a = ty + kRowsAtOnce * q, k = a * RJ + c;
         if (a >= 1 && c >= 1) {
-          const float D1 = sY[k] - sY[k - RJ], D2 = sX[k] - sX[k - 1];
+          const R D1 = sY[k] - sY[k - RJ], D2 = sX[k] - sX[k - 1];
           if (fl[q] & kTmzPlainE) {
             sE[k] = fmadd(fmadd(sE[k], pt[q].c1, D1), pt[q].c2n, D2);
             if ((fl[q] & kTmzDesign) && (fl[q] >> 31) && slot0 >= 0)
-              static_cast<float*>(t.hist)[((int64_t)(slot0 + s) * t.nb + b) * nd +
+              static_cast<T*>(t.hist)[((int64_t)(slot0 + s) * t.nb + b) * nd +
                                           design_index(t, li[q], j)] =
                   fmadd(pt[q].c2n * D2, pt[q].c1, D1);
           } else if (PSI && (fl[q] & kTmzPsiE)) {
@@ -769,15 +1406,15 @@ __global__ void __launch_bounds__(kTbThreads, kTbMinBlocks)
       }
       __syncthreads();
       if (src_e) {
-        tb_sources<false>(t, 0, n, ri0, rj0, RI, RJ, sE, sX, sY);
+        tb_sources<P, false>(t, 0, n, ri0, rj0, RI, RJ, sE, sX, sY);
         __syncthreads();
       }
   #pragma unroll
       for (int q = 0; q < Q; ++q) {
-        const int a = ty + kTbRows * q, k = a * RJ + c;
+        const int a = ty + kRowsAtOnce * q, k = a * RJ + c;
         if (a < RI - 1 && c < RJ - 1) {
-          const float e0 = sE[k];
-          const float dx = sE[k + 1] - e0, dy = sE[k + RJ] - e0;
+          const R e0 = sE[k];
+          const R dx = sE[k + 1] - e0, dy = sE[k + RJ] - e0;
           if (fl[q] & kTmzPlainX)
             sX[k] = fmadd(sX[k], pt[q].cxn, dx);
           else if (PSI && (fl[q] & kTmzPsiX))
@@ -788,84 +1425,80 @@ __global__ void __launch_bounds__(kTbThreads, kTbMinBlocks)
             sY[k] = y_cpml<P>(g, fl[q], pt[q].cy, li[q], sY[k], dy, sS + 3 * NP + k);
           if (rec_mon && (fl[q] & kTmzMonitor) && (fl[q] >> 31))
             t.mon[((int64_t)b * t.total_steps + (n - 1)) * nm + monitor_index(t, li[q], j)] =
-                (double)e0;
+                to_double(e0);
         }
       }
       __syncthreads();
       if (src_h) {
-        tb_sources<false>(t, 1, n, ri0, rj0, RI, RJ, sE, sX, sY);
+        tb_sources<P, false>(t, 1, n, ri0, rj0, RI, RJ, sE, sX, sY);
         __syncthreads();
       }
     }
   };
   if (psi_any)
-    steps(PsiTag<true>{});
+    steps(BoolTag<true>{});
   else
-    steps(PsiTag<false>{});
+    steps(BoolTag<false>{});
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     if (!(fl[q] >> 31)) continue;
-    const int k = (ty + kTbRows * q) * RJ + c;
+    const int k = (ty + kRowsAtOnce * q) * RJ + c;
     const int64_t lin = base + (int64_t)li[q] * t.ny + j;
-    static_cast<float*>(t.tmp[0])[lin] = sE[k];
-    static_cast<float*>(t.tmp[1])[lin] = sX[k];
-    static_cast<float*>(t.tmp[2])[lin] = sY[k];
+    static_cast<T*>(t.tmp[0])[lin] = sE[k];
+    static_cast<T*>(t.tmp[1])[lin] = sX[k];
+    static_cast<T*>(t.tmp[2])[lin] = sY[k];
     if (fl[q] & kTmzPsiE) {
-      static_cast<float*>(t.tmp[3])[lin] = sS[k];
-      static_cast<float*>(t.tmp[4])[lin] = sS[NP + k];
+      static_cast<T*>(t.tmp[3])[lin] = sS[k];
+      static_cast<T*>(t.tmp[4])[lin] = sS[NP + k];
     }
-    if (fl[q] & kTmzPsiX) static_cast<float*>(t.tmp[5])[lin] = sS[2 * NP + k];
-    if (fl[q] & kTmzPsiY) static_cast<float*>(t.tmp[6])[lin] = sS[3 * NP + k];
+    if (fl[q] & kTmzPsiX) static_cast<T*>(t.tmp[5])[lin] = sS[2 * NP + k];
+    if (fl[q] & kTmzPsiY) static_cast<T*>(t.tmp[6])[lin] = sS[3 * NP + k];
   }
 }
 
-// Adjoint steps n0 + nsub down to n0 + 1 of one tile (the transposes of
-// k_tmz_ah / k_tmz_ae, same order), the field adjoints from t.l to
-// t.tmp[0..2]; the gradient of step n uses hist slot n - step0 - 1.  The
-// psi adjoints are read from buffer rb and written to the other one, so no
-// block overwrites what another still reads (adjoint_blocked chooses rb so
-// that a call leaves them where the one-step kernels' step-parity
-// convention expects them).
-template <int RI>
-__global__ void __launch_bounds__(kTbThreads, kTbMinBlocks)
-    k_tmz_tb_adj(const GridDev g, const TmzDev t, int n0, int nsub, int step0, int rb) {
-  using P = PolF32;
-  using G = TbGeom<RI>;
-  constexpr int H = G::H, RJ = G::RJ, TI = G::TI, TJ = G::TJ, NP = G::NP, Q = G::Q;
-  extern __shared__ float4 tb_smem[];
-  float* sLE = reinterpret_cast<float*>(tb_smem);
-  float* sLX = sLE + NP;
-  float* sLY = sLX + NP;
-  float* sP = sLY + NP;      // psi adjoints of Ez (x, y), Hx, Hy: sP + k * NP
-  float* sW1 = sP + 4 * NP;  // curl weights of the H half: Hx
-  float* sW2 = sW1 + NP;     //   and Hy
-  float* sV1 = sW2 + NP;     // curl weights of the E half: Ez's first
-  float* sV2 = sV1 + NP;     //   and its second
-  const int c = threadIdx.x, ty = threadIdx.y, b = blockIdx.z;
-  const int ri0 = (int)blockIdx.y * TI - H, rj0 = (int)blockIdx.x * TJ - H;
+// The adjoint steps of a general tile, as tb_general_fwd.
+template <class P, int QW>
+__device__ void tb_general_adj(const GridDev& g, const TmzDev& t, int n0, int nsub, int step0,
+                               int rb, unsigned char* smem) {
+  using R = typename P::R;
+  using T = typename P::T;
+  using G = TbGeom<P, QW>;
+  constexpr int H = kTbHalo, RJ = kTbRJ, RI = G::RI, TI = G::TI, TJ = kTbTJ, NP = G::NP;
+  constexpr int kRowsAtOnce = kTbThreads / RJ, Q = RI / kRowsAtOnce;
+  R* sLE = reinterpret_cast<R*>(smem) + G::kHead;
+  R* sLX = sLE + NP;
+  R* sLY = sLX + NP;
+  R* sP = sLY + NP;      // psi adjoints of Ez (x, y), Hx, Hy: sP + k * NP
+  R* sW1 = sP + 4 * NP;  // curl weights of the H half: Hx
+  R* sW2 = sW1 + NP;     //   and Hy
+  R* sV1 = sW2 + NP;     // curl weights of the E half: Ez's first
+  R* sV2 = sV1 + NP;     //   and its second
+  const TbBlock blk(t);
+  const int c = threadIdx.x % RJ, ty = threadIdx.x / RJ, b = blk.b;
+  const int ri0 = blk.row * TI - H, rj0 = blk.col * TJ - H;
   const int j = wrap_index(rj0 + c, t.ny);
   const bool jtile = c >= H && c < H + TJ && rj0 + c < t.ny;
   const int64_t base = (int64_t)b * t.plane;
   const int wb = rb ^ 1;
   int li[Q];
-  TbPoint pt[Q];
+  TbPoint<R> pt[Q];
   unsigned fl[Q];
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
-    const int a = ty + kTbRows * q, k = a * RJ + c;
+    const int a = ty + kRowsAtOnce * q, k = a * RJ + c;
     li[q] = wrap_index(ri0 + a, t.nx);
-    fl[q] = tb_point(t, b, li[q], j, pt[q]);
+    fl[q] = tb_point<P>(t, b, li[q], j, pt[q]);
     if (jtile && a >= H && a < H + TI && ri0 + a < t.nx) fl[q] |= 1u << 31;  // tile point
     const int64_t lin = base + (int64_t)li[q] * t.ny + j;
-    sLE[k] = static_cast<const float*>(t.l[0])[lin];
-    sLX[k] = static_cast<const float*>(t.l[1])[lin];
-    sLY[k] = static_cast<const float*>(t.l[2])[lin];
+    sLE[k] = static_cast<const T*>(t.l[0])[lin];
+    sLX[k] = static_cast<const T*>(t.l[1])[lin];
+    sLY[k] = static_cast<const T*>(t.l[2])[lin];
     if (fl[q] & kTmzPsiE) {
-      sP[k] = static_cast<const float*>(t.phi[rb][0])[lin];
-      sP[NP + k] = static_cast<const float*>(t.phi[rb][1])[lin];
+      sP[k] = static_cast<const T*>(t.phi[rb][0])[lin];
+      sP[NP + k] = static_cast<const T*>(t.phi[rb][1])[lin];
     }
-    if (fl[q] & kTmzPsiX) sP[2 * NP + k] = static_cast<const float*>(t.phi[rb][2])[lin];
-    if (fl[q] & kTmzPsiY) sP[3 * NP + k] = static_cast<const float*>(t.phi[rb][3])[lin];
+    if (fl[q] & kTmzPsiX) sP[2 * NP + k] = static_cast<const T*>(t.phi[rb][2])[lin];
+    if (fl[q] & kTmzPsiY) sP[3 * NP + k] = static_cast<const T*>(t.phi[rb][3])[lin];
   }
   unsigned any = 0;
 #pragma unroll
@@ -888,22 +1521,22 @@ __global__ void __launch_bounds__(kTbThreads, kTbMinBlocks)
   auto steps = [&](auto tag) {
     constexpr bool PSI = decltype(tag)::value;
     auto hw = [&](int q) {
-      const int k = (ty + kTbRows * q) * RJ + c;
+      const int k = (ty + kRowsAtOnce * q) * RJ + c;
       sW1[k] = (fl[q] & kTmzPlainX) ? pt[q].cxn * sLX[k]
                : (PSI && (fl[q] & kTmzPsiX))
                    ? adjx_cpml<P, true>(g, fl[q], pt[q].cxn, j, sLX[k], sP + 2 * NP + k,
                                         sP + 2 * NP + k)
-                   : 0.f;
+                   : P::zero();
       sW2[k] = (fl[q] & kTmzPlainY) ? pt[q].cy * sLY[k]
                : (PSI && (fl[q] & kTmzPsiY))
                    ? adjy_cpml<P, true>(g, fl[q], pt[q].cy, li[q], sLY[k], sP + 3 * NP + k,
                                         sP + 3 * NP + k)
-                   : 0.f;
+                   : P::zero();
     };
     auto eu = [&](int q, int n) {
-      const int a = ty + kTbRows * q, k = a * RJ + c;
+      const int a = ty + kRowsAtOnce * q, k = a * RJ + c;
       if (a >= 1 && c >= 1) {
-        float le = sLE[k];
+        R le = sLE[k];
         if (fl[q] & kTmzMonitor) {
           bool has;
           le = le + P::from_double(seed_of(g, t, b, li[q], j, n, &has));
@@ -912,14 +1545,14 @@ __global__ void __launch_bounds__(kTbThreads, kTbMinBlocks)
       }
     };
     auto ew = [&](int q, int n) {
-      const int k = (ty + kTbRows * q) * RJ + c;
-      float w1, w2;
+      const int k = (ty + kRowsAtOnce * q) * RJ + c;
+      R w1, w2;
       if (fl[q] & kTmzPlainE) {
-        const float le = sLE[k];
+        const R le = sLE[k];
         w1 = pt[q].c1 * le;
         w2 = pt[q].c2n * le;
       } else {
-        w1 = w2 = 0.f;
+        w1 = w2 = P::zero();
         if (PSI && (fl[q] & kTmzPsiE))
           adje_cpml<P, true, true, true>(g, fl[q], pt[q].c1, li[q], j, sLE[k], sP + k, sP + k,
                                          sP + NP + k, sP + NP + k, w1, w2);
@@ -928,21 +1561,21 @@ __global__ void __launch_bounds__(kTbThreads, kTbMinBlocks)
       sV2[k] = w2;
       if ((fl[q] & kTmzDesign) && (fl[q] >> 31)) {
         const int64_t kk = (int64_t)b * nd + design_index(t, li[q], j);
-        const double le = (double)sLE[k];
-        const double inc = (double)static_cast<const float*>(
-            t.hist)[((int64_t)(n - step0 - 1) * t.nb + b) * nd + (kk - (int64_t)b * nd)];
+        const double le = to_double(sLE[k]);
+        const double inc = to_double(static_cast<const T*>(
+            t.hist)[((int64_t)(n - step0 - 1) * t.nb + b) * nd + (kk - (int64_t)b * nd)]);
         t.grad[kk] += le * inc * t.dc[kk].neg_reps;
       }
     };
     auto xu = [&](int q) {
-      const int a = ty + kTbRows * q, k = a * RJ + c;
+      const int a = ty + kRowsAtOnce * q, k = a * RJ + c;
       if (a < RI - 1 && c < RJ - 1) {
         sLX[k] = sLX[k] + (sV2[k] - sV2[k + 1]);
         sLY[k] = sLY[k] + (sV1[k] - sV1[k + RJ]);
       }
     };
     if (src_h) {
-      tb_sources<true>(t, 1, n0 + nsub, ri0, rj0, RI, RJ, sLE, sLX, sLY);
+      tb_sources<P, true>(t, 1, n0 + nsub, ri0, rj0, RI, RJ, sLE, sLX, sLY);
       __syncthreads();
     }
   #pragma unroll
@@ -954,7 +1587,7 @@ __global__ void __launch_bounds__(kTbThreads, kTbMinBlocks)
       for (int q = 0; q < Q; ++q) eu(q, n);
       if (src_e) {
         __syncthreads();
-        tb_sources<true>(t, 0, n, ri0, rj0, RI, RJ, sLE, sLX, sLY);
+        tb_sources<P, true>(t, 0, n, ri0, rj0, RI, RJ, sLE, sLX, sLY);
         __syncthreads();
       }
   #pragma unroll
@@ -965,7 +1598,7 @@ __global__ void __launch_bounds__(kTbThreads, kTbMinBlocks)
       if (s > 0) {
         if (src_h) {
           __syncthreads();
-          tb_sources<true>(t, 1, n - 1, ri0, rj0, RI, RJ, sLE, sLX, sLY);
+          tb_sources<P, true>(t, 1, n - 1, ri0, rj0, RI, RJ, sLE, sLX, sLY);
           __syncthreads();
         }
   #pragma unroll
@@ -975,44 +1608,423 @@ __global__ void __launch_bounds__(kTbThreads, kTbMinBlocks)
     }
   };
   if (psi_any)
-    steps(PsiTag<true>{});
+    steps(BoolTag<true>{});
   else
-    steps(PsiTag<false>{});
+    steps(BoolTag<false>{});
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     if (!(fl[q] >> 31)) continue;
-    const int k = (ty + kTbRows * q) * RJ + c;
+    const int k = (ty + kRowsAtOnce * q) * RJ + c;
     const int64_t lin = base + (int64_t)li[q] * t.ny + j;
-    static_cast<float*>(t.tmp[0])[lin] = sLE[k];
-    static_cast<float*>(t.tmp[1])[lin] = sLX[k];
-    static_cast<float*>(t.tmp[2])[lin] = sLY[k];
+    static_cast<T*>(t.tmp[0])[lin] = sLE[k];
+    static_cast<T*>(t.tmp[1])[lin] = sLX[k];
+    static_cast<T*>(t.tmp[2])[lin] = sLY[k];
     if (fl[q] & kTmzPsiE) {
-      static_cast<float*>(t.phi[wb][0])[lin] = sP[k];
-      static_cast<float*>(t.phi[wb][1])[lin] = sP[NP + k];
+      static_cast<T*>(t.phi[wb][0])[lin] = sP[k];
+      static_cast<T*>(t.phi[wb][1])[lin] = sP[NP + k];
     }
-    if (fl[q] & kTmzPsiX) static_cast<float*>(t.phi[wb][2])[lin] = sP[2 * NP + k];
-    if (fl[q] & kTmzPsiY) static_cast<float*>(t.phi[wb][3])[lin] = sP[3 * NP + k];
+    if (fl[q] & kTmzPsiX) static_cast<T*>(t.phi[wb][2])[lin] = sP[2 * NP + k];
+    if (fl[q] & kTmzPsiY) static_cast<T*>(t.phi[wb][3])[lin] = sP[3 * NP + k];
   }
 }
 
-// Region of both blocked kernels: 32 x 64 points; forward 7 arrays (56 KB),
-// adjoint 11 arrays (88 KB) of shared memory.  (Adjoint measured on GB300,
-// 512^2 x 64 designs, 2000 steps: 9 arrays and four barriers per step
-// 0.3168 s, 11 arrays and two barriers 0.3147 s, and with each design
-// pixel's gradient summed in shared memory over a launch, 104 KB, 0.3266 s;
-// a thread's own curl weights kept in registers from the pass that forms
-// them to the pass that gathers them, four fewer shared-memory loads per
-// point and step but spilling at 64 registers: 0.352 s, the E half's alone
-// 0.328 s, against 0.316 s.)
-constexpr int kTbFwdRI = kTbRI, kTbAdjRI = kTbRI;
-constexpr size_t kTbFwdSmem = (size_t)7 * kTbFwdRI * kTbRJ * sizeof(float);
-constexpr size_t kTbAdjSmem = (size_t)11 * kTbAdjRI * kTbRJ * sizeof(float);
+// Calls steps with the tile's form.
+template <int KIND, bool FANCY>
+struct TbForm {
+  static constexpr int kind = KIND;
+  static constexpr bool fancy = FANCY;
+};
+template <bool ADJ, class R, class F>
+__device__ __forceinline__ void tb_dispatch(const TbTile<R>& tile, F& steps) {
+  if (tile.kind == kTbRows)
+    steps(TbForm<kTbRows, false>{});
+  else if (tile.kind == kTbCols)
+    steps(TbForm<kTbCols, false>{});
+  else if (tile.kind == kTbBoth && (ADJ || !tile.fancy))
+    steps(TbForm<kTbBoth, false>{});
+  else if (tile.kind == kTbBoth)
+    steps(TbForm<kTbBoth, !ADJ>{});
+  else if (tile.fancy)
+    steps(TbForm<kTbPlain, true>{});
+  else
+    steps(TbForm<kTbPlain, false>{});
+}
 
-template <int RI>
-dim3 tb_grid(const TmzDev& t) {
-  using G = TbGeom<RI>;
-  return dim3((unsigned)((t.ny + G::TJ - 1) / G::TJ), (unsigned)((t.nx + G::TI - 1) / G::TI),
-              (unsigned)t.nb);
+// Forward steps n0+1 .. n0+nsub (nsub <= kTbHalo) of one tile, from the
+// state in t.f to the state in t.tmp (the launch's other blocks still read
+// t.f for their halos, so the result must not overwrite it).  slot0 >= 0:
+// record the design increments of step n0+1+s at hist slot slot0+s;
+// rec_mon: record monitor row n-1 of every step n.
+template <class P, int Q>
+__global__ void __launch_bounds__(kTbThreads, 2)
+    k_tmz_tb_fwd(const GridDev g, const TmzDev t, int n0, int nsub, int slot0, int rec_mon) {
+  using R = typename P::R;
+  using G = TbGeom<P, Q>;
+  using Two = Row2<R>;
+  extern __shared__ __align__(16) unsigned char tb_smem[];
+  const TbTile<R> tile =
+      static_cast<const TbTile<R>*>(t.tiles)[TbBlock(t).tile];
+  if (tile.kind == kTbGeneral) {
+    tb_general_fwd<P, Q>(g, t, n0, nsub, slot0, rec_mon, tb_smem);
+    return;
+  }
+  // rows left by the warps: sU slot w + 1 the last row of Hy of warp w, sD
+  // slot w the first row of Ez of warp w; slots 0 / kTbWarps: beyond the region
+  Two* const sU = reinterpret_cast<Two*>(tb_smem);
+  Two* const sD = sU + (kTbWarps + 1) * kTbRJ / 2;
+  R* const sR = reinterpret_cast<R*>(tb_smem) + G::kRows;  // layer rows' entries: Ez, Hy
+  const TbPlace<P, Q> p(t);
+  const int lane = p.lane, w = p.warp;
+  R e[Q][2], x[Q][2], y[Q][2];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    p.load(t, t.f[0], q, e[q]);
+    p.load(t, t.f[1], q, x[q]);
+    p.load(t, t.f[2], q, y[q]);
+  }
+  if (w == 0) sU[lane] = Two{P::zero(), P::zero()};
+  if (w == kTbWarps - 1) sD[kTbWarps * 32 + lane] = Two{P::zero(), P::zero()};
+  sU[(w + 1) * 32 + lane] = Two{y[Q - 1][0], y[Q - 1][1]};
+  constexpr unsigned kAll = 0xffffffffu;
+  const R cxn = tile.c[2], cy = tile.c[3], de = tile.d[0], dx = tile.d[1], dy = tile.d[2];
+  const bool design = slot0 >= 0 && (tile.any & kTmzDesign);
+  const bool src = tile.any & kTmzSrcE, mon = rec_mon && (tile.any & kTmzMonitor);
+  auto steps = [&](auto form) {
+    constexpr int KIND = decltype(form)::kind;
+    constexpr bool LAYER = KIND != kTbPlain, SP = decltype(form)::fancy;
+    TbCoef<P, Q, SP> cf;
+    TbLayer<P, Q, KIND> L;
+    TbSpecial<P, Q> sp;
+    cf.load(t, p);
+    if constexpr (SP) {
+      sp.init(tb_smem);
+      sp.load(t, p, tile);
+      if (src) sp.fetch(t, p, n0 + 1);
+    }
+    if constexpr (LAYER) {
+      L.load(t, p, t.f + 3);
+      L.fill(g, t, p, tile, sR);
+    }
+    __syncthreads();
+    if constexpr (LAYER) L.columns(sR, lane);
+    for (int s = 0; s < nsub; ++s) {
+      const int n = n0 + s + 1;
+      const Two up = sU[w * 32 + lane];
+      R u[2] = {up.a, up.b};
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const R xl = __shfl_up_sync(kAll, x[q][1], 1);
+        const R D2[2] = {x[q][0] - xl, x[q][1] - x[q][0]};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const R D1 = y[q][h] - u[h];
+          u[h] = y[q][h];
+          R c1, c2n;
+          cf.get(tile, q, h, c1, c2n);
+          if constexpr (SP)
+            if (design && (sp.row[q] & kTmzDesign))
+              sp.record(t, p, q, h, slot0 + s, c1, c2n, D1, D2[h]);
+          if constexpr (LAYER)
+            e[q][h] = L.e_fwd(sR, w * Q + q, q, h, e[q][h], c1, c2n, SP ? c1 : de, D1, D2[h]);
+          else
+            e[q][h] = fmadd(fmadd(e[q][h], c1, D1), c2n, D2[h]);
+        }
+        if constexpr (SP)
+          if (src) sp.source(p, q, e[q]);
+      }
+      if constexpr (SP)
+        if (src && s + 1 < nsub) sp.fetch(t, p, n + 1);
+      sD[w * 32 + lane] = Two{e[0][0], e[0][1]};
+      __syncthreads();
+      const Two dn = sD[(w + 1) * 32 + lane];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const R er = __shfl_down_sync(kAll, e[q][0], 1);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const R below = q + 1 < Q ? e[q + 1 < Q ? q + 1 : q][h] : (h ? dn.b : dn.a);
+          const R D1 = (h ? er : e[q][1]) - e[q][h], D2 = below - e[q][h];
+          if constexpr (LAYER) {
+            x[q][h] = L.x_fwd(q, h, x[q][h], cxn, dx, D1);
+            y[q][h] = L.y_fwd(sR, w * Q + q, q, h, y[q][h], cy, dy, D2);
+          } else {
+            x[q][h] = fmadd(x[q][h], cxn, D1);
+            y[q][h] = fmadd(y[q][h], cy, D2);
+          }
+        }
+        if constexpr (SP)
+          if (mon) sp.monitor(t, p, q, n, e[q]);
+      }
+      sU[(w + 1) * 32 + lane] = Two{y[Q - 1][0], y[Q - 1][1]};
+      __syncthreads();
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      if (!p.row_in_tile(t, q)) continue;
+      p.store(t, t.tmp[0], q, e[q]);
+      p.store(t, t.tmp[1], q, x[q]);
+      p.store(t, t.tmp[2], q, y[q]);
+    }
+    if constexpr (LAYER) L.store(t, p, t.tmp + 3);
+  };
+  tb_dispatch<false>(tile, steps);
+}
+
+// Adjoint steps n0 + nsub down to n0 + 1 of one tile (the transposes of
+// k_tmz_ah / k_tmz_ae, same order), the field adjoints from t.l to
+// t.tmp[0..2]; the gradient of step n uses hist slot n - step0 - 1.  The
+// psi adjoints are read from buffer rb and written to the other one, so no
+// block overwrites what another still reads (adjoint_blocked chooses rb so
+// that a call leaves them where the one-step kernels' step-parity
+// convention expects them).
+//
+// Per step: H-side sources, the curl weights w1, w2 of every Hx / Hy point,
+// lambda_E gathering them, E-side sources, the curl weights v1, v2 of every Ez
+// point and the gradient, lambda_X / lambda_Y gathering those.  The weights of
+// the neighbour along j come by a shuffle, those along i from the lane or the
+// next warp's row (w2 of its last row, v1 of its first).
+template <class P, int Q>
+__global__ void __launch_bounds__(kTbThreads, 2)
+    k_tmz_tb_adj(const GridDev g, const TmzDev t, int n0, int nsub, int step0, int rb) {
+  using R = typename P::R;
+  using G = TbGeom<P, Q>;
+  using Two = Row2<R>;
+  extern __shared__ __align__(16) unsigned char tb_smem[];
+  const TbTile<R> tile =
+      static_cast<const TbTile<R>*>(t.tiles)[TbBlock(t).tile];
+  // (an absorbing tile with sources, monitor or design pixels takes the
+  // general form here: 22 us per launch of a 128 x 123 lattice against 36 in
+  // registers, which spill)
+  if (tile.kind == kTbGeneral || (tile.kind == kTbBoth && tile.fancy)) {
+    tb_general_adj<P, Q>(g, t, n0, nsub, step0, rb, tb_smem);
+    return;
+  }
+  Two* const sU = reinterpret_cast<Two*>(tb_smem);        // w2 of the last rows
+  Two* const sD = sU + (kTbWarps + 1) * kTbRJ / 2;        // v1 of the first rows
+  R* const sR = reinterpret_cast<R*>(tb_smem) + G::kRows;
+  const TbPlace<P, Q> p(t);
+  const int lane = p.lane, w = p.warp;
+  R e[Q][2], x[Q][2], y[Q][2];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    p.load(t, t.l[0], q, e[q]);
+    p.load(t, t.l[1], q, x[q]);
+    p.load(t, t.l[2], q, y[q]);
+  }
+  if (w == 0) sU[lane] = Two{P::zero(), P::zero()};
+  if (w == kTbWarps - 1) sD[kTbWarps * 32 + lane] = Two{P::zero(), P::zero()};
+  constexpr unsigned kAll = 0xffffffffu;
+  const R cxn = tile.c[2], cy = tile.c[3], de = tile.d[0], dx = tile.d[1], dy = tile.d[2];
+  const bool design = tile.any & kTmzDesign, mon = tile.any & kTmzMonitor;
+  const bool src = tile.any & kTmzSrcE;
+  auto steps = [&](auto form) {
+    constexpr int KIND = decltype(form)::kind;
+    constexpr bool LAYER = KIND != kTbPlain, SP = decltype(form)::fancy;
+    TbCoef<P, Q, SP> cf;
+    TbLayer<P, Q, KIND> L;
+    TbSpecial<P, Q> sp;
+    cf.load(t, p);
+    if constexpr (SP) {
+      sp.init(tb_smem);
+      sp.load(t, p, tile);
+      if (design) sp.grad_load(t, p);
+    }
+    if constexpr (LAYER) {
+      L.load(t, p, t.phi[rb]);
+      L.fill(g, t, p, tile, sR);
+      __syncthreads();
+      L.columns(sR, lane);
+    }
+    // w2 of every point (a layer row's advance its psi adjoint)
+    R ya[Q][2];
+    auto hside = [&]() {
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if constexpr (LAYER)
+            ya[q][h] = L.y_adj(sR, w * Q + q, q, h, y[q][h], cy, dy);
+          else
+            ya[q][h] = cy * y[q][h];
+        }
+      sU[(w + 1) * 32 + lane] = Two{ya[Q - 1][0], ya[Q - 1][1]};
+    };
+    hside();
+    __syncthreads();
+    for (int s = nsub - 1; s >= 0; --s) {
+      const int n = n0 + s + 1;
+      if constexpr (SP)
+        if (design) sp.grad_fetch(t, p, n - step0 - 1);
+      const Two up = sU[w * 32 + lane];
+      R u[2] = {up.a, up.b};
+      R v1[Q][2], v2[Q][2];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        R wx[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if constexpr (LAYER)
+            wx[h] = L.x_adj(q, h, x[q][h], cxn, dx);
+          else
+            wx[h] = cxn * x[q][h];
+        }
+        const R wl = __shfl_up_sync(kAll, wx[1], 1);
+        if constexpr (SP)
+          if (mon) sp.seed(g, t, p, q, n, e[q]);
+        e[q][0] = e[q][0] + ((wl - wx[0]) + (u[0] - ya[q][0]));
+        e[q][1] = e[q][1] + ((wx[0] - wx[1]) + (u[1] - ya[q][1]));
+        u[0] = ya[q][0];
+        u[1] = ya[q][1];
+        if constexpr (SP)
+          if (src) sp.zero(p, q, e[q]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          R c1, c2n;
+          cf.get(tile, q, h, c1, c2n);
+          if constexpr (LAYER) {
+            L.e_adj(sR, w * Q + q, q, h, e[q][h], c1, c2n, SP ? c1 : de, v1[q][h], v2[q][h]);
+          } else {
+            v1[q][h] = c1 * e[q][h];
+            v2[q][h] = c2n * e[q][h];
+          }
+        }
+        if constexpr (SP)
+          if (design) sp.grad_add(t, p, q, e[q]);
+      }
+      sD[w * 32 + lane] = Two{v1[0][0], v1[0][1]};
+      __syncthreads();
+      const Two dn = sD[(w + 1) * 32 + lane];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const R vr = __shfl_down_sync(kAll, v2[q][0], 1);
+        const R d0 = q + 1 < Q ? v1[q + 1 < Q ? q + 1 : q][0] : dn.a;
+        const R d1 = q + 1 < Q ? v1[q + 1 < Q ? q + 1 : q][1] : dn.b;
+        x[q][0] = x[q][0] + (v2[q][0] - v2[q][1]);
+        x[q][1] = x[q][1] + (v2[q][1] - vr);
+        y[q][0] = y[q][0] + (v1[q][0] - d0);
+        y[q][1] = y[q][1] + (v1[q][1] - d1);
+      }
+      if (s > 0) hside();
+      __syncthreads();
+    }
+    if constexpr (SP)
+      if (design) sp.grad_store(t, p);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      if (!p.row_in_tile(t, q)) continue;
+      p.store(t, t.tmp[0], q, e[q]);
+      p.store(t, t.tmp[1], q, x[q]);
+      p.store(t, t.tmp[2], q, y[q]);
+    }
+    if constexpr (LAYER) L.store(t, p, t.phi[rb ^ 1]);
+  };
+  tb_dispatch<true>(tile, steps);
+}
+
+// What each tile is (TbTile), one block per tile; after k_tmz_map.
+template <class P, int Q>
+__global__ void __launch_bounds__(kTbThreads) k_tmz_tiles(const TmzDev t) {
+  using R = typename P::R;
+  using G = TbGeom<P, Q>;
+  constexpr unsigned plain = kTmzPlainE | kTmzPlainX | kTmzPlainY;
+  constexpr unsigned rowbits = kTmzOnE1 | kTmzOnY, colbits = kTmzOnE2 | kTmzOnX;
+  constexpr unsigned layer = rowbits | colbits | kTmzPsiE | kTmzPsiX | kTmzPsiY;
+  constexpr unsigned pmbits = 3u << kTmzPmlE | 3u << kTmzPmlX | 3u << kTmzPmlY;
+  __shared__ unsigned any_s;
+  __shared__ int same_s, vary_s, first_s[7], pm_s;
+  if (threadIdx.x == 0) {
+    any_s = 0;
+    same_s = 1;
+    vary_s = 0;
+    pm_s = -1;
+    for (int k = 0; k < 7; ++k) first_s[k] = -1;
+  }
+  __syncthreads();
+  const int cols = (t.ny + kTbTJ - 1) / kTbTJ;
+  const int ri0 = (int)blockIdx.x / cols * G::TI - kTbHalo;
+  const int rj0 = (int)blockIdx.x % cols * kTbTJ - kTbHalo;
+  auto at = [&](int a, int c) {
+    return (int64_t)wrap_index(ri0 + a, t.nx) * t.ny + wrap_index(rj0 + c, t.ny);
+  };
+  // coefficient k of a point, one of: plain c1, c2n, cx, cy; absorbing cdt of
+  // Ez, Hx, Hy
+  auto holds = [&](unsigned f, int k) {
+    constexpr unsigned bit[7] = {kTmzPlainE, kTmzPlainE, kTmzPlainX, kTmzPlainY,
+                                 kTmzPsiE,   kTmzPsiX,   kTmzPsiY};
+    return (f & bit[k]) != 0;
+  };
+  auto coef = [&](int64_t ll, int k) {
+    return P::ld(map_coef<P>(t, k < 4 ? k : (k == 4 ? 0 : k - 3)) + ll);
+  };
+  unsigned any = 0;
+  int first[7] = {-1, -1, -1, -1, -1, -1, -1}, pm_any = -1;
+  for (int q = threadIdx.x; q < G::NP; q += kTbThreads) {
+    const unsigned f = __ldg(t.pflags + at(q / kTbRJ, q % kTbRJ));
+    any |= f;
+    for (int k = 0; k < 7; ++k)
+      if (holds(f, k)) first[k] = q;  // any point that has one will do
+    if (f & kTmzPsiE) pm_any = f >> kTmzPmlE & 3;
+    if (f & kTmzPsiX) pm_any = f >> kTmzPmlX & 3;
+    if (f & kTmzPsiY) pm_any = f >> kTmzPmlY & 3;
+  }
+  any = __reduce_or_sync(0xffffffffu, any);
+  pm_any = __reduce_max_sync(0xffffffffu, pm_any);
+  for (int k = 0; k < 7; ++k) first[k] = __reduce_max_sync(0xffffffffu, first[k]);
+  if ((threadIdx.x & 31) == 0) {
+    atomicOr(&any_s, any);
+    atomicMax(&pm_s, pm_any);
+    for (int k = 0; k < 7; ++k) atomicMax(&first_s[k], first[k]);
+  }
+  __syncthreads();
+  R c[7];
+  for (int k = 0; k < 7; ++k)
+    c[k] = first_s[k] < 0 ? P::zero() : coef(at(first_s[k] / kTbRJ, first_s[k] % kTbRJ), k);
+  const unsigned pm = pm_s < 0 ? 0u : (unsigned)pm_s;
+  constexpr unsigned specials = kTmzSrcE | kTmzMonitor | kTmzDesign;
+  bool same = (any_s & ~(plain | layer | pmbits | specials)) == 0, even = true;
+  for (int q = threadIdx.x; q < G::NP && same; q += kTbThreads) {
+    const int a = q / kTbRJ, cc = q % kTbRJ;
+    const int64_t ll = at(a, cc);
+    const unsigned f = __ldg(t.pflags + ll) & ~specials;
+    const unsigned row = __ldg(t.pflags + at(a, 0)), col = __ldg(t.pflags + at(0, cc));
+    // absorbing exactly where the row or the column is on, plain elsewhere
+    const unsigned on = (row & rowbits) | (col & colbits);
+    unsigned want = on;
+    want |= (on & (kTmzOnE1 | kTmzOnE2)) ? kTmzPsiE | pm << kTmzPmlE : kTmzPlainE;
+    want |= (on & kTmzOnX) ? kTmzPsiX | pm << kTmzPmlX : kTmzPlainX;
+    want |= (on & kTmzOnY) ? kTmzPsiY | pm << kTmzPmlY : kTmzPlainY;
+    same = f == want;
+    for (int k = 0; k < 7; ++k)
+      if (holds(f, k) && coef(ll, k) != c[k]) {
+        if (k < 2 || k == 4)
+          even = false;  // Ez
+        else
+          same = false;
+      }
+  }
+  if (!same) same_s = 0;
+  if (!even || (any_s & kTmzDesign)) vary_s = 1;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    TbTile<R> o;
+    o.any = any_s;
+    const bool rows = any_s & rowbits, cols = any_s & colbits;
+    o.fancy = vary_s || (any_s & specials);
+    o.kind = rows ? (cols ? kTbBoth : kTbRows) : (cols ? kTbCols : kTbPlain);
+    if (o.kind != kTbPlain && o.fancy) o.kind = kTbBoth;  // one form for these
+    if (!same_s) o.kind = kTbGeneral;
+    o.pm = (int)pm;
+    for (int k = 0; k < 4; ++k) o.c[k] = c[k];
+    for (int k = 0; k < 3; ++k) o.d[k] = c[4 + k];
+    o.e = P::zero();
+    static_cast<TbTile<R>*>(t.tiles)[blockIdx.x] = o;
+  }
+}
+
+template <class P, int Q>
+unsigned tb_tiles(const TmzDev& t) {
+  using G = TbGeom<P, Q>;
+  return (unsigned)((t.ny + kTbTJ - 1) / kTbTJ) * (unsigned)((t.nx + G::TI - 1) / G::TI);
 }
 
 // ---------------------------------------------------------------------------
@@ -1118,24 +2130,31 @@ cudaError_t copy_state(void* const* dst, void* const* src, int n, int64_t bytes,
   return cudaSuccess;
 }
 
+// Rows per warp of the blocked kernels: regions of 32 x 64 points.  Measured on
+// GB300 (512^2 x 64 designs, 200 steps, forward / adjoint ms, 512 threads at 64
+// registers): 2 rows 12.8 / 16.2, 3 rows 12.1 / 21.8 (the adjoint spills); 256
+// threads at 128 registers, 4 rows 15.9 / 18.0, 6 rows 17.2 / 30.0.
+constexpr int kTbQ = 2;
+
+template <class P, int Q>
 cudaError_t forward_blocked(const GridDev& g, const TmzDev& t, int step0, int nsteps, int flags,
                             int per_launch, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(k_tmz_tb_fwd<kTbFwdRI>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)kTbFwdSmem);
+  constexpr size_t smem = TbGeom<P, Q>::fwd_bytes;
+  cudaError_t e = cudaFuncSetAttribute(k_tmz_tb_fwd<P, Q>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   if (t.tmp[0] == nullptr) return cudaErrorInvalidValue;
-  const dim3 grid = tb_grid<kTbFwdRI>(t), block(kTbRJ, kTbRows);
+  const unsigned grid = tb_tiles<P, Q>(t) * (unsigned)t.nb;
   const int launches = (nsteps + per_launch - 1) / per_launch;
   TmzDev u = t;
   if (launches % 2 == 1) {
-    e = copy_state(t.tmp, t.f, kTmzState, (int64_t)t.nb * t.plane * (int64_t)sizeof(float), s);
+    e = copy_state(t.tmp, t.f, kTmzState, (int64_t)t.nb * t.plane * (int64_t)sizeof(typename P::T), s);
     if (e != cudaSuccess) return e;
     swap_fields(u);
   }
   for (int k = 0; k < nsteps; k += per_launch) {
     const int m = nsteps - k < per_launch ? nsteps - k : per_launch;
-    k_tmz_tb_fwd<kTbFwdRI><<<grid, block, kTbFwdSmem, s>>>(
+    k_tmz_tb_fwd<P, Q><<<grid, kTbThreads, smem, s>>>(
         g, u, step0 + k, m, (flags & GMES_TMZ_RECORD_HIST) ? k : -1,
         (flags & GMES_TMZ_RECORD_MONITOR) ? 1 : 0);
     swap_fields(u);
@@ -1157,19 +2176,20 @@ int adj_launches(int nsteps, int per_launch) {
   return k < nsteps ? k : nsteps;
 }
 
+template <class P, int Q>
 cudaError_t adjoint_blocked(const GridDev& g, const TmzDev& t, int step0, int nsteps,
                             int per_launch, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(k_tmz_tb_adj<kTbAdjRI>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)kTbAdjSmem);
+  constexpr size_t smem = TbGeom<P, Q>::adj_bytes;
+  cudaError_t e = cudaFuncSetAttribute(k_tmz_tb_adj<P, Q>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   if (t.tmp[0] == nullptr) return cudaErrorInvalidValue;
   if (nsteps <= 0) return cudaSuccess;
-  const dim3 grid = tb_grid<kTbAdjRI>(t), block(kTbRJ, kTbRows);
+  const unsigned grid = tb_tiles<P, Q>(t) * (unsigned)t.nb;
   const int launches = adj_launches(nsteps, per_launch);
   TmzDev u = t;
   if (launches % 2 == 1) {
-    e = copy_state(t.tmp, t.l, 3, (int64_t)t.nb * t.plane * (int64_t)sizeof(float), s);
+    e = copy_state(t.tmp, t.l, 3, (int64_t)t.nb * t.plane * (int64_t)sizeof(typename P::T), s);
     if (e != cudaSuccess) return e;
     swap_adjoints(u);
   }
@@ -1178,7 +2198,7 @@ cudaError_t adjoint_blocked(const GridDev& g, const TmzDev& t, int step0, int ns
   for (int q = 0; q < launches; ++q) {
     // launch q takes an even share of the steps left
     const int m = (hi + (launches - q) - 1) / (launches - q);
-    k_tmz_tb_adj<kTbAdjRI><<<grid, block, kTbAdjSmem, s>>>(g, u, step0 + hi - m, m, step0, rb);
+    k_tmz_tb_adj<P, Q><<<grid, kTbThreads, smem, s>>>(g, u, step0 + hi - m, m, step0, rb);
     swap_adjoints(u);
     rb ^= 1;
     hi -= m;
@@ -1187,8 +2207,9 @@ cudaError_t adjoint_blocked(const GridDev& g, const TmzDev& t, int step0, int ns
 }
 
 // Steps per launch for a precision and the caller's request (0: default).
-int steps_per_launch(int precision, int requested) {
-  if (precision != GMES_FP32) return 1;
+// (The blocked kernels' source maps hold 15-bit source numbers.)
+int steps_per_launch(int precision, const TmzDev& t, int requested) {
+  if (precision != GMES_FP32 || t.nsrc >= (int)kTbHard - 1) return 1;
   if (requested <= 0) return kTbHalo;
   return requested < kTbHalo ? requested : kTbHalo;
 }
@@ -1214,17 +2235,20 @@ cudaError_t launch_tmz_design(int precision, const GridDev& g, const TmzDev& t,
       return cudaErrorInvalidValue;
   }
   if (t.nsrc > 0) k_tmz_map_sources<<<(t.nsrc + 127) / 128, 128, 0, s>>>(t);
+  if (precision == GMES_FP32 && t.tmp[0] != nullptr)
+    k_tmz_tiles<PolF32, kTbQ><<<tb_tiles<PolF32, kTbQ>(t), kTbThreads, 0, s>>>(t);
   return cudaGetLastError();
 }
 
 cudaError_t launch_tmz_forward(int precision, const GridDev& g, const TmzDev& t, int step0,
                                int nsteps, int flags, int block_steps, cudaStream_t s) {
-  const int per = steps_per_launch(precision, block_steps);
+  const int per = steps_per_launch(precision, t, block_steps);
   switch (precision) {
     case GMES_FP64:
       return forward<PolF64>(g, t, step0, nsteps, flags, s);
     case GMES_FP32:
-      if (per > 1) return forward_blocked(g, t, step0, nsteps, flags, per, s);
+      if (per > 1)
+        return forward_blocked<PolF32, kTbQ>(g, t, step0, nsteps, flags, per, s);
       return forward<PolF32>(g, t, step0, nsteps, flags, s);
     case GMES_DF64:
       return forward<PolDF>(g, t, step0, nsteps, flags, s);
@@ -1235,12 +2259,13 @@ cudaError_t launch_tmz_forward(int precision, const GridDev& g, const TmzDev& t,
 
 cudaError_t launch_tmz_adjoint(int precision, const GridDev& g, const TmzDev& t, int step0,
                                int nsteps, int block_steps, cudaStream_t s) {
-  const int per = steps_per_launch(precision, block_steps);
+  const int per = steps_per_launch(precision, t, block_steps);
   switch (precision) {
     case GMES_FP64:
       return adjoint<PolF64>(g, t, step0, nsteps, s);
     case GMES_FP32:
-      if (per > 1) return adjoint_blocked(g, t, step0, nsteps, per, s);
+      if (per > 1)
+        return adjoint_blocked<PolF32, kTbQ>(g, t, step0, nsteps, per, s);
       return adjoint<PolF32>(g, t, step0, nsteps, s);
     case GMES_DF64:
       return adjoint<PolDF>(g, t, step0, nsteps, s);

@@ -952,8 +952,8 @@ struct TmzLayout {
   int64_t array;  // bytes of one [nb][nx][ny] array, 256-aligned
   int64_t state, adjoint, design, hist, monitor, grad, scratch;
   // the design buffer: per-pixel coefficients, then the lattice map's
-  // flags and its four coefficient arrays
-  int64_t design_coef, map_flags, map_coef;
+  // flags and its four coefficient arrays, and the blocked kernels' tiles
+  int64_t design_coef, map_flags, map_coef, tiles;
 };
 
 // Whether the FP32 forward and adjoint run the temporally blocked kernels,
@@ -974,7 +974,11 @@ TmzLayout tmz_layout(const gmes_grid_desc& g, const gmes_tmz_batch& b) {
   L.design_coef = align256((int64_t)b.nbatch * nd * (int64_t)sizeof(DesignCoef));
   L.map_flags = align256(plane * 4);
   L.map_coef = align256(plane * es);
-  L.design = L.design_coef + L.map_flags + 4 * L.map_coef;
+  // at most one tile per 8 x 8 lattice points, plus the edges
+  L.tiles = tmz_blocked(g, b) ? align256(((int64_t)g.n[0] / 8 + 1) * ((int64_t)g.n[1] / 8 + 1) *
+                                         (int64_t)sizeof(TbTile<double>))
+                              : 0;
+  L.design = L.design_coef + L.map_flags + 4 * L.map_coef + L.tiles;
   L.hist = align256((int64_t)b.hist_steps * b.nbatch * nd * es);
   L.monitor = align256((int64_t)b.nbatch * b.total_steps * nm * 8);
   L.grad = align256((int64_t)b.nbatch * nd * 8);
@@ -1047,6 +1051,8 @@ TmzDev make_tmz_dev(const gmes_grid_desc& g, const gmes_tmz_batch& b) {
   const char* map = static_cast<const char*>(b.design) + L.design_coef;
   t.pflags = reinterpret_cast<const uint32_t*>(map);
   for (int k = 0; k < 4; ++k) t.pcoef[k] = map + L.map_flags + k * L.map_coef;
+  if (tmz_blocked(g, b))
+    t.tiles = static_cast<char*>(b.design) + L.design_coef + L.map_flags + 4 * L.map_coef;
   t.hist = b.hist;
   t.mon = b.monitor;
   t.grad = b.grad;

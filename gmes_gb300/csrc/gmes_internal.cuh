@@ -411,6 +411,7 @@ struct TmzDev {
   // c1, -c2 (Ez), -c1 (Hx), c2 (Hy) as [nx][ny] arrays of the precision's type.
   const uint32_t* pflags;
   const void* pcoef[4];
+  void* tiles;              // TbTile of every tile of the blocked kernels, or null
   void* l[3];
   void* phi[2][4];          // ping-pong buffers of the psi adjoints
   const DesignCoef* dc;     // [nb][nd]
@@ -420,6 +421,23 @@ struct TmzDev {
   const double* weight;     // [nb] or null
   const gmes_point_source* src;
   const double* src_val;    // [total_steps][2][nsrc]
+};
+
+// A tile of the blocked kernels: the flags that its region's points hold
+// between them and what the tile is.  kTbPlain: every point plain; kTbRows,
+// kTbCols, kTbBoth: plain points and, in whole rows, whole columns or both,
+// absorbing points of layer pm that are on along x or y; kTbGeneral: the rest.
+// In all but the last Hx and Hy have one coefficient each (c[2], c[3] plain, d[1], d[2]
+// absorbing) and there are no H sources.  fancy (kTbPlain and kTbBoth, which
+// then stands for rows or columns alone too): Ez's coefficients differ from
+// point to point, or some point carries an Ez source, a monitor or a design
+// pixel; otherwise they are c[0], c[1] plain, d[0] absorbing.
+enum : int32_t { kTbGeneral = 0, kTbPlain = 1, kTbRows = 2, kTbCols = 3, kTbBoth = 4 };
+template <class R>
+struct TbTile {
+  uint32_t any;
+  int32_t kind, pm, fancy;
+  R c[4], d[3], e;
 };
 
 // Flags of the resolved lattice map.  "Plain": the update is
