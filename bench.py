@@ -735,7 +735,7 @@ def run_design(args):
                      "kernel": fwd_kernel, "peak_source": peak[1]},
         "wall_s": round(wall, 3), "grad_finite": bool(torch.isfinite(g).all()),
         "clocks": clocks,
-        "gpu_launches": args.steps * (design_launches(prob, precision, args.block_steps) + 2),
+        "gpu_launches": args.steps * (prob.launches() + 2),
     }
     if not args.no_cpu_baseline:
         result["cpu_baseline"] = design_cpu_baseline(space, geom, src, design, monitor, eps,
@@ -744,9 +744,10 @@ def run_design(args):
 
 
 def design_launches(prob, precision, block_steps, max_block_steps=4):
-    """Kernel launches of one forward + backward.
+    """Kernel launches of one forward + backward, at most.
 
-    One step per launch: E, E sources, H, H sources per step of every pass.
+    One step per launch: four per step of every pass (the library now takes
+    two, or one launch for a whole call; ``TMzAdjoint.launches`` counts them).
     FP32 temporally blocked (block_steps 0 = the library's most, 4): the
     forward takes one launch per block of up to that many steps of each
     call; the adjoint the fewest launches of at most that many steps whose

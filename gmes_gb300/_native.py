@@ -35,7 +35,7 @@ EXPORTS = [
     "gmes_graph_destroy", "gmes_rasterize", "gmes_batch_step_noalloc",
     "gmes_tmz_sizes", "gmes_tmz_check", "gmes_tmz_set_design", "gmes_tmz_reset",
     "gmes_tmz_forward", "gmes_tmz_objective", "gmes_tmz_adjoint", "gmes_points_update",
-    "gmes_copy_async", "gmes_nonfinite", "gmes_step_launches",
+    "gmes_copy_async", "gmes_nonfinite", "gmes_step_launches", "gmes_tmz_launches",
 ]
 NOALLOC_MAX_GRIDS = 64
 
@@ -191,6 +191,7 @@ def load():
     lib.gmes_tmz_set_design.argtypes = [G, B, C.c_void_p, C.c_void_p]
     lib.gmes_tmz_reset.argtypes = [G, B, C.c_int32, C.c_void_p]
     lib.gmes_tmz_forward.argtypes = [G, B, C.c_int32, C.c_int32, C.c_int32, C.c_void_p]
+    lib.gmes_tmz_launches.argtypes = [G, B, C.c_int32, C.c_int32, P(C.c_int64)]
     lib.gmes_tmz_objective.argtypes = [G, B, C.c_int32, C.c_void_p, C.c_void_p]
     lib.gmes_tmz_adjoint.argtypes = [G, B, C.c_int32, C.c_int32, C.c_void_p]
     lib.gmes_points_update.argtypes = [P(PointsC), C.c_void_p, C.c_void_p, C.c_void_p,

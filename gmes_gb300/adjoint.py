@@ -192,6 +192,16 @@ class TMzAdjoint:
         for s0 in range(0, self.nsteps, self.segment):
             yield s0 // self.segment, s0, min(self.segment, self.nsteps - s0)
 
+    def launches(self):
+        """Step kernels launched by one forward and one backward."""
+        def of(nsteps, adjoint):
+            out = C.c_int64()
+            self._call("gmes_tmz_launches", nsteps, adjoint, C.byref(out))
+            return out.value
+        if self.keep_history:
+            return of(self.nsteps, 0) + of(self.nsteps, 1)
+        return sum(2 * of(k, 0) + of(k, 1) for _, _, k in self._segments())
+
     def lattice(self, k):
         """State array k (0 Ez, 1 Hx, 2 Hy, 3..6 psi) as a (batch, nx, ny) float64 tensor."""
         return self._array(self.state, k)

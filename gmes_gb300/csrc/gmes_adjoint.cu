@@ -50,7 +50,7 @@
 // functions, and this file is compiled without implicit multiply-add
 // contraction (every fused operation is an explicit fmadd), so the two
 // forms give bit-identical fields, adjoints and gradients.
-#include "gmes_internal.cuh"
+#include "gmes_barrier.cuh"
 
 namespace gmes {
 namespace {
@@ -85,6 +85,22 @@ __device__ __forceinline__ bool lattice_point(const TmzDev& t, Lat& p) {
   p.base = (int64_t)p.b * t.plane;
   p.lin = (int64_t)p.i * t.ny + p.j;
   return true;
+}
+
+// Point `at` of all designs' lattices (persistent kernels).
+struct LatDiv {
+  uint32_t m_plane, m_row;
+  int s_plane, s_row;
+};
+__device__ __forceinline__ Lat lattice_at(const TmzDev& t, const LatDiv& d, unsigned at) {
+  Lat p;
+  p.b = (int)tile_quot(at, d.m_plane, d.s_plane);
+  const unsigned r = at - (unsigned)p.b * (unsigned)t.plane;
+  p.i = (int)tile_quot(r, d.m_row, d.s_row);
+  p.j = (int)(r - (unsigned)p.i * (unsigned)t.ny);
+  p.base = (int64_t)p.b * t.plane;
+  p.lin = r;
+  return p;
 }
 
 __device__ __forceinline__ int64_t design_index(const TmzDev& t, int i, int j) {
@@ -353,14 +369,50 @@ __global__ void k_tmz_map(const GridDev g, const TmzDev t) {
   P::st(const_cast<T*>(map_coef<P>(t, 3)) + ll, cy);
 }
 
-// Marks the points that carry a point source of either half (after
-// k_tmz_map, which clears those bits).
+// Marks the points that carry a point source of either half, with a place in
+// the list to look for it from (after k_tmz_map, which clears both).
 __global__ void k_tmz_map_sources(const TmzDev t) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= t.nsrc) return;
   const gmes_point_source s = t.src[k];
   if (s.comp < 2 || s.comp > 4 || s.offset < 0 || s.offset >= t.plane) return;
-  atomicOr(const_cast<uint32_t*>(t.pflags) + s.offset, s.comp == 2 ? kTmzSrcE : kTmzSrcH);
+  uint32_t* p = const_cast<uint32_t*>(t.pflags) + s.offset;
+  const uint32_t place = (uint32_t)(k + 1 < kTmzPlaces ? k + 1 : kTmzPlaces) << kTmzPlace;
+  constexpr uint32_t low = (1u << kTmzPlace) - 1;
+  uint32_t was = *p, seen;
+  do {
+    seen = was;
+    const uint32_t high = (seen & ~low) > place ? seen & ~low : place;
+    was = atomicCAS(p, seen, (seen & low) | high | (s.comp == 2 ? kTmzSrcE : kTmzSrcH));
+  } while (was != seen);
+}
+
+// The point source of lattice point ll in the array of Ez, Hx or Hy (k = 0, 1,
+// 2), -1: none; fl: the point's flags.  The last of several in the list.
+__device__ __forceinline__ int source_at(const TmzDev& t, unsigned fl, int k, int64_t ll) {
+  const int place = (int)(fl >> kTmzPlace) & kTmzPlaces;
+  int q = (place < kTmzPlaces && place < t.nsrc ? place : t.nsrc) - 1;
+  while (q >= 0 && (t.src[q].offset != ll || t.src[q].comp != k + 2)) --q;
+  return q;
+}
+
+// Point sources (gmes/pw_source.py:74-131) of that point: a field value after
+// the source of step n, and whether a hard source sits there (the value it
+// writes does not depend on the field before it, so its adjoint is zero;
+// current sources leave it as it is).
+template <class P>
+__device__ __forceinline__ typename P::R with_source(const TmzDev& t, unsigned fl, int k,
+                                                     int64_t ll, int n, typename P::R f) {
+  const int q = source_at(t, fl, k, ll);
+  if (q < 0) return f;
+  const typename P::R v = P::from_double(
+      __ldg(t.src_val + ((int64_t)(n - 1) * 2 + (k == 0 ? 0 : 1)) * t.nsrc + q));
+  return t.src[q].mode == 0 ? v : f - v;
+}
+__device__ __forceinline__ bool hard_source(const TmzDev& t, unsigned fl, int k, int64_t ll) {
+  if (!(fl & (k == 0 ? kTmzSrcE : kTmzSrcH))) return false;
+  const int q = source_at(t, fl, k, ll);
+  return q >= 0 && t.src[q].mode == 0;
 }
 
 // Plain-form Ez coefficients (c1, -c2) of lattice point (i, j) = ll of
@@ -387,9 +439,10 @@ __device__ __forceinline__ typename P::R weight_x(const GridDev& g, const TmzDev
   const T* lx = static_cast<const T*>(t.l[1]) + base + ll;
   const typename P::R c = P::ld(map_coef<P>(t, 2) + ll);  // issued with the flags
   const unsigned fl = __ldg(t.pflags + ll);
-  if (fl & kTmzPlainX) return c * P::ldw(lx);
+  const typename P::R l = hard_source(t, fl, 1, ll) ? P::zero() : P::ldw(lx);
+  if (fl & kTmzPlainX) return c * l;
   if (!(fl & kTmzPsiX)) return P::zero();
-  return adjx_cpml<P, OWN>(g, fl, c, j, P::ldw(lx),
+  return adjx_cpml<P, OWN>(g, fl, c, j, l,
                            static_cast<const T*>(t.phi[rb][2]) + base + ll,
                            OWN ? static_cast<T*>(t.phi[wb][2]) + base + ll : nullptr);
 }
@@ -401,9 +454,10 @@ __device__ __forceinline__ typename P::R weight_y(const GridDev& g, const TmzDev
   const T* ly = static_cast<const T*>(t.l[2]) + base + ll;
   const typename P::R c = P::ld(map_coef<P>(t, 3) + ll);  // issued with the flags
   const unsigned fl = __ldg(t.pflags + ll);
-  if (fl & kTmzPlainY) return c * P::ldw(ly);
+  const typename P::R l = hard_source(t, fl, 2, ll) ? P::zero() : P::ldw(ly);
+  if (fl & kTmzPlainY) return c * l;
   if (!(fl & kTmzPsiY)) return P::zero();
-  return adjy_cpml<P, OWN>(g, fl, c, i, P::ldw(ly),
+  return adjy_cpml<P, OWN>(g, fl, c, i, l,
                            static_cast<const T*>(t.phi[rb][3]) + base + ll,
                            OWN ? static_cast<T*>(t.phi[wb][3]) + base + ll : nullptr);
 }
@@ -437,26 +491,27 @@ __device__ __forceinline__ void weight_e(const GridDev& g, const TmzDev& t, int 
 }
 
 // ---------------------------------------------------------------------------
-// One-step forward kernels.
+// One step of one lattice point, forward (step n; slot: where its design
+// increment is recorded, row: its monitor row, -1 not).
 // ---------------------------------------------------------------------------
 template <class P>
-__global__ void __launch_bounds__(kBX* kBY) k_tmz_fe(const GridDev g, const TmzDev t, int slot) {
+__device__ __forceinline__ void point_fe(const GridDev& g, const TmzDev& t, const Lat& p, int n,
+                                         int slot) {
   using R = typename P::R;
   using T = typename P::T;
-  Lat p;
-  if (!lattice_point(t, p)) return;
   const int im = p.i == 0 ? t.nx - 1 : p.i - 1, jm = p.j == 0 ? t.ny - 1 : p.j - 1;
   T* E = static_cast<T*>(t.f[0]) + p.base;
   const T* X = static_cast<const T*>(t.f[1]) + p.base;
   const T* Y = static_cast<const T*>(t.f[2]) + p.base;
   const unsigned fl = __ldg(t.pflags + p.lin);
-  const R D1 = P::ld(Y + p.lin) - P::ld(Y + (int64_t)im * t.ny + p.j);
-  const R D2 = P::ld(X + p.lin) - P::ld(X + (int64_t)p.i * t.ny + jm);
+  const R D1 = P::ldw(Y + p.lin) - P::ldw(Y + (int64_t)im * t.ny + p.j);
+  const R D2 = P::ldw(X + p.lin) - P::ldw(X + (int64_t)p.i * t.ny + jm);
   const R e = P::ldw(E + p.lin);
+  R r = e;
   if (fl & kTmzPlainE) {
     R c1, c2n;
     e_coef<P>(t, p.b, p.i, p.j, p.lin, fl, c1, c2n);
-    P::st(E + p.lin, fmadd(fmadd(e, c1, D1), c2n, D2));
+    r = fmadd(fmadd(e, c1, D1), c2n, D2);
     if ((fl & kTmzDesign) && slot >= 0) {
       const int64_t nd = (int64_t)t.dn[0] * t.dn[1];
       P::st(static_cast<T*>(t.hist) + ((int64_t)slot * t.nb + p.b) * nd +
@@ -464,80 +519,66 @@ __global__ void __launch_bounds__(kBX* kBY) k_tmz_fe(const GridDev g, const TmzD
             fmadd(c2n * D2, c1, D1));
     }
   } else if (fl & kTmzPsiE) {
-    P::st(E + p.lin, e_cpml<P>(g, fl, P::ld(map_coef<P>(t, 0) + p.lin), p.i, p.j, e, D1, D2,
-                               static_cast<T*>(t.f[3]) + p.base + p.lin,
-                               static_cast<T*>(t.f[4]) + p.base + p.lin));
+    r = e_cpml<P>(g, fl, P::ld(map_coef<P>(t, 0) + p.lin), p.i, p.j, e, D1, D2,
+                  static_cast<T*>(t.f[3]) + p.base + p.lin,
+                  static_cast<T*>(t.f[4]) + p.base + p.lin);
   }
+  if (fl & kTmzSrcE) r = with_source<P>(t, fl, 0, p.lin, n, r);
+  P::st(E + p.lin, r);
 }
 
 template <class P>
-__global__ void __launch_bounds__(kBX* kBY) k_tmz_fh(const GridDev g, const TmzDev t, int row) {
+__device__ __forceinline__ void point_fh(const GridDev& g, const TmzDev& t, const Lat& p, int n,
+                                         int row) {
   using R = typename P::R;
   using T = typename P::T;
-  Lat p;
-  if (!lattice_point(t, p)) return;
   const int ip = p.i + 1 == t.nx ? 0 : p.i + 1, jp = p.j + 1 == t.ny ? 0 : p.j + 1;
   const T* E = static_cast<const T*>(t.f[0]) + p.base;
   T* X = static_cast<T*>(t.f[1]) + p.base;
   T* Y = static_cast<T*>(t.f[2]) + p.base;
   const unsigned fl = __ldg(t.pflags + p.lin);
   const R cxn = P::ld(map_coef<P>(t, 2) + p.lin), cy = P::ld(map_coef<P>(t, 3) + p.lin);
-  const R e0 = P::ld(E + p.lin);
-  const R dx = P::ld(E + (int64_t)p.i * t.ny + jp) - e0;  // D1 of Hx
-  const R dy = P::ld(E + (int64_t)ip * t.ny + p.j) - e0;  // D2 of Hy
+  const R e0 = P::ldw(E + p.lin);
+  const R dx = P::ldw(E + (int64_t)p.i * t.ny + jp) - e0;  // D1 of Hx
+  const R dy = P::ldw(E + (int64_t)ip * t.ny + p.j) - e0;  // D2 of Hy
+  const R x0 = P::ldw(X + p.lin), y0 = P::ldw(Y + p.lin);
+  R x = x0, y = y0;
   if (fl & kTmzPlainX)
-    P::st(X + p.lin, fmadd(P::ldw(X + p.lin), cxn, dx));
+    x = fmadd(x0, cxn, dx);
   else if (fl & kTmzPsiX)
-    P::st(X + p.lin, x_cpml<P>(g, fl, cxn, p.j, P::ldw(X + p.lin), dx,
-                               static_cast<T*>(t.f[5]) + p.base + p.lin));
+    x = x_cpml<P>(g, fl, cxn, p.j, x0, dx, static_cast<T*>(t.f[5]) + p.base + p.lin);
   if (fl & kTmzPlainY)
-    P::st(Y + p.lin, fmadd(P::ldw(Y + p.lin), cy, dy));
+    y = fmadd(y0, cy, dy);
   else if (fl & kTmzPsiY)
-    P::st(Y + p.lin, y_cpml<P>(g, fl, cy, p.i, P::ldw(Y + p.lin), dy,
-                               static_cast<T*>(t.f[6]) + p.base + p.lin));
+    y = y_cpml<P>(g, fl, cy, p.i, y0, dy, static_cast<T*>(t.f[6]) + p.base + p.lin);
+  if (fl & kTmzSrcH) {
+    x = with_source<P>(t, fl, 1, p.lin, n, x);
+    y = with_source<P>(t, fl, 2, p.lin, n, y);
+  }
+  P::st(X + p.lin, x);
+  P::st(Y + p.lin, y);
   if (row >= 0 && (fl & kTmzMonitor)) {
     const int64_t nm = (int64_t)t.mn[0] * t.mn[1];
     t.mon[((int64_t)p.b * t.total_steps + row) * nm + monitor_index(t, p.i, p.j)] = to_double(e0);
   }
 }
 
-// Point sources of one half (gmes/pw_source.py:74-131) for every design:
-// comp 2/3/4 = E/X/Y lattice array, offset = i * ny + j.  Entries that do
-// not name a lattice point of that half are skipped.
-template <class P>
-__global__ void k_tmz_src(const TmzDev t, int side, int n) {
-  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= (int64_t)t.nsrc * t.nb) return;
-  const int b = (int)(q / t.nsrc), k = (int)(q - (int64_t)b * t.nsrc);
-  const gmes_point_source s = t.src[k];
-  if (s.comp < 2 || s.comp > 4 || (s.comp == 2) != (side == 0)) return;
-  if (s.offset < 0 || s.offset >= t.plane) return;
-  const double v = t.src_val[((int64_t)(n - 1) * 2 + side) * t.nsrc + k];
-  using T = typename P::T;
-  T* f = static_cast<T*>(t.f[s.comp - 2]) + (int64_t)b * t.plane + s.offset;
-  if (s.mode == 0)
-    P::st(f, P::from_double(v));
-  else
-    P::st(f, P::ldw(f) - P::from_double(v));
-}
-
 // ---------------------------------------------------------------------------
-// One-step adjoint kernels.
+// One step of one lattice point, adjoint.
 // ---------------------------------------------------------------------------
 // Transpose of the H half of step n, plus the objective's seed for the
 // state after step n: lambda_E gathers the curl weights of its four H
 // neighbours; the owner advances the Hx/Hy psi adjoints.
 template <class P>
-__global__ void __launch_bounds__(kBX* kBY)
-    k_tmz_ah(const GridDev g, const TmzDev t, int n, int rb, int wb) {
+__device__ __forceinline__ void point_ah(const GridDev& g, const TmzDev& t, const Lat& p, int n,
+                                         int rb, int wb) {
   using R = typename P::R;
   using T = typename P::T;
-  Lat p;
-  if (!lattice_point(t, p)) return;
   const int im = p.i == 0 ? t.nx - 1 : p.i - 1, jm = p.j == 0 ? t.ny - 1 : p.j - 1;
   T* LE = static_cast<T*>(t.l[0]) + p.base + p.lin;
   R le = P::ldw(LE);
-  if (__ldg(t.pflags + p.lin) & kTmzMonitor) {
+  const unsigned fl = __ldg(t.pflags + p.lin);
+  if (fl & kTmzMonitor) {
     bool has;
     le = le + P::from_double(seed_of(g, t, p.b, p.i, p.j, n, &has));
   }
@@ -546,19 +587,18 @@ __global__ void __launch_bounds__(kBX* kBY)
   const R bx = weight_x<P, true>(g, t, p.i, p.j, p.lin, p.base, rb, wb);
   const R c = weight_y<P, false>(g, t, im, p.j, lim, p.base, rb, wb);
   const R d = weight_y<P, true>(g, t, p.i, p.j, p.lin, p.base, rb, wb);
-  P::st(LE, le + ((a - bx) + (c - d)));
+  le = le + ((a - bx) + (c - d));
+  P::st(LE, hard_source(t, fl, 0, p.lin) ? P::zero() : le);
 }
 
 // Transpose of the E half of step n: lambda_X, lambda_Y gather the curl
 // weights of their two Ez neighbours; the owner advances the Ez psi
 // adjoints and, in the design region, accumulates the gradient.
 template <class P>
-__global__ void __launch_bounds__(kBX* kBY)
-    k_tmz_ae(const GridDev g, const TmzDev t, int slot, int rb, int wb) {
+__device__ __forceinline__ void point_ae(const GridDev& g, const TmzDev& t, const Lat& p,
+                                         int slot, int rb, int wb) {
   using R = typename P::R;
   using T = typename P::T;
-  Lat p;
-  if (!lattice_point(t, p)) return;
   const int ip = p.i + 1 == t.nx ? 0 : p.i + 1, jp = p.j + 1 == t.ny ? 0 : p.j + 1;
   const int64_t ljp = (int64_t)p.i * t.ny + jp, lip = (int64_t)ip * t.ny + p.j;
   R w1, w2, u1, u2, v1, v2;
@@ -567,9 +607,12 @@ __global__ void __launch_bounds__(kBX* kBY)
   weight_e<P, false, true, false>(g, t, p.b, ip, p.j, lip, p.base, rb, wb, v1, v2);
   T* LX = static_cast<T*>(t.l[1]) + p.base + p.lin;
   T* LY = static_cast<T*>(t.l[2]) + p.base + p.lin;
-  P::st(LX, P::ldw(LX) + (w2 - u2));
-  P::st(LY, P::ldw(LY) + (w1 - v1));
-  if (__ldg(t.pflags + p.lin) & kTmzDesign) {
+  const unsigned fl = __ldg(t.pflags + p.lin);
+  const R lx = hard_source(t, fl, 1, p.lin) ? P::zero() : P::ldw(LX);
+  const R ly = hard_source(t, fl, 2, p.lin) ? P::zero() : P::ldw(LY);
+  P::st(LX, lx + (w2 - u2));
+  P::st(LY, ly + (w1 - v1));
+  if (fl & kTmzDesign) {
     const int64_t nd = (int64_t)t.dn[0] * t.dn[1];
     const int64_t dp = design_index(t, p.i, p.j);
     const int64_t k = (int64_t)p.b * nd + dp;
@@ -580,19 +623,88 @@ __global__ void __launch_bounds__(kBX* kBY)
   }
 }
 
-// Transpose of a half's hard sources: the value written does not depend
-// on the field before it, so its adjoint is zeroed.  Current sources add a
-// constant and leave the adjoint unchanged.
+// ---------------------------------------------------------------------------
+// One-step kernels: a half-step of every lattice point per launch, or a whole
+// call's steps in one cooperative launch with a grid-wide barrier after each
+// half (gmes_barrier.cuh).  The point's sources act in the body (with_source,
+// hard_source), so a step is two launches, not four: FP64 300x243 x 6 designs,
+// 200 steps with checkpoints, forward / backward 5.95 / 14.2 ms -> 4.39 / 11.4.
+// What is left at that size is the launches themselves, 7-11 us per half-step
+// of 0.44 M points; one cooperative launch of 512-thread blocks, two to an SM
+// (62 registers), pays a 1.4 us barrier instead: 3.33 / 8.65 ms.  tmz_chunked
+// says up to what size.
+// ---------------------------------------------------------------------------
 template <class P>
-__global__ void k_tmz_adj_src(const TmzDev t, int side) {
-  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= (int64_t)t.nsrc * t.nb) return;
-  const int b = (int)(q / t.nsrc), k = (int)(q - (int64_t)b * t.nsrc);
-  const gmes_point_source s = t.src[k];
-  if (s.mode != 0 || s.comp < 2 || s.comp > 4 || (s.comp == 2) != (side == 0)) return;
-  if (s.offset < 0 || s.offset >= t.plane) return;
-  P::st(static_cast<typename P::T*>(t.l[s.comp - 2]) + (int64_t)b * t.plane + s.offset,
-        P::zero());
+__global__ void __launch_bounds__(kBX* kBY)
+    k_tmz_fe(const GridDev g, const TmzDev t, int n, int slot) {
+  Lat p;
+  if (lattice_point(t, p)) point_fe<P>(g, t, p, n, slot);
+}
+template <class P>
+__global__ void __launch_bounds__(kBX* kBY)
+    k_tmz_fh(const GridDev g, const TmzDev t, int n, int row) {
+  Lat p;
+  if (lattice_point(t, p)) point_fh<P>(g, t, p, n, row);
+}
+template <class P>
+__global__ void __launch_bounds__(kBX* kBY)
+    k_tmz_ah(const GridDev g, const TmzDev t, int n, int rb, int wb) {
+  Lat p;
+  if (lattice_point(t, p)) point_ah<P>(g, t, p, n, rb, wb);
+}
+template <class P>
+__global__ void __launch_bounds__(kBX* kBY)
+    k_tmz_ae(const GridDev g, const TmzDev t, int slot, int rb, int wb) {
+  Lat p;
+  if (lattice_point(t, p)) point_ae<P>(g, t, p, slot, rb, wb);
+}
+
+constexpr int kChunkThreads = 512;
+
+// Groups of 32 points go round the blocks in turn, so that every SM gets its
+// share of the absorbing layer, the design and the sources.
+template <class F>
+__device__ __forceinline__ void for_points(const TmzDev& t, const LatDiv& d, F f) {
+  const unsigned total = (unsigned)(t.plane * t.nb), groups = (total + 31) / 32;
+  for (unsigned q = blockIdx.x + (threadIdx.x >> 5) * gridDim.x; q < groups;
+       q += kChunkThreads / 32 * gridDim.x) {
+    const unsigned at = q * 32 + (threadIdx.x & 31);
+    if (at < total) f(lattice_at(t, d, at));
+  }
+}
+
+// Forward steps step0 + 1 .. step0 + nsteps (flags: GMES_TMZ_RECORD_*).
+template <class P>
+__global__ void __launch_bounds__(kChunkThreads, 2)
+    k_tmz_chunk_fwd(const __grid_constant__ GridDev g, const __grid_constant__ TmzDev t,
+                    const LatDiv d, int step0, int nsteps, int flags, int* error) {
+  unsigned* const word = barrier_words + 8 * t.word;
+  for (int k = 0; k < nsteps; ++k) {
+    const int n = step0 + k + 1;
+    for_points(t, d, [&](const Lat& p) {
+      point_fe<P>(g, t, p, n, (flags & GMES_TMZ_RECORD_HIST) ? k : -1);
+    });
+    if (!grid_barrier(word, error)) return;
+    for_points(t, d, [&](const Lat& p) {
+      point_fh<P>(g, t, p, n, (flags & GMES_TMZ_RECORD_MONITOR) ? n - 1 : -1);
+    });
+    if (k + 1 < nsteps && !grid_barrier(word, error)) return;
+  }
+}
+
+// Adjoint steps step0 + nsteps down to step0 + 1.
+template <class P>
+__global__ void __launch_bounds__(kChunkThreads, 2)
+    k_tmz_chunk_adj(const __grid_constant__ GridDev g, const __grid_constant__ TmzDev t,
+                    const LatDiv d, int step0, int nsteps, int* error) {
+  unsigned* const word = barrier_words + 8 * t.word;
+  for (int k = nsteps - 1; k >= 0; --k) {
+    const int n = step0 + k + 1, rb = n & 1, wb = rb ^ 1;
+    for_points(t, d, [&](const Lat& p) { point_ah<P>(g, t, p, n, rb, wb); });
+    if (!grid_barrier(word, error)) return;
+    for_points(t, d, [&](const Lat& p) { point_ae<P>(g, t, p, k, rb, wb); });
+    if (k > 0 && !grid_barrier(word, error)) return;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1980,7 +2092,8 @@ __global__ void __launch_bounds__(kTbThreads) k_tmz_tiles(const TmzDev t) {
   for (int k = 0; k < 7; ++k)
     c[k] = first_s[k] < 0 ? P::zero() : coef(at(first_s[k] / kTbRJ, first_s[k] % kTbRJ), k);
   const unsigned pm = pm_s < 0 ? 0u : (unsigned)pm_s;
-  constexpr unsigned specials = kTmzSrcE | kTmzMonitor | kTmzDesign;
+  constexpr unsigned specials =
+      kTmzSrcE | kTmzMonitor | kTmzDesign | ~((1u << kTmzPlace) - 1);
   bool same = (any_s & ~(plain | layer | pmbits | specials)) == 0, even = true;
   for (int q = threadIdx.x; q < G::NP && same; q += kTbThreads) {
     const int a = q / kTbRJ, cc = q % kTbRJ;
@@ -2070,33 +2183,76 @@ dim3 lattice_grid(const TmzDev& t) {
               (unsigned)t.nb);
 }
 
+// Blocks of a chunk kernel and its index quotients.
+template <class K>
+cudaError_t chunk_shape(K* kernel, const TmzDev& t, LatDiv& d, int& blocks) {
+  int per_sm = 0;
+  const cudaError_t e =
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kChunkThreads, 0);
+  if (e != cudaSuccess) return e;
+  if (per_sm < 1) return cudaErrorLaunchOutOfResources;
+  const int64_t groups = (t.plane * t.nb + 31) / 32, sms = sm_count();
+  // one block per SM while its warps take at most one group each
+  const int64_t most = groups <= sms * (kChunkThreads / 32) ? sms : sms * per_sm;
+  blocks = (int)(groups < most ? groups : most);
+  tile_div_of((uint32_t)t.plane, d.m_plane, d.s_plane);
+  tile_div_of((uint32_t)t.ny, d.m_row, d.s_row);
+  return cudaSuccess;
+}
+
+// Names the points of the sources as they are now: a caller may have set
+// others since the design.
+void map_sources(const TmzDev& t, cudaStream_t s) {
+  if (t.nsrc > 0) k_tmz_map_sources<<<(t.nsrc + 127) / 128, 128, 0, s>>>(t);
+}
+
 template <class P>
 cudaError_t forward(const GridDev& g, const TmzDev& t, int step0, int nsteps, int flags,
                     cudaStream_t s) {
+  if (nsteps <= 0) return cudaSuccess;
+  map_sources(t, s);
+  if (t.word >= 0) {
+    LatDiv d;
+    int blocks = 0;
+    const cudaError_t e = chunk_shape(k_tmz_chunk_fwd<P>, t, d, blocks);
+    if (e != cudaSuccess) return e;
+    GridDev gg = g;
+    TmzDev tt = t;
+    int* error = wait_error_word();
+    void* args[] = {&gg, &tt, &d, &step0, &nsteps, &flags, &error};
+    return cudaLaunchCooperativeKernel((const void*)k_tmz_chunk_fwd<P>, dim3((unsigned)blocks),
+                                       dim3(kChunkThreads), args, 0, s);
+  }
   const dim3 grid = lattice_grid(t), block(kBX, kBY);
-  const int64_t nq = (int64_t)t.nsrc * t.nb;
-  const unsigned sblocks = (unsigned)((nq + 127) / 128);
   for (int k = 0; k < nsteps; ++k) {
     const int n = step0 + k + 1;
-    k_tmz_fe<P><<<grid, block, 0, s>>>(g, t, (flags & GMES_TMZ_RECORD_HIST) ? k : -1);
-    if (nq > 0) k_tmz_src<P><<<sblocks, 128, 0, s>>>(t, 0, n);
-    k_tmz_fh<P><<<grid, block, 0, s>>>(g, t, (flags & GMES_TMZ_RECORD_MONITOR) ? n - 1 : -1);
-    if (nq > 0) k_tmz_src<P><<<sblocks, 128, 0, s>>>(t, 1, n);
+    k_tmz_fe<P><<<grid, block, 0, s>>>(g, t, n, (flags & GMES_TMZ_RECORD_HIST) ? k : -1);
+    k_tmz_fh<P><<<grid, block, 0, s>>>(g, t, n, (flags & GMES_TMZ_RECORD_MONITOR) ? n - 1 : -1);
   }
   return cudaGetLastError();
 }
 
 template <class P>
 cudaError_t adjoint(const GridDev& g, const TmzDev& t, int step0, int nsteps, cudaStream_t s) {
+  if (nsteps <= 0) return cudaSuccess;
+  map_sources(t, s);
+  if (t.word >= 0) {
+    LatDiv d;
+    int blocks = 0;
+    const cudaError_t e = chunk_shape(k_tmz_chunk_adj<P>, t, d, blocks);
+    if (e != cudaSuccess) return e;
+    GridDev gg = g;
+    TmzDev tt = t;
+    int* error = wait_error_word();
+    void* args[] = {&gg, &tt, &d, &step0, &nsteps, &error};
+    return cudaLaunchCooperativeKernel((const void*)k_tmz_chunk_adj<P>, dim3((unsigned)blocks),
+                                       dim3(kChunkThreads), args, 0, s);
+  }
   const dim3 grid = lattice_grid(t), block(kBX, kBY);
-  const int64_t nq = (int64_t)t.nsrc * t.nb;
-  const unsigned sblocks = (unsigned)((nq + 127) / 128);
   for (int k = nsteps - 1; k >= 0; --k) {
     const int n = step0 + k + 1;
     const int rb = n & 1, wb = rb ^ 1;
-    if (nq > 0) k_tmz_adj_src<P><<<sblocks, 128, 0, s>>>(t, 1);
     k_tmz_ah<P><<<grid, block, 0, s>>>(g, t, n, rb, wb);
-    if (nq > 0) k_tmz_adj_src<P><<<sblocks, 128, 0, s>>>(t, 0);
     k_tmz_ae<P><<<grid, block, 0, s>>>(g, t, k, rb, wb);
   }
   return cudaGetLastError();
@@ -2238,6 +2394,33 @@ cudaError_t launch_tmz_design(int precision, const GridDev& g, const TmzDev& t,
   if (precision == GMES_FP32 && t.tmp[0] != nullptr)
     k_tmz_tiles<PolF32, kTbQ><<<tb_tiles<PolF32, kTbQ>(t), kTbThreads, 0, s>>>(t);
   return cudaGetLastError();
+}
+
+// Lattice points of all designs up to which a call's steps run as one
+// cooperative launch.  Measured on GB300, 60 steps forward / adjoint ms, two
+// launches per step -> one launch (with the sources in kernels of their own,
+// four launches per step, in brackets):
+//   FP64  128x123 x 1    (1.28 / 1.24)   0.74 / 0.75  -> 0.53 / 0.51
+//         256x251 x 4    (1.82 / 2.19)   1.33 / 1.74  -> 0.87 / 1.21
+//         400x395 x 24   (6.39 / 12.0)   5.80 / 11.6  -> 5.47 / 10.5
+//         512x507 x 64   (20.3 / 40.8)   19.4 / 40.5  -> 23.2 / 46.8
+//   df64  128x123 x 8    (1.39 / 1.27)   0.96 / 0.86  -> 0.63 / 0.60
+//         256x251 x 16   (2.20 / 2.61)   1.70 / 2.12  -> 1.53 / 2.25
+//         512x507 x 64   (19.7 / 29.6)   16.8 / 27.9  -> 22.0 / 43.3
+// A small lattice's half-step is bound by its launch; a large one by the FP64
+// pipe or L2, for which the one-launch kernel has fewer warps (62 registers).
+constexpr int64_t kChunkPoints = 1 << 22, kChunkPointsDf = 1 << 20;
+
+bool tmz_chunked(int precision, const TmzDev& t, int block_steps) {
+  return steps_per_launch(precision, t, block_steps) == 1 && wait_error_word() != nullptr &&
+         t.plane * t.nb <= (precision == GMES_DF64 ? kChunkPointsDf : kChunkPoints);
+}
+
+int64_t tmz_launches(int precision, const TmzDev& t, int block_steps, int nsteps, bool adj) {
+  const int per = steps_per_launch(precision, t, block_steps);
+  if (nsteps <= 0) return 0;
+  if (per > 1) return adj ? adj_launches(nsteps, per) : (nsteps + per - 1) / per;
+  return (t.nsrc > 0) + (tmz_chunked(precision, t, block_steps) ? 1 : 2 * (int64_t)nsteps);
 }
 
 cudaError_t launch_tmz_forward(int precision, const GridDev& g, const TmzDev& t, int step0,

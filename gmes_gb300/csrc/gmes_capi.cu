@@ -952,7 +952,7 @@ struct TmzLayout {
   int64_t array;  // bytes of one [nb][nx][ny] array, 256-aligned
   int64_t state, adjoint, design, hist, monitor, grad, scratch;
   // the design buffer: per-pixel coefficients, then the lattice map's
-  // flags and its four coefficient arrays, and the blocked kernels' tiles
+  // flags and four coefficient arrays, and the blocked kernels' tiles
   int64_t design_coef, map_flags, map_coef, tiles;
 };
 
@@ -1051,8 +1051,9 @@ TmzDev make_tmz_dev(const gmes_grid_desc& g, const gmes_tmz_batch& b) {
   const char* map = static_cast<const char*>(b.design) + L.design_coef;
   t.pflags = reinterpret_cast<const uint32_t*>(map);
   for (int k = 0; k < 4; ++k) t.pcoef[k] = map + L.map_flags + k * L.map_coef;
-  if (tmz_blocked(g, b))
-    t.tiles = static_cast<char*>(b.design) + L.design_coef + L.map_flags + 4 * L.map_coef;
+  char* after = static_cast<char*>(b.design) + L.design_coef + L.map_flags + 4 * L.map_coef;
+  if (tmz_blocked(g, b)) t.tiles = after;
+  t.word = -1;
   t.hist = b.hist;
   t.mon = b.monitor;
   t.grad = b.grad;
@@ -1129,6 +1130,16 @@ gmes_status gmes_tmz_set_design(const gmes_grid_desc* g, const gmes_tmz_batch* b
   return GMES_OK;
 }
 
+gmes_status gmes_tmz_launches(const gmes_grid_desc* g, const gmes_tmz_batch* b, int32_t nsteps,
+                              int32_t adjoint, int64_t* launches) {
+  gmes_status st = check_tmz(g, b, true);
+  if (st != GMES_OK) return st;
+  if (launches == nullptr) return fail(GMES_ERR_VALUE, "launches is NULL");
+  *launches = tmz_launches(g->precision, make_tmz_dev(*g, *b), b->block_steps, nsteps,
+                           adjoint != 0);
+  return GMES_OK;
+}
+
 gmes_status gmes_tmz_reset(const gmes_grid_desc* g, const gmes_tmz_batch* b, int32_t what,
                            void* stream) {
   gmes_status st = check_tmz(g, b, true);
@@ -1154,7 +1165,12 @@ gmes_status gmes_tmz_forward(const gmes_grid_desc* g, const gmes_tmz_batch* b, i
   if ((flags & ~3) != 0) return fail(GMES_ERR_VALUE, "unknown flags 0x%x", flags);
   if ((flags & GMES_TMZ_RECORD_HIST) && nsteps > b->hist_steps)
     return fail(GMES_ERR_VALUE, "%d steps exceed the hist capacity %d", nsteps, b->hist_steps);
-  cudaError_t e = launch_tmz_forward(g->precision, make_grid_dev(*g), make_tmz_dev(*g, *b),
+  st = check_wait_error();
+  if (st != GMES_OK) return st;
+  TmzDev t = make_tmz_dev(*g, *b);
+  if (tmz_chunked(g->precision, t, b->block_steps))
+    t.word = take_word(static_cast<cudaStream_t>(stream));
+  cudaError_t e = launch_tmz_forward(g->precision, make_grid_dev(*g), t,
                                      step0, nsteps, flags, b->block_steps,
                                      static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "launching the forward kernels");
@@ -1183,7 +1199,12 @@ gmes_status gmes_tmz_adjoint(const gmes_grid_desc* g, const gmes_tmz_batch* b, i
                 b->total_steps);
   if (nsteps > b->hist_steps)
     return fail(GMES_ERR_VALUE, "%d steps exceed the hist capacity %d", nsteps, b->hist_steps);
-  cudaError_t e = launch_tmz_adjoint(g->precision, make_grid_dev(*g), make_tmz_dev(*g, *b),
+  st = check_wait_error();
+  if (st != GMES_OK) return st;
+  TmzDev t = make_tmz_dev(*g, *b);
+  if (tmz_chunked(g->precision, t, b->block_steps))
+    t.word = take_word(static_cast<cudaStream_t>(stream));
+  cudaError_t e = launch_tmz_adjoint(g->precision, make_grid_dev(*g), t,
                                      step0, nsteps, b->block_steps,
                                      static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "launching the adjoint kernels");

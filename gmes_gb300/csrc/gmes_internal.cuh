@@ -412,6 +412,7 @@ struct TmzDev {
   const uint32_t* pflags;
   const void* pcoef[4];
   void* tiles;              // TbTile of every tile of the blocked kernels, or null
+  int32_t word;             // barrier word of the persistent kernels, -1: none to be had
   void* l[3];
   void* phi[2][4];          // ping-pong buffers of the psi adjoints
   const DesignCoef* dc;     // [nb][nd]
@@ -447,7 +448,9 @@ struct TbTile {
 // kTmzSrcE / kTmzSrcH: a point source of the E / H half sits on the point.
 // For psi points, kTmzOn*: which of the point's profiles are on (Ez: along
 // x and y; Hx: along y; Hy: along x) and the 2-bit fields at kTmzPml*: the
-// class's profile set.
+// class's profile set.  The 9 bits from kTmzPlace on: where in the list of
+// point sources to look from, towards its start, for those of this point, plus
+// one (kTmzPlaces: from the end).  Bit 31 is the kernels' own.
 enum : uint32_t {
   kTmzPlainE = 1, kTmzPlainX = 2, kTmzPlainY = 4,
   kTmzPsiE = 8, kTmzPsiX = 16, kTmzPsiY = 32,
@@ -455,7 +458,8 @@ enum : uint32_t {
   kTmzSrcE = 256, kTmzSrcH = 512,
   kTmzOnE1 = 1024, kTmzOnE2 = 2048, kTmzOnX = 4096, kTmzOnY = 8192
 };
-constexpr int kTmzPmlE = 16, kTmzPmlX = 18, kTmzPmlY = 20;  // bit offsets
+constexpr int kTmzPmlE = 16, kTmzPmlX = 18, kTmzPmlY = 20, kTmzPlace = 22;  // bit offsets
+constexpr int kTmzPlaces = 511;
 static_assert(GMES_MAX_PML <= 4, "2-bit profile-set fields");
 
 cudaError_t launch_tmz_design(int precision, const GridDev& g, const TmzDev& t,
@@ -464,6 +468,10 @@ cudaError_t launch_tmz_forward(int precision, const GridDev& g, const TmzDev& t,
                                int nsteps, int flags, int block_steps, cudaStream_t s);
 cudaError_t launch_tmz_adjoint(int precision, const GridDev& g, const TmzDev& t, int step0,
                                int nsteps, int block_steps, cudaStream_t s);
+// Whether a call's steps run as one cooperative launch (given a barrier word).
+bool tmz_chunked(int precision, const TmzDev& t, int block_steps);
+// Launches of one forward or adjoint call.
+int64_t tmz_launches(int precision, const TmzDev& t, int block_steps, int nsteps, bool adj);
 cudaError_t launch_tmz_objective(const GridDev& g, const TmzDev& t, int nsteps, double* J,
                                  cudaStream_t s);
 

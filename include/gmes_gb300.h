@@ -518,6 +518,13 @@ gmes_status gmes_tmz_check(const gmes_grid_desc* g, const gmes_tmz_batch* b);
    the resolved update of every lattice point (flags and coefficients). */
 gmes_status gmes_tmz_set_design(const gmes_grid_desc* g, const gmes_tmz_batch* b,
                                 const double* eps, void* stream);
+/*
+ * The kernels that one gmes_tmz_forward (adjoint = 0) or gmes_tmz_adjoint call
+ * of nsteps steps launches, in *launches.
+ */
+gmes_status gmes_tmz_launches(const gmes_grid_desc* g, const gmes_tmz_batch* b, int32_t nsteps,
+                              int32_t adjoint, int64_t* launches);
+
 /* Zero the state (what & 1) and/or the adjoint and grad (what & 2). */
 gmes_status gmes_tmz_reset(const gmes_grid_desc* g, const gmes_tmz_batch* b, int32_t what,
                            void* stream);
