@@ -1022,6 +1022,20 @@ __device__ __forceinline__ void ghost_cell(const GridDev& g, const GridDev& gi, 
   if (is_active<MASK, c0 + 2>(g)) ghost_images<P, c0 + 2, CX>(g, gi, x, l2, all);
 }
 
+// ghost_images of component c's own point alone.
+template <class P, bool CX>
+__device__ __forceinline__ void ghost_own(const GridDev& g, const GridDev& gi, int c,
+                                          const int x[3], int l) {
+  switch (c) {
+    case 0: ghost_images<P, 0, CX>(g, gi, x, l, true); break;
+    case 1: ghost_images<P, 1, CX>(g, gi, x, l, true); break;
+    case 2: ghost_images<P, 2, CX>(g, gi, x, l, true); break;
+    case 3: ghost_images<P, 3, CX>(g, gi, x, l, true); break;
+    case 4: ghost_images<P, 4, CX>(g, gi, x, l, true); break;
+    case 5: ghost_images<P, 5, CX>(g, gi, x, l, true); break;
+  }
+}
+
 // Point sources of one half-step (gmes/pw_source.py:74-131), applied after
 // that half's material update.  `v` has been computed on the host in FP64.
 template <class P, bool STRICT>

@@ -352,14 +352,17 @@ __global__ void __launch_bounds__(kPersistThreads, GMES_PERSIST_BLOCKS)
       }
       if (nown > 0) {
         __syncthreads();
-        if ((int)threadIdx.x < nown) {
-          const OwnSource o = own[threadIdx.x];
-          if ((o.comp < 3) == (SIDE == 0) && (o.i >= 0 || last)) {
-            const int64_t slot = 2 * (int64_t)(c.st0 + st) + SIDE;
-            source_point<P, false>(g, SIDE, slot, o.q);
-            if constexpr (CX) source_point<P, false>(gi, SIDE, slot, o.q);
-            if (images && o.i >= 0) ghost_cell<P, SIDE, MASK, CX>(g, gi, o.i, o.j, o.k, all);
-          }
+        const OwnSource o = own[threadIdx.x < (unsigned)nown ? threadIdx.x : 0];
+        const bool on = (int)threadIdx.x < nown && (o.comp < 3) == (SIDE == 0);
+        if (on && (o.i >= 0 || last)) {
+          const int64_t slot = 2 * (int64_t)(c.st0 + st) + SIDE;
+          source_point<P, false>(g, SIDE, slot, o.q);
+          if constexpr (CX) source_point<P, false>(gi, SIDE, slot, o.q);
+        }
+        __syncthreads();  // sources may share a point
+        if (images && on && o.i >= 0) {
+          const int x[3] = {o.i, o.j, o.k};
+          ghost_own<P, CX>(g, gi, o.comp, x, (int)g.src[o.q].offset);
         }
       }
     };
