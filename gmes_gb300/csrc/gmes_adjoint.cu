@@ -637,24 +637,28 @@ __device__ __forceinline__ void point_ae(const GridDev& g, const TmzDev& t, cons
 template <class P>
 __global__ void __launch_bounds__(kBX* kBY)
     k_tmz_fe(const GridDev g, const TmzDev t, int n, int slot) {
+  after_launch();
   Lat p;
   if (lattice_point(t, p)) point_fe<P>(g, t, p, n, slot);
 }
 template <class P>
 __global__ void __launch_bounds__(kBX* kBY)
     k_tmz_fh(const GridDev g, const TmzDev t, int n, int row) {
+  after_launch();
   Lat p;
   if (lattice_point(t, p)) point_fh<P>(g, t, p, n, row);
 }
 template <class P>
 __global__ void __launch_bounds__(kBX* kBY)
     k_tmz_ah(const GridDev g, const TmzDev t, int n, int rb, int wb) {
+  after_launch();
   Lat p;
   if (lattice_point(t, p)) point_ah<P>(g, t, p, n, rb, wb);
 }
 template <class P>
 __global__ void __launch_bounds__(kBX* kBY)
     k_tmz_ae(const GridDev g, const TmzDev t, int slot, int rb, int wb) {
+  after_launch();
   Lat p;
   if (lattice_point(t, p)) point_ae<P>(g, t, p, slot, rb, wb);
 }
@@ -2226,8 +2230,10 @@ cudaError_t forward(const GridDev& g, const TmzDev& t, int step0, int nsteps, in
   const dim3 grid = lattice_grid(t), block(kBX, kBY);
   for (int k = 0; k < nsteps; ++k) {
     const int n = step0 + k + 1;
-    k_tmz_fe<P><<<grid, block, 0, s>>>(g, t, n, (flags & GMES_TMZ_RECORD_HIST) ? k : -1);
-    k_tmz_fh<P><<<grid, block, 0, s>>>(g, t, n, (flags & GMES_TMZ_RECORD_MONITOR) ? n - 1 : -1);
+    launch_after(k > 0, k_tmz_fe<P>, grid, block, s, g, t, n,
+                 (flags & GMES_TMZ_RECORD_HIST) ? k : -1);
+    launch_after(true, k_tmz_fh<P>, grid, block, s, g, t, n,
+                 (flags & GMES_TMZ_RECORD_MONITOR) ? n - 1 : -1);
   }
   return cudaGetLastError();
 }
@@ -2252,8 +2258,8 @@ cudaError_t adjoint(const GridDev& g, const TmzDev& t, int step0, int nsteps, cu
   for (int k = nsteps - 1; k >= 0; --k) {
     const int n = step0 + k + 1;
     const int rb = n & 1, wb = rb ^ 1;
-    k_tmz_ah<P><<<grid, block, 0, s>>>(g, t, n, rb, wb);
-    k_tmz_ae<P><<<grid, block, 0, s>>>(g, t, k, rb, wb);
+    launch_after(k + 1 < nsteps, k_tmz_ah<P>, grid, block, s, g, t, n, rb, wb);
+    launch_after(true, k_tmz_ae<P>, grid, block, s, g, t, k, rb, wb);
   }
   return cudaGetLastError();
 }

@@ -204,6 +204,34 @@ struct GridDev {
   int64_t fst[3][2];
 };
 
+// Programmatic launches: a kernel that begins with after_launch() may be
+// launched with `early`, so that its blocks come up as those of the kernel
+// before it drain; it then waits for that kernel to have finished and reads
+// only afterwards what it wrote.  Every thread waits, first of all, so that a
+// kernel's end means the end of all before it.  The first launch of a call, and
+// one after a kernel of another kind, is a plain one.  What this hides is the
+// start of a kernel behind the end of the one before, some 0.7 us of a launch.
+// Measured on GB300, us per step of 4 to 6 launches: 64^3 FP32 19.5 -> 18.5, 128^3
+// 69.4 -> 66.4, 256^3 389 -> 384, FP64 868 -> 865, df64 605 -> 601;
+// 131x97x163 FP32 dispersive 74.3 -> 72.6.
+__device__ __forceinline__ void after_launch() {
+  asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+}
+template <class... K, class... A>
+void launch_after(bool early, void (*kernel)(K...), dim3 grid, dim3 threads, cudaStream_t s,
+                  A... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = threads;
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = early ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, K(args)...);
+}
+
 // Host-side launch plan of one grid: its real-plane view, the imaginary-
 // plane view of a complex grid, and the TFSF incident-field grid's plan.
 struct Plan {

@@ -187,6 +187,7 @@ struct ArgDescs<PolDF> {
 template <class P, int SIDE, bool STRICT, bool DISP, int MASK, class I>
 __global__ void __launch_bounds__(kCellThreads, CellMinBlocks<P, SIDE, DISP>::value)
     k_cell(const GridDev g, int bx_log2, int i0) {
+  after_launch();
   const int bx = 1 << bx_log2;
   const int tx = threadIdx.x & (bx - 1);
   const int ty = threadIdx.x >> bx_log2;
@@ -219,13 +220,14 @@ __global__ void __launch_bounds__(kCellThreads, CellMinBlocks<P, SIDE, DISP>::va
 template <class P, bool STRICT, int MASK, class I>
 void launch_cell(const GridDev& d, int side, bool disp, dim3 grid, int bx_log2, int i0,
                  cudaStream_t s) {
+  auto go = [&](auto kernel) { launch_after(true, kernel, grid, kCellThreads, s, d, bx_log2, i0); };
   if (side == 0) {
     if (disp)
-      k_cell<P, 0, STRICT, true, MASK, I><<<grid, kCellThreads, 0, s>>>(d, bx_log2, i0);
+      go(k_cell<P, 0, STRICT, true, MASK, I>);
     else
-      k_cell<P, 0, STRICT, false, MASK, I><<<grid, kCellThreads, 0, s>>>(d, bx_log2, i0);
+      go(k_cell<P, 0, STRICT, false, MASK, I>);
   } else {
-    k_cell<P, 1, STRICT, false, MASK, I><<<grid, kCellThreads, 0, s>>>(d, bx_log2, i0);
+    go(k_cell<P, 1, STRICT, false, MASK, I>);
   }
 }
 
@@ -267,6 +269,7 @@ __device__ __forceinline__ void ghost_point(const GridDev& g, int side, int item
 
 template <class T>
 __global__ void k_ghost(const GridDev g, int side, int64_t maxplane) {
+  after_launch();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= maxplane) return;
   ghost_point<T>(g, side, blockIdx.y, t);
@@ -277,6 +280,7 @@ __global__ void k_ghost(const GridDev g, int side, int64_t maxplane) {
 // one).  Same points, same copies.
 template <class T>
 __global__ void k_ghost32(const GridDev g, int side, unsigned maxplane) {
+  after_launch();
   const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= maxplane) return;
   const int item = blockIdx.y;
@@ -359,6 +363,7 @@ __device__ __forceinline__ void ghost_point_c(const GridDev& g, int side, int it
 
 template <bool STRICT>
 __global__ void k_ghost_c(const GridDev g, int side, int64_t maxplane) {
+  after_launch();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= maxplane) return;
   ghost_point_c<STRICT>(g, side, blockIdx.y, t);
@@ -368,6 +373,7 @@ __global__ void k_ghost_c(const GridDev g, int side, int64_t maxplane) {
 // that half's material update.  The values were computed on the host in FP64.
 template <class P, bool STRICT>
 __global__ void k_sources(const GridDev g, int side, int64_t slot) {
+  after_launch();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= g.nsrc) return;
   source_point<P, STRICT>(g, side, slot, q);
@@ -380,6 +386,7 @@ __global__ void k_sources(const GridDev g, int side, int64_t slot) {
 // reference's operation order (coef is the signed dt/(eps d) * amp).
 template <class P, bool STRICT>
 __global__ void k_transparent(const GridDev g, int side) {
+  after_launch();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= g.ntfsf) return;
   const gmes_transparent& t = g.tfsf[q];
@@ -421,6 +428,7 @@ __global__ void k_transparent(const GridDev g, int side) {
 // components after its updates, sources and TFSF corrections.
 template <class P>
 __global__ void k_probes(const GridDev g, int side, int64_t slot) {
+  after_launch();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= g.nprobe) return;
   const gmes_probe pr = g.probe[q];
@@ -463,6 +471,7 @@ static_assert(sizeof(GridDev) % 16 == 0, "GridDev is copied as 16-byte words");
 template <class P, int SIDE, bool STRICT, bool DISP>
 __global__ void __launch_bounds__(kBatchThreads, MultiMinBlocks<P, SIDE, DISP>::value)
     k_multi_cell(const BatchView v, int s, int64_t per) {
+  after_launch();
   __shared__ __align__(16) unsigned char desc[sizeof(GridDev)];
   const GridDev& g = *reinterpret_cast<const GridDev*>(desc);
   int cached = -1;
@@ -512,6 +521,7 @@ __global__ void __launch_bounds__(kBatchThreads, MultiMinBlocks<P, SIDE, DISP>::
 template <class P, int SIDE, bool STRICT, bool DISP>
 __global__ void __launch_bounds__(kBatchThreads, MultiMinBlocks<P, SIDE, DISP>::value)
     k_multi_cell_arg(const BatchView v, int s, int64_t per, const __grid_constant__ BatchDescs d) {
+  after_launch();
   const int64_t b0 = (int64_t)blockIdx.x * per;
   const int64_t b1 = b0 + per < v.tiles ? b0 + per : v.tiles;
   for (int64_t b = b0; b < b1; ++b) {
@@ -541,6 +551,7 @@ __global__ void __launch_bounds__(kBatchThreads, MultiMinBlocks<P, SIDE, DISP>::
 
 template <class T>
 __global__ void k_multi_ghost(const BatchView v, int side, int s) {
+  after_launch();
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < v.ghosts;
        t += (int64_t)gridDim.x * blockDim.x) {
     const int job = find_job<int64_t>(v.ghost_prefix, v.njobs, t);
@@ -554,6 +565,7 @@ __global__ void k_multi_ghost(const BatchView v, int side, int s) {
 
 template <class P, bool STRICT>
 __global__ void k_multi_sources(const BatchView v, int side, int s) {
+  after_launch();
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < v.srcs; t += gridDim.x * blockDim.x) {
     const int job = find_job<int>(v.src_prefix, v.njobs, t);
     if (s >= __ldg(v.steps + job)) continue;
@@ -571,7 +583,7 @@ cudaError_t run_steps(const Plan& p, int nsteps, int side_mask, int st0, cudaStr
 // A complex grid runs every per-plane kernel on its real and imaginary
 // planes; only the ghost copy couples them.
 template <class P, bool STRICT>
-void run_half(const Plan& p, int side, int st, cudaStream_t s) {
+void run_half(const Plan& p, int side, int st, bool early, cudaStream_t s) {
   using T = typename P::T;
   const GridDev& d = p.re;
   int64_t maxplane = 1;
@@ -584,11 +596,11 @@ void run_half(const Plan& p, int side, int st, cudaStream_t s) {
   const dim3 ggrid((unsigned)((maxplane + 255) / 256), 6);
   constexpr int kMaxY = 65535;
   if (p.cplx)
-    k_ghost_c<STRICT><<<ggrid, 256, 0, s>>>(d, 1 - side, maxplane);
+    launch_after(early, k_ghost_c<STRICT>, ggrid, 256, s, d, 1 - side, maxplane);
   else if (offsets_fit_i32(d))
-    k_ghost32<T><<<ggrid, 256, 0, s>>>(d, 1 - side, (unsigned)maxplane);
+    launch_after(early, k_ghost32<T>, ggrid, 256, s, d, 1 - side, (unsigned)maxplane);
   else
-    k_ghost<T><<<ggrid, 256, 0, s>>>(d, 1 - side, maxplane);
+    launch_after(early, k_ghost<T>, ggrid, 256, s, d, 1 - side, maxplane);
   const CellTiling tl = cell_tiling(d.n);
   const int bx_log2 = tl.bx_log2, bx = tl.bx, by = tl.by;
   const int nplanes = p.cplx ? 2 : 1;
@@ -611,9 +623,12 @@ void run_half(const Plan& p, int side, int st, cudaStream_t s) {
   for (int part = 0; part < nplanes; ++part) {
     const GridDev& v = part == 0 ? p.re : p.im;
     if (v.nsrc > 0)
-      k_sources<P, STRICT><<<(v.nsrc + 127) / 128, 128, 0, s>>>(v, side, 2 * (int64_t)st + side);
-    if (v.ntfsf > 0) k_transparent<P, STRICT><<<(v.ntfsf + 127) / 128, 128, 0, s>>>(v, side);
-    if (v.nprobe > 0) k_probes<P><<<(v.nprobe + 127) / 128, 128, 0, s>>>(v, side, st);
+      launch_after(true, k_sources<P, STRICT>, dim3((v.nsrc + 127) / 128), 128, s, v, side,
+                   2 * (int64_t)st + side);
+    if (v.ntfsf > 0)
+      launch_after(true, k_transparent<P, STRICT>, dim3((v.ntfsf + 127) / 128), 128, s, v, side);
+    if (v.nprobe > 0)
+      launch_after(true, k_probes<P>, dim3((v.nprobe + 127) / 128), 128, s, v, side, (int64_t)st);
   }
   if (side == 0 && p.incident != nullptr) {
     if (p.incident->word >= 0 && persist_takes(*p.incident))
@@ -626,8 +641,8 @@ void run_half(const Plan& p, int side, int st, cudaStream_t s) {
 template <class P, bool STRICT>
 cudaError_t run_steps(const Plan& p, int nsteps, int side_mask, int st0, cudaStream_t s) {
   for (int st = 0; st < nsteps; ++st) {
-    if (side_mask & 1) run_half<P, STRICT>(p, 0, st0 + st, s);
-    if (side_mask & 2) run_half<P, STRICT>(p, 1, st0 + st, s);
+    if (side_mask & 1) run_half<P, STRICT>(p, 0, st0 + st, st > 0, s);
+    if (side_mask & 2) run_half<P, STRICT>(p, 1, st0 + st, (st > 0 || (side_mask & 1)) && p.incident == nullptr, s);
   }
   return cudaGetLastError();
 }
@@ -664,29 +679,28 @@ cudaError_t run_batch(const BatchView& v, const GridDev* host_jobs, bool disp, i
     std::memset(&descs, 0, sizeof(descs));
     for (int q = 0; q < v.njobs; ++q) descs.jobs[q] = host_jobs[q];
   }
+  bool early = false;  // the first launch is a plain one
+  auto go = [&](auto kernel, int blocks_, int threads, auto... args) {
+    if (blocks_ <= 0) return;
+    launch_after(early, kernel, dim3((unsigned)blocks_), threads, st, v, args...);
+    early = true;
+  };
+  auto cell = [&](int s, auto by_arg, auto by_copy) {
+    if (arg)
+      go(by_arg, cells, kBatchThreads, s, per, descs);
+    else
+      go(by_copy, cells, kBatchThreads, s, per);
+  };
   for (int s = 0; s < nsteps; ++s) {
     for (int side = 0; side < 2; ++side) {
-      if (gblocks > 0) k_multi_ghost<T><<<gblocks, 256, 0, st>>>(v, 1 - side, s);
-      if (cells > 0) {
-        if (arg) {
-          if (side == 0) {
-            if (disp)
-              k_multi_cell_arg<P, 0, STRICT, true><<<cells, kBatchThreads, 0, st>>>(v, s, per, descs);
-            else
-              k_multi_cell_arg<P, 0, STRICT, false><<<cells, kBatchThreads, 0, st>>>(v, s, per, descs);
-          } else {
-            k_multi_cell_arg<P, 1, STRICT, false><<<cells, kBatchThreads, 0, st>>>(v, s, per, descs);
-          }
-        } else if (side == 0) {
-          if (disp)
-            k_multi_cell<P, 0, STRICT, true><<<cells, kBatchThreads, 0, st>>>(v, s, per);
-          else
-            k_multi_cell<P, 0, STRICT, false><<<cells, kBatchThreads, 0, st>>>(v, s, per);
-        } else {
-          k_multi_cell<P, 1, STRICT, false><<<cells, kBatchThreads, 0, st>>>(v, s, per);
-        }
-      }
-      if (sblocks > 0) k_multi_sources<P, STRICT><<<sblocks, 128, 0, st>>>(v, side, s);
+      go(k_multi_ghost<T>, gblocks, 256, 1 - side, s);
+      if (side == 1)
+        cell(s, k_multi_cell_arg<P, 1, STRICT, false>, k_multi_cell<P, 1, STRICT, false>);
+      else if (disp)
+        cell(s, k_multi_cell_arg<P, 0, STRICT, true>, k_multi_cell<P, 0, STRICT, true>);
+      else
+        cell(s, k_multi_cell_arg<P, 0, STRICT, false>, k_multi_cell<P, 0, STRICT, false>);
+      go(k_multi_sources<P, STRICT>, sblocks, 128, side, s);
     }
   }
   return cudaGetLastError();
