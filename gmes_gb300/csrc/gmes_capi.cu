@@ -614,7 +614,7 @@ gmes_status gmes_step(const gmes_grid_desc* g, int32_t nsteps, void* stream) {
   if (st != GMES_OK) return st;
   Plan inc;
   Plan p = make_plan(*g, &inc);
-  if (persist_takes(p) || (p.incident != nullptr && persist_takes(inc)))
+  if (persist_takes(p, nsteps) || (p.incident != nullptr && persist_takes(inc, 1)))
     p.word = inc.word = take_word(static_cast<cudaStream_t>(stream));
   cudaError_t e = launch_step(*g, p, nsteps, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "launching step kernels");
@@ -634,11 +634,11 @@ gmes_status gmes_step_launches(const gmes_grid_desc* g, int32_t nsteps, int64_t*
   };
   if (nsteps == 0)
     *launches = 0;
-  else if (persist_takes(p))
+  else if (persist_takes(p, nsteps))
     *launches = 1;
   else
     *launches = (int64_t)nsteps * (2 * per_half(p) + (p.incident == nullptr ? 0
-                                                      : persist_takes(inc)  ? 1
+                                                      : persist_takes(inc, 1) ? 1
                                                                             : 2 * per_half(inc)));
   return GMES_OK;
 }

@@ -518,7 +518,7 @@ int sm_count();
 // kRingWords are dealt in turn to direct launches, the others belong to
 // captured graphs.
 constexpr int kRingWords = 1024, kGraphWords = 4096;
-bool persist_takes(const Plan& p);
+bool persist_takes(const Plan& p, int nsteps);
 cudaError_t launch_persist(const Plan& p, int nsteps, int st0, cudaStream_t s);
 
 // Launchers implemented per precision in gmes_step.cu.

@@ -461,24 +461,34 @@ cudaError_t launch_disp(const Plan& p, int nsteps, int st0, cudaStream_t s) {
 //   TMz / TEz   200^2 FP64 15.4 -> 6.1, 301x277 FP64 19.9 -> 8.4 FP32 16.9 -> 7.6,
 //               1000x777 FP64 73.6 -> 26.4, 1400^2 FP64 159 -> 56 FP32 95 -> 32
 //               df64 132 -> 67, 2000^2 FP64 313 -> 127 FP32 189 -> 91
-//   3-D         48x40x44 FP64 22.9 -> 13.0, 64^3 FP64 35.7 -> 29.3, 72^3 FP64
-//               44.1 -> 37.0 FP32 23.9 -> 22.2, 80^3 FP64 48.8 -> 44.1 FP32
-//               25.5 -> 26.7 df64 35.5 -> 37.2, 96^3 FP64 70.9 -> 72.2
-//   3-D media   63x45x37 Drude / Lorentz / DCP + UPML FP64 38.9 -> 24.8, 80^3
-//               73.9 -> 79.1
-//   complex     64x64x48 39.7 -> 29.7, 80^3 65.5 -> 59.6, 96^3 101.9 -> 96.4
 // Grids of at most three components gain at every size (only their active
-// components' points are visited, with the inactive curl terms left out);
-// 3-D ones while their launches weigh more than the one-plane kernel's
-// shared neighbour loads.
-constexpr int64_t kPersistCells = 3 << 17, kPersistCellsComplex = 1 << 20;
+// components' points are visited, with the inactive curl terms left out), from
+// the first step on (64^2 FP64 19.1 -> 17.1, 301x277 20.9 -> 20.4).  3-D grids
+// gain while their launches weigh more than the one-plane kernel's shared
+// neighbour loads, and in calls long enough for the tables; with the launches
+// overlapped, a call of 1 / 2 / 4 / 20 steps:
+//   48x40x44 FP64   26.9 -> 30.9   25.8 -> 23.4   25.4 -> 19.3   25.0 -> 15.9
+//            FP32   21.2 -> 25.1   18.7 -> 16.5   17.2 -> 12.9   16.7 ->  9.8
+//            df64   22.5 -> 26.9   20.0 -> 19.2   19.0 -> 14.9   18.5 -> 11.8
+//   24^3     FP64   26.3 -> 22.0   22.3 -> 14.8   21.1 -> 10.9   21.0 ->  7.6
+//   32^3     FP32   21.5 -> 21.1   18.0 -> 13.5   16.0 -> 10.0   15.7 ->  7.0
+//   64^3     FP64   38.7 -> 54.0   36.3 -> 45.6   34.7 -> 41.0   33.8 -> 37.0
+//            FP32   25.0 -> 36.0   22.1 -> 26.9   20.0 -> 22.3   18.9 -> 18.6
+//   63x45x37 Drude / Lorentz / DCP + UPML
+//            FP64   42.8 -> 37.5   40.5 -> 30.9   38.6 -> 27.1   37.7 -> 24.0
+//   complex 32x32x30 28.6 -> 20.9  25.6 -> 14.7   24.7 -> 11.9   27.1 ->  9.4
+//   complex 64x64x48 41.5 -> 41.5  39.8 -> 35.0   38.5 -> 32.3   37.5 -> 29.4
+constexpr int64_t kPersistCells = 1 << 17, kPersistCellsComplex = 1 << 18;
+constexpr int64_t kPersistCellsOneStep = 1 << 15;
 
-bool persist_takes(const Plan& p) {
+bool persist_takes(const Plan& p, int nsteps) {
   const GridDev& d = p.re;
   if (p.precision == GMES_FP64_STRICT || wait_error_word() == nullptr) return false;
   if (d.nsrc > kPersistSources || d.ntfsf > 0 || d.nprobe > 0 || !offsets_fit_i32(d)) return false;
   if (__builtin_popcount((unsigned)d.active) <= 3) return true;
-  return (int64_t)d.n[0] * d.n[1] * d.n[2] <= (p.cplx ? kPersistCellsComplex : kPersistCells);
+  const int64_t most =
+      nsteps == 1 ? kPersistCellsOneStep : (p.cplx ? kPersistCellsComplex : kPersistCells);
+  return (int64_t)d.n[0] * d.n[1] * d.n[2] <= most;
 }
 
 cudaError_t launch_persist(const Plan& p, int nsteps, int st0, cudaStream_t s) {

@@ -631,7 +631,7 @@ void run_half(const Plan& p, int side, int st, bool early, cudaStream_t s) {
       launch_after(true, k_probes<P>, dim3((v.nprobe + 127) / 128), 128, s, v, side, (int64_t)st);
   }
   if (side == 0 && p.incident != nullptr) {
-    if (p.incident->word >= 0 && persist_takes(*p.incident))
+    if (p.incident->word >= 0 && persist_takes(*p.incident, 1))
       launch_persist(*p.incident, 1, st, s);
     else
       run_steps<P, STRICT>(*p.incident, 1, 3, st, s);
@@ -770,7 +770,7 @@ cudaError_t launch_nonfinite(const gmes_grid_desc& g, const GridDev& d, int32_t*
 }
 
 cudaError_t launch_step(const gmes_grid_desc& g, const Plan& p, int nsteps, cudaStream_t s) {
-  if (p.word >= 0 && persist_takes(p)) return launch_persist(p, nsteps, 0, s);
+  if (p.word >= 0 && persist_takes(p, nsteps)) return launch_persist(p, nsteps, 0, s);
   return dispatch_precision(g, p, nsteps, 3, 0, s);
 }
 

@@ -69,7 +69,7 @@ CASES = {
     "cube_many_classes": dict(cls=G.FDTD, size=(2.4, 2.0, 2.2), many=True),
     "cube_two_layers": dict(cls=G.FDTD, size=(2.4, 2.4, 2.0), pml="two"),
     "cube_dcp_upml": dict(cls=G.FDTD, size=(2.2, 2.0, 1.9), medium="dcp", pml="upml"),
-    "cube_two_rounds": dict(cls=G.FDTD, size=(6.5, 5.7, 6.1), medium="drude"),
+    "cube_two_rounds": dict(cls=G.FDTD, size=(5.1, 5.3, 4.8), medium="drude"),
     "tmz_wide": dict(cls=G.TMzFDTD, size=(30.1, 44.3, 0), medium="dcp"),
 }
 RUN = [(n, p) for n in CASES for p in ("fp64", "fp32", "df64")]
