@@ -43,12 +43,14 @@
 // look-ups every step; CPML points inside a profile go through the
 // per-point functions below.
 //
-// Two kernel forms.  The one-step kernels advance every lattice point by
-// one half-step per launch.  The temporally blocked kernels (FP32) advance
-// a tile of one design by up to kTbHalo steps per launch from a region of
-// shared memory (see k_tmz_tb_fwd).  Both use the same map and per-point
+// Three kernel forms.  The one-step kernels advance every lattice point by one
+// half-step per launch; up to some millions of points the steps of a call are
+// one cooperative launch of the same bodies (k_tmz_chunk_fwd, k_tmz_chunk_adj).
+// The temporally blocked kernels (FP32) advance a tile of one design by up to
+// kTbHalo steps per launch from a region in registers (see k_tmz_tb_fwd), or in
+// shared memory for tiles of mixed points.  All use the same map and arithmetic
 // functions, and this file is compiled without implicit multiply-add
-// contraction (every fused operation is an explicit fmadd), so the two
+// contraction (every fused operation is an explicit fmadd), so the
 // forms give bit-identical fields, adjoints and gradients.
 #include "gmes_barrier.cuh"
 
