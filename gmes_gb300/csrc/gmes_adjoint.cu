@@ -2399,7 +2399,7 @@ cudaError_t launch_tmz_design(int precision, const GridDev& g, const TmzDev& t,
       return cudaErrorInvalidValue;
   }
   if (t.nsrc > 0) k_tmz_map_sources<<<(t.nsrc + 127) / 128, 128, 0, s>>>(t);
-  if (precision == GMES_FP32 && t.tmp[0] != nullptr)
+  if (precision == GMES_FP32)
     k_tmz_tiles<PolF32, kTbQ><<<tb_tiles<PolF32, kTbQ>(t), kTbThreads, 0, s>>>(t);
   return cudaGetLastError();
 }

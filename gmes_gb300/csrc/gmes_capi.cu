@@ -974,10 +974,12 @@ TmzLayout tmz_layout(const gmes_grid_desc& g, const gmes_tmz_batch& b) {
   L.design_coef = align256((int64_t)b.nbatch * nd * (int64_t)sizeof(DesignCoef));
   L.map_flags = align256(plane * 4);
   L.map_coef = align256(plane * es);
-  // at most one tile per 8 x 8 lattice points, plus the edges
-  L.tiles = tmz_blocked(g, b) ? align256(((int64_t)g.n[0] / 8 + 1) * ((int64_t)g.n[1] / 8 + 1) *
-                                         (int64_t)sizeof(TbTile<double>))
-                              : 0;
+  // at most one tile per 8 x 8 lattice points, plus the edges (whatever
+  // block_steps is now: it may change between calls)
+  L.tiles = g.precision == GMES_FP32
+                ? align256(((int64_t)g.n[0] / 8 + 1) * ((int64_t)g.n[1] / 8 + 1) *
+                           (int64_t)sizeof(TbTile<double>))
+                : 0;
   L.design = L.design_coef + L.map_flags + 4 * L.map_coef + L.tiles;
   L.hist = align256((int64_t)b.hist_steps * b.nbatch * nd * es);
   L.monitor = align256((int64_t)b.nbatch * b.total_steps * nm * 8);
@@ -1052,7 +1054,7 @@ TmzDev make_tmz_dev(const gmes_grid_desc& g, const gmes_tmz_batch& b) {
   t.pflags = reinterpret_cast<const uint32_t*>(map);
   for (int k = 0; k < 4; ++k) t.pcoef[k] = map + L.map_flags + k * L.map_coef;
   char* after = static_cast<char*>(b.design) + L.design_coef + L.map_flags + 4 * L.map_coef;
-  if (tmz_blocked(g, b)) t.tiles = after;
+  if (g.precision == GMES_FP32) t.tiles = after;
   t.word = -1;
   t.hist = b.hist;
   t.mon = b.monitor;

@@ -73,3 +73,29 @@ def test_more_sources_than_places():
     assert np.abs(one[8]).max() > 0
     for k, (a, b) in enumerate(zip(one, four)):
         assert np.array_equal(a, b), k
+
+
+def test_block_steps_may_change_after_the_design_is_set():
+    import ctypes as C
+
+    from gmes_gb300 import _native as N
+    from gmes_gb300.adjoint import TMzAdjoint
+    args = _args(130, 140)
+    eps = np.random.default_rng(4).uniform(1.0, 9.0, (2, 9, 8))
+    prob = TMzAdjoint(*args, batch=2, precision="fp32", courant_ratio=0.9)
+    prob.forward(eps)
+    want = [prob.lattice(k).cpu().numpy() for k in range(7)]
+    st = C.c_void_p(prob.grid.stream)
+    prob.grid._enter()
+    prob.design.fill_(0xab)  # nothing of the first design is left
+    prob.grid._leave()
+    prob.grid.synchronize()
+    scratch, prob.desc.scratch, prob.desc.block_steps = prob.desc.scratch, None, 1
+    prob._call("gmes_tmz_set_design", C.c_void_p(prob.eps.data_ptr()), st)
+    prob.desc.scratch, prob.desc.block_steps = scratch, 4
+    prob._call("gmes_tmz_reset", 1, st)
+    prob._call("gmes_tmz_forward", 0, prob.nsteps, N.TMZ_RECORD_MONITOR, st)
+    prob.grid.synchronize()
+    assert np.abs(want[0]).max() > 0
+    for k, w in enumerate(want):
+        assert np.array_equal(prob.lattice(k).cpu().numpy(), w), k
