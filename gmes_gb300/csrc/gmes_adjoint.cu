@@ -1776,6 +1776,7 @@ __device__ __forceinline__ void tb_dispatch(const TbTile<R>& tile, F& steps) {
 template <class P, int Q>
 __global__ void __launch_bounds__(kTbThreads, 2)
     k_tmz_tb_fwd(const GridDev g, const TmzDev t, int n0, int nsub, int slot0, int rec_mon) {
+  after_launch();
   using R = typename P::R;
   using G = TbGeom<P, Q>;
   using Two = Row2<R>;
@@ -1904,6 +1905,7 @@ __global__ void __launch_bounds__(kTbThreads, 2)
 template <class P, int Q>
 __global__ void __launch_bounds__(kTbThreads, 2)
     k_tmz_tb_adj(const GridDev g, const TmzDev t, int n0, int nsub, int step0, int rb) {
+  after_launch();
   using R = typename P::R;
   using G = TbGeom<P, Q>;
   using Two = Row2<R>;
@@ -2232,9 +2234,9 @@ cudaError_t forward(const GridDev& g, const TmzDev& t, int step0, int nsteps, in
   const dim3 grid = lattice_grid(t), block(kBX, kBY);
   for (int k = 0; k < nsteps; ++k) {
     const int n = step0 + k + 1;
-    launch_after(k > 0, k_tmz_fe<P>, grid, block, s, g, t, n,
+    launch_after(k > 0, k_tmz_fe<P>, grid, block, 0, s, g, t, n,
                  (flags & GMES_TMZ_RECORD_HIST) ? k : -1);
-    launch_after(true, k_tmz_fh<P>, grid, block, s, g, t, n,
+    launch_after(true, k_tmz_fh<P>, grid, block, 0, s, g, t, n,
                  (flags & GMES_TMZ_RECORD_MONITOR) ? n - 1 : -1);
   }
   return cudaGetLastError();
@@ -2260,8 +2262,8 @@ cudaError_t adjoint(const GridDev& g, const TmzDev& t, int step0, int nsteps, cu
   for (int k = nsteps - 1; k >= 0; --k) {
     const int n = step0 + k + 1;
     const int rb = n & 1, wb = rb ^ 1;
-    launch_after(k + 1 < nsteps, k_tmz_ah<P>, grid, block, s, g, t, n, rb, wb);
-    launch_after(true, k_tmz_ae<P>, grid, block, s, g, t, k, rb, wb);
+    launch_after(k + 1 < nsteps, k_tmz_ah<P>, grid, block, 0, s, g, t, n, rb, wb);
+    launch_after(true, k_tmz_ae<P>, grid, block, 0, s, g, t, k, rb, wb);
   }
   return cudaGetLastError();
 }
@@ -2318,9 +2320,9 @@ cudaError_t forward_blocked(const GridDev& g, const TmzDev& t, int step0, int ns
   }
   for (int k = 0; k < nsteps; k += per_launch) {
     const int m = nsteps - k < per_launch ? nsteps - k : per_launch;
-    k_tmz_tb_fwd<P, Q><<<grid, kTbThreads, smem, s>>>(
-        g, u, step0 + k, m, (flags & GMES_TMZ_RECORD_HIST) ? k : -1,
-        (flags & GMES_TMZ_RECORD_MONITOR) ? 1 : 0);
+    launch_after(k > 0, k_tmz_tb_fwd<P, Q>, dim3(grid), kTbThreads, smem, s, g, u, step0 + k, m,
+                 (flags & GMES_TMZ_RECORD_HIST) ? k : -1,
+                 (flags & GMES_TMZ_RECORD_MONITOR) ? 1 : 0);
     swap_fields(u);
   }
   return cudaGetLastError();
@@ -2362,7 +2364,8 @@ cudaError_t adjoint_blocked(const GridDev& g, const TmzDev& t, int step0, int ns
   for (int q = 0; q < launches; ++q) {
     // launch q takes an even share of the steps left
     const int m = (hi + (launches - q) - 1) / (launches - q);
-    k_tmz_tb_adj<P, Q><<<grid, kTbThreads, smem, s>>>(g, u, step0 + hi - m, m, step0, rb);
+    launch_after(q > 0, k_tmz_tb_adj<P, Q>, dim3(grid), kTbThreads, smem, s, g, u,
+                 step0 + hi - m, m, step0, rb);
     swap_adjoints(u);
     rb ^= 1;
     hi -= m;

@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kCellThreads, CellMinBlocks<P, SIDE, DISP>::va
 template <class P, bool STRICT, int MASK, class I>
 void launch_cell(const GridDev& d, int side, bool disp, dim3 grid, int bx_log2, int i0,
                  cudaStream_t s) {
-  auto go = [&](auto kernel) { launch_after(true, kernel, grid, kCellThreads, s, d, bx_log2, i0); };
+  auto go = [&](auto kernel) { launch_after(true, kernel, grid, kCellThreads, 0, s, d, bx_log2, i0); };
   if (side == 0) {
     if (disp)
       go(k_cell<P, 0, STRICT, true, MASK, I>);
@@ -596,11 +596,11 @@ void run_half(const Plan& p, int side, int st, bool early, cudaStream_t s) {
   const dim3 ggrid((unsigned)((maxplane + 255) / 256), 6);
   constexpr int kMaxY = 65535;
   if (p.cplx)
-    launch_after(early, k_ghost_c<STRICT>, ggrid, 256, s, d, 1 - side, maxplane);
+    launch_after(early, k_ghost_c<STRICT>, ggrid, 256, 0, s, d, 1 - side, maxplane);
   else if (offsets_fit_i32(d))
-    launch_after(early, k_ghost32<T>, ggrid, 256, s, d, 1 - side, (unsigned)maxplane);
+    launch_after(early, k_ghost32<T>, ggrid, 256, 0, s, d, 1 - side, (unsigned)maxplane);
   else
-    launch_after(early, k_ghost<T>, ggrid, 256, s, d, 1 - side, maxplane);
+    launch_after(early, k_ghost<T>, ggrid, 256, 0, s, d, 1 - side, maxplane);
   const CellTiling tl = cell_tiling(d.n);
   const int bx_log2 = tl.bx_log2, bx = tl.bx, by = tl.by;
   const int nplanes = p.cplx ? 2 : 1;
@@ -623,12 +623,12 @@ void run_half(const Plan& p, int side, int st, bool early, cudaStream_t s) {
   for (int part = 0; part < nplanes; ++part) {
     const GridDev& v = part == 0 ? p.re : p.im;
     if (v.nsrc > 0)
-      launch_after(true, k_sources<P, STRICT>, dim3((v.nsrc + 127) / 128), 128, s, v, side,
+      launch_after(true, k_sources<P, STRICT>, dim3((v.nsrc + 127) / 128), 128, 0, s, v, side,
                    2 * (int64_t)st + side);
     if (v.ntfsf > 0)
-      launch_after(true, k_transparent<P, STRICT>, dim3((v.ntfsf + 127) / 128), 128, s, v, side);
+      launch_after(true, k_transparent<P, STRICT>, dim3((v.ntfsf + 127) / 128), 128, 0, s, v, side);
     if (v.nprobe > 0)
-      launch_after(true, k_probes<P>, dim3((v.nprobe + 127) / 128), 128, s, v, side, (int64_t)st);
+      launch_after(true, k_probes<P>, dim3((v.nprobe + 127) / 128), 128, 0, s, v, side, (int64_t)st);
   }
   if (side == 0 && p.incident != nullptr) {
     if (p.incident->word >= 0 && persist_takes(*p.incident, 1))
@@ -682,7 +682,7 @@ cudaError_t run_batch(const BatchView& v, const GridDev* host_jobs, bool disp, i
   bool early = false;  // the first launch is a plain one
   auto go = [&](auto kernel, int blocks_, int threads, auto... args) {
     if (blocks_ <= 0) return;
-    launch_after(early, kernel, dim3((unsigned)blocks_), threads, st, v, args...);
+    launch_after(early, kernel, dim3((unsigned)blocks_), threads, 0, st, v, args...);
     early = true;
   };
   auto cell = [&](int s, auto by_arg, auto by_copy) {
