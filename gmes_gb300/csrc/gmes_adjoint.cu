@@ -422,8 +422,8 @@ __device__ __forceinline__ bool hard_source(const TmzDev& t, unsigned fl, int k,
 template <class P>
 __device__ __forceinline__ void e_coef(const TmzDev& t, int b, int i, int j, int64_t ll,
                                        unsigned fl, typename P::R& c1, typename P::R& c2n) {
-  c1 = P::ld(map_coef<P>(t, 0) + ll);
-  c2n = P::ld(map_coef<P>(t, 1) + ll);
+  c1 = P::ldc(map_coef<P>(t, 0) + ll);
+  c2n = P::ldc(map_coef<P>(t, 1) + ll);
   if (fl & kTmzDesign) {
     const DesignCoef* dc = t.dc + (int64_t)b * t.dn[0] * t.dn[1] + design_index(t, i, j);
     c1 = P::cfg(&dc->c1);
@@ -439,7 +439,7 @@ __device__ __forceinline__ typename P::R weight_x(const GridDev& g, const TmzDev
                                                   int64_t ll, int64_t base, int rb, int wb) {
   using T = typename P::T;
   const T* lx = static_cast<const T*>(t.l[1]) + base + ll;
-  const typename P::R c = P::ld(map_coef<P>(t, 2) + ll);  // issued with the flags
+  const typename P::R c = P::ldc(map_coef<P>(t, 2) + ll);  // issued with the flags
   const unsigned fl = __ldg(t.pflags + ll);
   const typename P::R l = hard_source(t, fl, 1, ll) ? P::zero() : P::ldw(lx);
   if (fl & kTmzPlainX) return c * l;
@@ -454,7 +454,7 @@ __device__ __forceinline__ typename P::R weight_y(const GridDev& g, const TmzDev
                                                   int64_t ll, int64_t base, int rb, int wb) {
   using T = typename P::T;
   const T* ly = static_cast<const T*>(t.l[2]) + base + ll;
-  const typename P::R c = P::ld(map_coef<P>(t, 3) + ll);  // issued with the flags
+  const typename P::R c = P::ldc(map_coef<P>(t, 3) + ll);  // issued with the flags
   const unsigned fl = __ldg(t.pflags + ll);
   const typename P::R l = hard_source(t, fl, 2, ll) ? P::zero() : P::ldw(ly);
   if (fl & kTmzPlainY) return c * l;
@@ -521,7 +521,7 @@ __device__ __forceinline__ void point_fe(const GridDev& g, const TmzDev& t, cons
             fmadd(c2n * D2, c1, D1));
     }
   } else if (fl & kTmzPsiE) {
-    r = e_cpml<P>(g, fl, P::ld(map_coef<P>(t, 0) + p.lin), p.i, p.j, e, D1, D2,
+    r = e_cpml<P>(g, fl, P::ldc(map_coef<P>(t, 0) + p.lin), p.i, p.j, e, D1, D2,
                   static_cast<T*>(t.f[3]) + p.base + p.lin,
                   static_cast<T*>(t.f[4]) + p.base + p.lin);
   }
@@ -539,7 +539,7 @@ __device__ __forceinline__ void point_fh(const GridDev& g, const TmzDev& t, cons
   T* X = static_cast<T*>(t.f[1]) + p.base;
   T* Y = static_cast<T*>(t.f[2]) + p.base;
   const unsigned fl = __ldg(t.pflags + p.lin);
-  const R cxn = P::ld(map_coef<P>(t, 2) + p.lin), cy = P::ld(map_coef<P>(t, 3) + p.lin);
+  const R cxn = P::ldc(map_coef<P>(t, 2) + p.lin), cy = P::ldc(map_coef<P>(t, 3) + p.lin);
   const R e0 = P::ldw(E + p.lin);
   const R dx = P::ldw(E + (int64_t)p.i * t.ny + jp) - e0;  // D1 of Hx
   const R dy = P::ldw(E + (int64_t)ip * t.ny + p.j) - e0;  // D2 of Hy
@@ -1347,7 +1347,7 @@ struct TbSpecial {
   __device__ __forceinline__ void grad_fetch(const TmzDev& t, const TbPlace<P, Q>& p, int slot) {
     const int64_t b = ((int64_t)slot * t.nb + p.b) * t.dn[0] * t.dn[1];
     pixels(t, p, [&](int q, int h, int64_t dp) {
-      v[q][h] = P::ld(static_cast<const T*>(t.hist) + b + dp);
+      v[q][h] = P::ldw(static_cast<const T*>(t.hist) + b + dp);
     });
   }
   __device__ __forceinline__ void grad_add(const TmzDev& t, const TbPlace<P, Q>& p, int q,
@@ -1418,8 +1418,8 @@ __device__ __forceinline__ unsigned tb_point(const TmzDev& t, int b, int i, int 
   const int64_t ll = (int64_t)i * t.ny + j;
   const unsigned f = __ldg(t.pflags + ll);
   e_coef<P>(t, b, i, j, ll, f, p.c1, p.c2n);
-  p.cxn = P::ld(map_coef<P>(t, 2) + ll);
-  p.cy = P::ld(map_coef<P>(t, 3) + ll);
+  p.cxn = P::ldc(map_coef<P>(t, 2) + ll);
+  p.cy = P::ldc(map_coef<P>(t, 3) + ll);
   return f;
 }
 
@@ -1481,15 +1481,15 @@ __device__ void tb_general_fwd(const GridDev& g, const TmzDev& t, int n0, int ns
     fl[q] = tb_point<P>(t, b, li[q], j, pt[q]);
     if (jtile && a >= H && a < H + TI && ri0 + a < t.nx) fl[q] |= 1u << 31;  // tile point
     const int64_t lin = base + (int64_t)li[q] * t.ny + j;
-    sE[k] = __ldg(static_cast<const T*>(t.f[0]) + lin);
-    sX[k] = __ldg(static_cast<const T*>(t.f[1]) + lin);
-    sY[k] = __ldg(static_cast<const T*>(t.f[2]) + lin);
+    sE[k] = static_cast<const T*>(t.f[0])[lin];
+    sX[k] = static_cast<const T*>(t.f[1])[lin];
+    sY[k] = static_cast<const T*>(t.f[2])[lin];
     if (fl[q] & kTmzPsiE) {
-      sS[k] = __ldg(static_cast<const T*>(t.f[3]) + lin);
-      sS[NP + k] = __ldg(static_cast<const T*>(t.f[4]) + lin);
+      sS[k] = static_cast<const T*>(t.f[3])[lin];
+      sS[NP + k] = static_cast<const T*>(t.f[4])[lin];
     }
-    if (fl[q] & kTmzPsiX) sS[2 * NP + k] = __ldg(static_cast<const T*>(t.f[5]) + lin);
-    if (fl[q] & kTmzPsiY) sS[3 * NP + k] = __ldg(static_cast<const T*>(t.f[6]) + lin);
+    if (fl[q] & kTmzPsiX) sS[2 * NP + k] = static_cast<const T*>(t.f[5])[lin];
+    if (fl[q] & kTmzPsiY) sS[3 * NP + k] = static_cast<const T*>(t.f[6])[lin];
   }
   unsigned any = 0;
 #pragma unroll
@@ -2074,7 +2074,7 @@ __global__ void __launch_bounds__(kTbThreads) k_tmz_tiles(const TmzDev t) {
     return (f & bit[k]) != 0;
   };
   auto coef = [&](int64_t ll, int k) {
-    return P::ld(map_coef<P>(t, k < 4 ? k : (k == 4 ? 0 : k - 3)) + ll);
+    return P::ldc(map_coef<P>(t, k < 4 ? k : (k == 4 ? 0 : k - 3)) + ll);
   };
   unsigned any = 0;
   int first[7] = {-1, -1, -1, -1, -1, -1, -1}, pm_any = -1;

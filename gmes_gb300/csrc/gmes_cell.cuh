@@ -603,13 +603,13 @@ __device__ __forceinline__ bool is_active(const GridDev& g) {
     return (g.active >> C) & 1;
 }
 
-// COH: the field may have been written by another block of this launch (the
-// persistent kernel), so it is read coherently.
-template <class P, int MASK, int C, bool COH = false, class I>
+// Fields are read with plain loads: the kernels that call this come up while the
+// kernel before them still writes (after_launch), or step several times in one
+// launch, and a read-only load is for data that nobody writes meanwhile.
+template <class P, int MASK, int C, class I>
 __device__ __forceinline__ typename P::R ldf(const GridDev& g, I off) {
   if (!is_active<MASK, C>(g)) return P::zero();
-  const typename P::T* p = static_cast<const typename P::T*>(g.f[C]) + off;
-  return COH ? P::ldw(p) : P::ld(p);
+  return P::ldw(static_cast<const typename P::T*>(g.f[C]) + off);
 }
 
 template <int MASK, int C, class I>
@@ -788,7 +788,7 @@ struct EarlyCoef {
 // 42.54 -> 30.1 / 29.7 / 34.3 / 31.1 Gcell/s at 6 / 7 / 8 / 10 blocks per SM
 // (64 registers at 8), dispersive FP32 25.42 -> 22.35; df64 (5, 6 blocks)
 // 26.74 -> 17.5 / 20.7, FP64 (6 blocks) 19.25 -> 16.99.
-template <class P, int SIDE, bool DISP, int MASK, class I, bool COH = false>
+template <class P, int SIDE, bool DISP, int MASK, class I>
 __device__ __forceinline__ void cell_body_fast(const GridDev& g, int i, int j, int k) {
   using R = typename P::R;
   using T = typename P::T;
@@ -804,32 +804,32 @@ __device__ __forceinline__ void cell_body_fast(const GridDev& g, int i, int j, i
   const I l0 = SIDE == 0 ? oX : oX + X1 + 1;
   const I l1 = SIDE == 0 ? oY : oY + Y0 + 1;
   const I l2 = SIDE == 0 ? oZ : oZ + Z0 + Z1;
-  const R f0 = ldf<P, MASK, c0, COH>(g, l0), f1 = ldf<P, MASK, c0 + 1, COH>(g, l1),
-          f2 = ldf<P, MASK, c0 + 2, COH>(g, l2);
+  const R f0 = ldf<P, MASK, c0>(g, l0), f1 = ldf<P, MASK, c0 + 1>(g, l1),
+          f2 = ldf<P, MASK, c0 + 2>(g, l2);
   R d01, d02, d11, d12, d21, d22;  // (D1, D2) of each component
   if constexpr (SIDE == 0) {
-    const R hz_a = ldf<P, MASK, 5, COH>(g, oZ + Z0 + Z1);  // Hz[i+1, j+1, k]
-    const R hz_b = ldf<P, MASK, 5, COH>(g, oZ + Z0);       // Hz[i+1, j,   k]
-    const R hz_c = ldf<P, MASK, 5, COH>(g, oZ + Z1);       // Hz[i,   j+1, k]
-    const R hy_a = ldf<P, MASK, 4, COH>(g, oY + Y0 + 1);   // Hy[i+1, j, k+1]
-    const R hy_b = ldf<P, MASK, 4, COH>(g, oY + Y0);       // Hy[i+1, j, k]
-    const R hy_c = ldf<P, MASK, 4, COH>(g, oY + 1);        // Hy[i,   j, k+1]
-    const R hx_a = ldf<P, MASK, 3, COH>(g, oX + X1 + 1);   // Hx[i, j+1, k+1]
-    const R hx_b = ldf<P, MASK, 3, COH>(g, oX + X1);       // Hx[i, j+1, k]
-    const R hx_c = ldf<P, MASK, 3, COH>(g, oX + 1);        // Hx[i, j,   k+1]
+    const R hz_a = ldf<P, MASK, 5>(g, oZ + Z0 + Z1);  // Hz[i+1, j+1, k]
+    const R hz_b = ldf<P, MASK, 5>(g, oZ + Z0);       // Hz[i+1, j,   k]
+    const R hz_c = ldf<P, MASK, 5>(g, oZ + Z1);       // Hz[i,   j+1, k]
+    const R hy_a = ldf<P, MASK, 4>(g, oY + Y0 + 1);   // Hy[i+1, j, k+1]
+    const R hy_b = ldf<P, MASK, 4>(g, oY + Y0);       // Hy[i+1, j, k]
+    const R hy_c = ldf<P, MASK, 4>(g, oY + 1);        // Hy[i,   j, k+1]
+    const R hx_a = ldf<P, MASK, 3>(g, oX + X1 + 1);   // Hx[i, j+1, k+1]
+    const R hx_b = ldf<P, MASK, 3>(g, oX + X1);       // Hx[i, j+1, k]
+    const R hx_c = ldf<P, MASK, 3>(g, oX + 1);        // Hx[i, j,   k+1]
     d01 = curl_diff(hz_a, hz_b); d02 = curl_diff(hy_a, hy_b);
     d11 = curl_diff(hx_a, hx_b); d12 = curl_diff(hz_a, hz_c);
     d21 = curl_diff(hy_a, hy_c); d22 = curl_diff(hx_a, hx_c);
   } else {
-    const R ez_0 = ldf<P, MASK, 2, COH>(g, oZ);       // Ez[i, j, k]
-    const R ez_j = ldf<P, MASK, 2, COH>(g, oZ + Z1);  // Ez[i, j+1, k]
-    const R ez_i = ldf<P, MASK, 2, COH>(g, oZ + Z0);  // Ez[i+1, j, k]
-    const R ey_0 = ldf<P, MASK, 1, COH>(g, oY);       // Ey[i, j, k]
-    const R ey_k = ldf<P, MASK, 1, COH>(g, oY + 1);   // Ey[i, j, k+1]
-    const R ey_i = ldf<P, MASK, 1, COH>(g, oY + Y0);  // Ey[i+1, j, k]
-    const R ex_0 = ldf<P, MASK, 0, COH>(g, oX);       // Ex[i, j, k]
-    const R ex_k = ldf<P, MASK, 0, COH>(g, oX + 1);   // Ex[i, j, k+1]
-    const R ex_j = ldf<P, MASK, 0, COH>(g, oX + X1);  // Ex[i, j+1, k]
+    const R ez_0 = ldf<P, MASK, 2>(g, oZ);       // Ez[i, j, k]
+    const R ez_j = ldf<P, MASK, 2>(g, oZ + Z1);  // Ez[i, j+1, k]
+    const R ez_i = ldf<P, MASK, 2>(g, oZ + Z0);  // Ez[i+1, j, k]
+    const R ey_0 = ldf<P, MASK, 1>(g, oY);       // Ey[i, j, k]
+    const R ey_k = ldf<P, MASK, 1>(g, oY + 1);   // Ey[i, j, k+1]
+    const R ey_i = ldf<P, MASK, 1>(g, oY + Y0);  // Ey[i+1, j, k]
+    const R ex_0 = ldf<P, MASK, 0>(g, oX);       // Ex[i, j, k]
+    const R ex_k = ldf<P, MASK, 0>(g, oX + 1);   // Ex[i, j, k+1]
+    const R ex_j = ldf<P, MASK, 0>(g, oX + X1);  // Ex[i, j+1, k]
     d01 = curl_diff(ez_j, ez_0); d02 = curl_diff(ey_k, ey_0);
     d11 = curl_diff(ex_k, ex_0); d12 = curl_diff(ez_i, ez_0);
     d21 = curl_diff(ey_i, ey_0); d22 = curl_diff(ex_j, ex_0);

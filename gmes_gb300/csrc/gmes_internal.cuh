@@ -307,7 +307,7 @@ __device__ __forceinline__ df operator*(df a, df b) {
 struct PolF64 {
   using T = double;
   using R = double;
-  static __device__ __forceinline__ R ld(const T* p) { return __ldg(p); }
+  static __device__ __forceinline__ R ldc(const T* p) { return __ldg(p); }
   static __device__ __forceinline__ R ldw(const T* p) { return *p; }
   static __device__ __forceinline__ void st(T* p, R v) { *p = v; }
   static __device__ __forceinline__ R cf(const Coef& c) { return c.d; }
@@ -319,7 +319,7 @@ struct PolF64 {
 struct PolF32 {
   using T = float;
   using R = float;
-  static __device__ __forceinline__ R ld(const T* p) { return __ldg(p); }
+  static __device__ __forceinline__ R ldc(const T* p) { return __ldg(p); }
   static __device__ __forceinline__ R ldw(const T* p) { return *p; }
   static __device__ __forceinline__ void st(T* p, R v) { *p = v; }
   static __device__ __forceinline__ R cf(const Coef& c) { return c.hi; }
@@ -331,7 +331,7 @@ struct PolF32 {
 struct PolDF {
   using T = float2;
   using R = df;
-  static __device__ __forceinline__ R ld(const T* p) {
+  static __device__ __forceinline__ R ldc(const T* p) {
     const float2 v = __ldg(p);
     return {v.x, v.y};
   }

@@ -152,7 +152,7 @@ struct Point {
   template <int B>
   __device__ __forceinline__ R at(const GridDev& g, int si, int sj, int sk) const {
     const int f0 = (int)g.fst[B % 3][0], f1 = (int)g.fst[B % 3][1];
-    return ldf<P, MASK, B, true>(g, (x[0] + si) * f0 + (x[1] + sj) * f1 + x[2] + sk);
+    return ldf<P, MASK, B>(g, (x[0] + si) * f0 + (x[1] + sj) * f1 + x[2] + sk);
   }
   __device__ __forceinline__ void diffs(const GridDev& g, R& p1, R& p2) const {
     constexpr int B1 = (E ? 3 : 0) + a2, B2 = (E ? 3 : 0) + a1;  // read by D1, D2
@@ -180,7 +180,7 @@ __device__ __forceinline__ void table_point(const GridDev& g, const unsigned cha
   using R = typename P::R;
   using T = typename P::T;
   const Point<P, C, MASK> pt(g, i, j, k);
-  const R F = ldf<P, MASK, C, true>(g, pt.l);
+  const R F = ldf<P, MASK, C>(g, pt.l);
   R p1, p2;
   pt.diffs(g, p1, p2);
   int id, kind = -1;
