@@ -42,7 +42,7 @@ def nvcc():
 def _digest(src, flags):
     h = hashlib.sha256()
     h.update(" ".join(flags).encode())
-    for p in sorted(list(CSRC.glob("*.cuh")) + [ROOT / "include" / "gmes_gb300.h", src]):
+    for p in sorted(list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + [ROOT / "include" / "gmes_gb300.h", src]):
         h.update(p.read_bytes())
     return h.hexdigest()[:16]
 

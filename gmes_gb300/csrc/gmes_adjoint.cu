@@ -683,18 +683,19 @@ __device__ __forceinline__ void for_points(const TmzDev& t, const LatDiv& d, F f
 template <class P>
 __global__ void __launch_bounds__(kChunkThreads, 2)
     k_tmz_chunk_fwd(const __grid_constant__ GridDev g, const __grid_constant__ TmzDev t,
-                    const LatDiv d, int step0, int nsteps, int flags, int* error) {
-  unsigned* const word = barrier_words + 8 * t.word;
+                    const LatDiv d, const __grid_constant__ Meeting meet, int step0, int nsteps, int flags, 
+                    int* error) {
   for (int k = 0; k < nsteps; ++k) {
     const int n = step0 + k + 1;
     for_points(t, d, [&](const Lat& p) {
       point_fe<P>(g, t, p, n, (flags & GMES_TMZ_RECORD_HIST) ? k : -1);
     });
-    if (!grid_barrier(word, error)) return;
+    if (!grid_barrier(meet, error)) return;
+    if (k + 1 == nsteps) leave_barrier(meet);
     for_points(t, d, [&](const Lat& p) {
       point_fh<P>(g, t, p, n, (flags & GMES_TMZ_RECORD_MONITOR) ? n - 1 : -1);
     });
-    if (k + 1 < nsteps && !grid_barrier(word, error)) return;
+    if (k + 1 < nsteps && !grid_barrier(meet, error)) return;
   }
 }
 
@@ -702,14 +703,14 @@ __global__ void __launch_bounds__(kChunkThreads, 2)
 template <class P>
 __global__ void __launch_bounds__(kChunkThreads, 2)
     k_tmz_chunk_adj(const __grid_constant__ GridDev g, const __grid_constant__ TmzDev t,
-                    const LatDiv d, int step0, int nsteps, int* error) {
-  unsigned* const word = barrier_words + 8 * t.word;
+                    const LatDiv d, const __grid_constant__ Meeting meet, int step0, int nsteps, int* error) {
   for (int k = nsteps - 1; k >= 0; --k) {
     const int n = step0 + k + 1, rb = n & 1, wb = rb ^ 1;
     for_points(t, d, [&](const Lat& p) { point_ah<P>(g, t, p, n, rb, wb); });
-    if (!grid_barrier(word, error)) return;
+    if (!grid_barrier(meet, error)) return;
+    if (k == 0) leave_barrier(meet);
     for_points(t, d, [&](const Lat& p) { point_ae<P>(g, t, p, k, rb, wb); });
-    if (k > 0 && !grid_barrier(word, error)) return;
+    if (k > 0 && !grid_barrier(meet, error)) return;
   }
 }
 
@@ -2215,19 +2216,20 @@ void map_sources(const TmzDev& t, cudaStream_t s) {
 }
 
 template <class P>
-cudaError_t forward(const GridDev& g, const TmzDev& t, int step0, int nsteps, int flags,
-                    cudaStream_t s) {
+cudaError_t forward(const GridDev& g, const TmzDev& t, const Meeting& meet, int step0, int nsteps,
+                    int flags, cudaStream_t s) {
   if (nsteps <= 0) return cudaSuccess;
   map_sources(t, s);
-  if (t.word >= 0) {
+  if (meet.slot >= 0) {
     LatDiv d;
     int blocks = 0;
     const cudaError_t e = chunk_shape(k_tmz_chunk_fwd<P>, t, d, blocks);
     if (e != cudaSuccess) return e;
     GridDev gg = g;
     TmzDev tt = t;
+    Meeting m = meet;
     int* error = wait_error_word();
-    void* args[] = {&gg, &tt, &d, &step0, &nsteps, &flags, &error};
+    void* args[] = {&gg, &tt, &d, &m, &step0, &nsteps, &flags, &error};
     return cudaLaunchCooperativeKernel((const void*)k_tmz_chunk_fwd<P>, dim3((unsigned)blocks),
                                        dim3(kChunkThreads), args, 0, s);
   }
@@ -2243,18 +2245,20 @@ cudaError_t forward(const GridDev& g, const TmzDev& t, int step0, int nsteps, in
 }
 
 template <class P>
-cudaError_t adjoint(const GridDev& g, const TmzDev& t, int step0, int nsteps, cudaStream_t s) {
+cudaError_t adjoint(const GridDev& g, const TmzDev& t, const Meeting& meet, int step0, int nsteps,
+                    cudaStream_t s) {
   if (nsteps <= 0) return cudaSuccess;
   map_sources(t, s);
-  if (t.word >= 0) {
+  if (meet.slot >= 0) {
     LatDiv d;
     int blocks = 0;
     const cudaError_t e = chunk_shape(k_tmz_chunk_adj<P>, t, d, blocks);
     if (e != cudaSuccess) return e;
     GridDev gg = g;
     TmzDev tt = t;
+    Meeting m = meet;
     int* error = wait_error_word();
-    void* args[] = {&gg, &tt, &d, &step0, &nsteps, &error};
+    void* args[] = {&gg, &tt, &d, &m, &step0, &nsteps, &error};
     return cudaLaunchCooperativeKernel((const void*)k_tmz_chunk_adj<P>, dim3((unsigned)blocks),
                                        dim3(kChunkThreads), args, 0, s);
   }
@@ -2434,35 +2438,37 @@ int64_t tmz_launches(int precision, const TmzDev& t, int block_steps, int nsteps
   return (t.nsrc > 0) + (tmz_chunked(precision, t, block_steps) ? 1 : 2 * (int64_t)nsteps);
 }
 
-cudaError_t launch_tmz_forward(int precision, const GridDev& g, const TmzDev& t, int step0,
-                               int nsteps, int flags, int block_steps, cudaStream_t s) {
+cudaError_t launch_tmz_forward(int precision, const GridDev& g, const TmzDev& t,
+                               const Meeting& meet, int step0, int nsteps, int flags,
+                               int block_steps, cudaStream_t s) {
   const int per = steps_per_launch(precision, t, block_steps);
   switch (precision) {
     case GMES_FP64:
-      return forward<PolF64>(g, t, step0, nsteps, flags, s);
+      return forward<PolF64>(g, t, meet, step0, nsteps, flags, s);
     case GMES_FP32:
       if (per > 1)
         return forward_blocked<PolF32, kTbQ>(g, t, step0, nsteps, flags, per, s);
-      return forward<PolF32>(g, t, step0, nsteps, flags, s);
+      return forward<PolF32>(g, t, meet, step0, nsteps, flags, s);
     case GMES_DF64:
-      return forward<PolDF>(g, t, step0, nsteps, flags, s);
+      return forward<PolDF>(g, t, meet, step0, nsteps, flags, s);
     default:
       return cudaErrorInvalidValue;
   }
 }
 
-cudaError_t launch_tmz_adjoint(int precision, const GridDev& g, const TmzDev& t, int step0,
-                               int nsteps, int block_steps, cudaStream_t s) {
+cudaError_t launch_tmz_adjoint(int precision, const GridDev& g, const TmzDev& t,
+                               const Meeting& meet, int step0, int nsteps, int block_steps,
+                               cudaStream_t s) {
   const int per = steps_per_launch(precision, t, block_steps);
   switch (precision) {
     case GMES_FP64:
-      return adjoint<PolF64>(g, t, step0, nsteps, s);
+      return adjoint<PolF64>(g, t, meet, step0, nsteps, s);
     case GMES_FP32:
       if (per > 1)
         return adjoint_blocked<PolF32, kTbQ>(g, t, step0, nsteps, per, s);
-      return adjoint<PolF32>(g, t, step0, nsteps, s);
+      return adjoint<PolF32>(g, t, meet, step0, nsteps, s);
     case GMES_DF64:
-      return adjoint<PolDF>(g, t, step0, nsteps, s);
+      return adjoint<PolDF>(g, t, meet, step0, nsteps, s);
     default:
       return cudaErrorInvalidValue;
   }

@@ -11,9 +11,12 @@ namespace {
 // and returns; every other block then gives up too.
 constexpr int kBarrierPolls = 1 << 22;
 
-// The barrier words, 32 bytes apart; each returns to zero low bits after every
-// barrier.
-__device__ unsigned barrier_words[8 * (kRingWords + kGraphWords)];
+// A barrier slot: the blocks' arrivals (zero low bits after every barrier) and
+// the blocks that have left the launch's last one.
+struct alignas(32) Slot {
+  unsigned word, left;
+};
+__device__ Slot slots[kStreamSlots + kGraphSlots];
 
 __device__ __forceinline__ unsigned load_acquire(const unsigned* p) {
   unsigned v;
@@ -31,11 +34,13 @@ __device__ __forceinline__ unsigned add_acq_rel(unsigned* p, unsigned v) {
 
 // All blocks of the (cooperative) launch arrive before any leaves.  Each adds
 // one, block 0 the rest of 2^31, so the word's top bit flips when the last
-// block has arrived and the low bits are zero again.  False: gave up.
-__device__ __forceinline__ bool grid_barrier(unsigned* word, int* error) {
+// block has arrived and the low bits are zero again (the arrival scheme of the
+// grid barrier in CUDA's cooperative groups header).  False: gave up.
+__device__ __forceinline__ bool grid_barrier(const Meeting& m, int* error) {
   __shared__ int good;
   __syncthreads();
   if (threadIdx.x == 0) {
+    unsigned* const word = &slots[m.slot].word;
     const unsigned old =
         add_acq_rel(word, blockIdx.x == 0 ? 0x80000000u - (gridDim.x - 1) : 1u);
     int n = 0;
@@ -45,6 +50,17 @@ __device__ __forceinline__ bool grid_barrier(unsigned* word, int* error) {
   }
   __syncthreads();
   return good != 0;
+}
+
+// After a launch's last barrier: once all its blocks are here, the slot may go
+// to another stream.
+__device__ __forceinline__ void leave_barrier(const Meeting& m) {
+  if (m.done == nullptr || threadIdx.x != 0) return;
+  Slot& s = slots[m.slot];
+  if (add_acq_rel(&s.left, 1u) != gridDim.x - 1) return;
+  s.left = 0;
+  __threadfence_system();
+  *static_cast<volatile uint32_t*>(m.done) = m.number;
 }
 
 }  // namespace

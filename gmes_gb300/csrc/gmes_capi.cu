@@ -7,14 +7,13 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
-#include <deque>
 #include <functional>
 #include <mutex>
 #include <string>
-#include <unordered_map>
 #include <vector>
 
 #include "gmes_internal.cuh"
+#include "gmes_slots.h"
 
 namespace gmes {
 namespace {
@@ -48,26 +47,34 @@ int elem_size(int32_t precision) {
   }
 }
 
-// The word that kernels set when a wait ran past its limit: pinned, allocated
-// once per process outside any stream capture (gmes_build_coefficients).
-std::atomic<int*> g_wait_error{nullptr};
+// What kernels tell the host of their grid-wide barriers: pinned, allocated
+// once per process outside any stream capture (gmes_build_coefficients) and
+// kept, as the pool of slots is (graphs may give theirs back at exit).
+struct BarrierHost {
+  int error;                    // a wait ran past its limit
+  uint32_t done[kStreamSlots];  // number of the last launch that left a slot
+};
+std::atomic<BarrierHost*> g_barriers{nullptr};
+SlotPool* g_slots = nullptr;  // set before g_barriers
 
-cudaError_t ensure_wait_error() {
+cudaError_t ensure_barriers() {
   static std::mutex m;
   std::lock_guard<std::mutex> lock(m);
-  if (g_wait_error.load() != nullptr) return cudaSuccess;
+  if (g_barriers.load() != nullptr) return cudaSuccess;
   void* p = nullptr;
   const cudaError_t e =
-      cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+      cudaHostAlloc(&p, sizeof(BarrierHost), cudaHostAllocPortable | cudaHostAllocMapped);
   if (e != cudaSuccess) return e;
-  *static_cast<int*>(p) = 0;
-  g_wait_error.store(static_cast<int*>(p));
+  std::memset(p, 0, sizeof(BarrierHost));
+  BarrierHost* b = static_cast<BarrierHost*>(p);
+  g_slots = new SlotPool(kStreamSlots, kGraphSlots, b->done);
+  g_barriers.store(b);
   return cudaSuccess;
 }
 
 // GMES_ERR_CUDA once a kernel has given up waiting.
 gmes_status check_wait_error() {
-  const int* w = g_wait_error.load();
+  const int* w = wait_error_word();
   if (w != nullptr && *static_cast<const volatile int*>(w) != 0)
     return fail(GMES_ERR_CUDA, "a step kernel gave up waiting for its other blocks: the fields "
                                "it was stepping are not valid");
@@ -147,7 +154,10 @@ gmes_status check_aux(const gmes_grid_desc* g) {
 
 }  // namespace
 
-int* wait_error_word() { return g_wait_error.load(); }
+int* wait_error_word() {
+  BarrierHost* b = g_barriers.load();
+  return b == nullptr ? nullptr : &b->error;
+}
 
 int sm_count() {
   int dev = 0, n = 0;
@@ -270,43 +280,41 @@ BatchView batch_view(const gmes_batch& b) {
   return v;
 }
 
-// Barrier words of the persistent kernel (gmes_persist.cu).  A direct launch
-// takes the next word of a ring far longer than the launches that can be in
-// flight; a graph captured here keeps a word until it is destroyed, and the
-// word then goes to the back of the queue, so that it is dealt again only
-// thousands of captures after its graph's last launch.  A capture begun by the
-// caller gets none: its graph's lifetime is not known here.
-std::mutex g_word_mutex;
-std::deque<int> g_free_words;                    // of destroyed graphs
-int g_next_word = kRingWords;                    // never used yet
-std::unordered_map<void*, int> g_graph_words;    // graph -> its word
-std::atomic<unsigned> g_ring_word{0};
-struct Capture {
-  int word = -1;
-};
-thread_local Capture* g_capture = nullptr;       // the capture this thread runs
+// Where a cooperative launch on this stream meets: at the stream's slot or, in a
+// capture, at one that the captured graph keeps (a user object gives it back
+// when the graph, its executables and their launches are gone).
+void give_graph_slot(void* slot) { g_slots->give_graph((int)(intptr_t)slot); }
 
-int take_word(cudaStream_t s) {
+Meeting meeting(cudaStream_t s) {
+  Meeting m;
+  BarrierHost* const b = g_barriers.load();
+  if (b == nullptr) return m;
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) return -1;
-  if (st == cudaStreamCaptureStatusNone) return (int)(g_ring_word++ % kRingWords);
-  if (g_capture == nullptr) return -1;
-  if (g_capture->word < 0) {
-    std::lock_guard<std::mutex> lock(g_word_mutex);
-    if (g_next_word < kRingWords + kGraphWords) {
-      g_capture->word = g_next_word++;
-    } else if (!g_free_words.empty()) {
-      g_capture->word = g_free_words.front();
-      g_free_words.pop_front();
-    }
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo(s, &st, nullptr, &graph, nullptr, nullptr, nullptr) != cudaSuccess)
+    return m;
+  if (st == cudaStreamCaptureStatusNone) {
+    unsigned long long id = 0;
+    if (cudaStreamGetId(s, &id) != cudaSuccess) return m;
+    m.slot = g_slots->enter(id, &m.number);
+    if (m.slot >= 0) m.done = b->done + m.slot;
+    return m;
   }
-  return g_capture->word;
-}
-
-void give_word(int word) {
-  if (word < 0) return;
-  std::lock_guard<std::mutex> lock(g_word_mutex);
-  g_free_words.push_back(word);
+  if (st != cudaStreamCaptureStatusActive) return m;
+  const int slot = g_slots->take_graph();
+  if (slot < 0) return m;
+  cudaUserObject_t keep = nullptr;
+  if (cudaUserObjectCreate(&keep, (void*)(intptr_t)slot, give_graph_slot, 1,
+                           cudaUserObjectNoDestructorSync) != cudaSuccess) {
+    g_slots->give_graph(slot);
+    return m;
+  }
+  if (cudaGraphRetainUserObject(graph, keep, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+    cudaUserObjectRelease(keep, 1);  // gives the slot back
+    return m;
+  }
+  m.slot = slot;
+  return m;
 }
 
 // Host copies of the descriptors of the last kHostBatches prepared batches,
@@ -376,7 +384,6 @@ Plan make_plan(const gmes_grid_desc& g, Plan* inc) {
   p.disp = (g.flags & GMES_FLAG_DISPERSIVE) != 0;
   p.im = p.cplx ? make_im_view(p.re, g) : p.re;
   p.precision = g.precision;
-  p.word = -1;
   p.incident = nullptr;
   if (g.ntfsf > 0 && g.incident != nullptr && inc != nullptr) {
     *inc = make_plan(*g.incident, nullptr);
@@ -488,7 +495,7 @@ gmes_status gmes_build_coefficients(const gmes_grid_desc* g, const gmes_class_de
   const CoefLayout L = coef_layout(*g);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   char* base = static_cast<char*>(g->coef);
-  cudaError_t e = ensure_wait_error();
+  cudaError_t e = ensure_barriers();
   if (e == cudaSuccess && ncls > 0)
     e = cudaMemcpyAsync(base + L.raw_classes, classes, ncls * sizeof(gmes_class_desc),
                         cudaMemcpyHostToDevice, s);
@@ -615,7 +622,7 @@ gmes_status gmes_step(const gmes_grid_desc* g, int32_t nsteps, void* stream) {
   Plan inc;
   Plan p = make_plan(*g, &inc);
   if (persist_takes(p, nsteps) || (p.incident != nullptr && persist_takes(inc, 1)))
-    p.word = inc.word = take_word(static_cast<cudaStream_t>(stream));
+    p.meet = inc.meet = meeting(static_cast<cudaStream_t>(stream));
   cudaError_t e = launch_step(*g, p, nsteps, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "launching step kernels");
   return GMES_OK;
@@ -770,32 +777,18 @@ static gmes_status capture(cudaStream_t s, void** exec_out,
   if (exec_out == nullptr) return fail(GMES_ERR_VALUE, "graph_exec is NULL");
   cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return cuda_fail(e, "beginning stream capture");
-  Capture cap;
-  g_capture = &cap;
   gmes_status st = body();
-  g_capture = nullptr;
   cudaGraph_t graph = nullptr;
   e = cudaStreamEndCapture(s, &graph);
   if (st != GMES_OK) {
     if (graph) cudaGraphDestroy(graph);
-    give_word(cap.word);
     return st;
   }
-  if (e != cudaSuccess) {
-    give_word(cap.word);
-    return cuda_fail(e, "ending stream capture");
-  }
+  if (e != cudaSuccess) return cuda_fail(e, "ending stream capture");
   cudaGraphExec_t exec = nullptr;
   e = cudaGraphInstantiate(&exec, graph, 0);
   cudaGraphDestroy(graph);
-  if (e != cudaSuccess) {
-    give_word(cap.word);
-    return cuda_fail(e, "instantiating graph");
-  }
-  if (cap.word >= 0) {
-    std::lock_guard<std::mutex> lock(g_word_mutex);
-    g_graph_words[exec] = cap.word;
-  }
+  if (e != cudaSuccess) return cuda_fail(e, "instantiating graph");
   *exec_out = exec;
   return GMES_OK;
 }
@@ -824,17 +817,7 @@ gmes_status gmes_graph_launch(void* graph_exec, void* stream) {
 
 gmes_status gmes_graph_destroy(void* graph_exec) {
   if (graph_exec == nullptr) return GMES_OK;
-  int word = -1;
-  {
-    std::lock_guard<std::mutex> lock(g_word_mutex);
-    const auto it = g_graph_words.find(graph_exec);
-    if (it != g_graph_words.end()) {
-      word = it->second;
-      g_graph_words.erase(it);
-    }
-  }
   cudaError_t e = cudaGraphExecDestroy(static_cast<cudaGraphExec_t>(graph_exec));
-  give_word(word);
   if (e != cudaSuccess) return cuda_fail(e, "destroying graph");
   return GMES_OK;
 }
@@ -1055,7 +1038,6 @@ TmzDev make_tmz_dev(const gmes_grid_desc& g, const gmes_tmz_batch& b) {
   for (int k = 0; k < 4; ++k) t.pcoef[k] = map + L.map_flags + k * L.map_coef;
   char* after = static_cast<char*>(b.design) + L.design_coef + L.map_flags + 4 * L.map_coef;
   if (g.precision == GMES_FP32) t.tiles = after;
-  t.word = -1;
   t.hist = b.hist;
   t.mon = b.monitor;
   t.grad = b.grad;
@@ -1169,10 +1151,11 @@ gmes_status gmes_tmz_forward(const gmes_grid_desc* g, const gmes_tmz_batch* b, i
     return fail(GMES_ERR_VALUE, "%d steps exceed the hist capacity %d", nsteps, b->hist_steps);
   st = check_wait_error();
   if (st != GMES_OK) return st;
-  TmzDev t = make_tmz_dev(*g, *b);
+  const TmzDev t = make_tmz_dev(*g, *b);
+  Meeting meet;
   if (tmz_chunked(g->precision, t, b->block_steps))
-    t.word = take_word(static_cast<cudaStream_t>(stream));
-  cudaError_t e = launch_tmz_forward(g->precision, make_grid_dev(*g), t,
+    meet = meeting(static_cast<cudaStream_t>(stream));
+  cudaError_t e = launch_tmz_forward(g->precision, make_grid_dev(*g), t, meet,
                                      step0, nsteps, flags, b->block_steps,
                                      static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "launching the forward kernels");
@@ -1203,10 +1186,11 @@ gmes_status gmes_tmz_adjoint(const gmes_grid_desc* g, const gmes_tmz_batch* b, i
     return fail(GMES_ERR_VALUE, "%d steps exceed the hist capacity %d", nsteps, b->hist_steps);
   st = check_wait_error();
   if (st != GMES_OK) return st;
-  TmzDev t = make_tmz_dev(*g, *b);
+  const TmzDev t = make_tmz_dev(*g, *b);
+  Meeting meet;
   if (tmz_chunked(g->precision, t, b->block_steps))
-    t.word = take_word(static_cast<cudaStream_t>(stream));
-  cudaError_t e = launch_tmz_adjoint(g->precision, make_grid_dev(*g), t,
+    meet = meeting(static_cast<cudaStream_t>(stream));
+  cudaError_t e = launch_tmz_adjoint(g->precision, make_grid_dev(*g), t, meet,
                                      step0, nsteps, b->block_steps,
                                      static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "launching the adjoint kernels");

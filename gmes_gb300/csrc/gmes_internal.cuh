@@ -234,6 +234,15 @@ void launch_after(bool early, void (*kernel)(K...), dim3 grid, dim3 threads, siz
   cudaLaunchKernelEx(&c, kernel, K(args)...);
 }
 
+// Where the blocks of a cooperative launch meet (gmes_barrier.cuh,
+// gmes_slots.h): slot -1 is none; done: where the launch's last block to leave
+// writes the launch's number, NULL for nowhere.
+struct Meeting {
+  int32_t slot = -1;
+  uint32_t number = 0;
+  uint32_t* done = nullptr;
+};
+
 // Host-side launch plan of one grid: its real-plane view, the imaginary-
 // plane view of a complex grid, and the TFSF incident-field grid's plan.
 struct Plan {
@@ -241,7 +250,7 @@ struct Plan {
   bool cplx, disp;
   const Plan* incident;
   int precision;
-  int word;  // barrier word of the persistent kernel, -1: none to be had
+  Meeting meet;  // of the persistent kernel
 };
 
 // ---------------------------------------------------------------------------
@@ -442,7 +451,6 @@ struct TmzDev {
   const uint32_t* pflags;
   const void* pcoef[4];
   void* tiles;              // TbTile of every tile of the blocked kernels, or null
-  int32_t word;             // barrier word of the persistent kernels, -1: none to be had
   void* l[3];
   void* phi[2][4];          // ping-pong buffers of the psi adjoints
   const DesignCoef* dc;     // [nb][nd]
@@ -494,11 +502,13 @@ static_assert(GMES_MAX_PML <= 4, "2-bit profile-set fields");
 
 cudaError_t launch_tmz_design(int precision, const GridDev& g, const TmzDev& t,
                               const double* eps, cudaStream_t s);
-cudaError_t launch_tmz_forward(int precision, const GridDev& g, const TmzDev& t, int step0,
-                               int nsteps, int flags, int block_steps, cudaStream_t s);
-cudaError_t launch_tmz_adjoint(int precision, const GridDev& g, const TmzDev& t, int step0,
-                               int nsteps, int block_steps, cudaStream_t s);
-// Whether a call's steps run as one cooperative launch (given a barrier word).
+cudaError_t launch_tmz_forward(int precision, const GridDev& g, const TmzDev& t,
+                               const Meeting& meet, int step0, int nsteps, int flags,
+                               int block_steps, cudaStream_t s);
+cudaError_t launch_tmz_adjoint(int precision, const GridDev& g, const TmzDev& t,
+                               const Meeting& meet, int step0, int nsteps, int block_steps,
+                               cudaStream_t s);
+// Whether a call's steps run as one cooperative launch (given a barrier slot).
 bool tmz_chunked(int precision, const TmzDev& t, int block_steps);
 // Launches of one forward or adjoint call.
 int64_t tmz_launches(int precision, const TmzDev& t, int block_steps, int nsteps, bool adj);
@@ -516,12 +526,12 @@ int* wait_error_word();
 int sm_count();
 
 // Whole chunks of steps of a small grid in one launch (gmes_persist.cu).
-// Its grid-wide barrier counts in a word of its own per launch in flight:
-// kRingWords are dealt in turn to direct launches, the others belong to
-// captured graphs.
-constexpr int kRingWords = 1024, kGraphWords = 4096;
+// Barrier slots of direct launches (one per stream with launches in flight) and
+// of captured ones.
+constexpr int kStreamSlots = 1024, kGraphSlots = 4096;
 bool persist_takes(const Plan& p, int nsteps);
-cudaError_t launch_persist(const Plan& p, int nsteps, int st0, cudaStream_t s);
+cudaError_t launch_persist(const Plan& p, const Meeting& meet, int nsteps, int st0,
+                           cudaStream_t s);
 
 // Launchers implemented per precision in gmes_step.cu.
 cudaError_t launch_step(const gmes_grid_desc& g, const Plan& p, int nsteps, cudaStream_t s);

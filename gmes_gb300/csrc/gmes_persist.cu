@@ -64,7 +64,8 @@ struct PersistCfg {
   int cells;
   uint32_t m_row, m_plane; // quotients of a cell index (tile_quot)
   int s_row, s_plane;
-  int nsteps, st0, word;
+  int nsteps, st0;
+  Meeting meet;
   TabLayout tab;
 };
 
@@ -233,7 +234,6 @@ template <class P, bool DISP, int MASK, bool CX>
 __global__ void __launch_bounds__(kPersistThreads, GMES_PERSIST_BLOCKS)
     k_persist(const __grid_constant__ GridDev g, const __grid_constant__ GridDev gi,
               const __grid_constant__ PersistCfg c, int* error) {
-  unsigned* const word = barrier_words + 8 * c.word;
   __shared__ OwnSource own[kPersistSources];
   __shared__ int nown;
   extern __shared__ __align__(16) unsigned char tab[];
@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(kPersistThreads, GMES_PERSIST_BLOCKS)
     cell_of(t, i, j, k);
     ghost_cell<P, 1, MASK, CX>(g, gi, i, j, k, c.nsteps == 1);
   }
-  if (!grid_barrier(word, error)) return;
+  if (!grid_barrier(c.meet, error)) return;
   for (int st = 0; st < c.nsteps; ++st) {
     const bool last = st + 1 == c.nsteps;
     auto half = [&](auto tag) {
@@ -367,9 +367,10 @@ __global__ void __launch_bounds__(kPersistThreads, GMES_PERSIST_BLOCKS)
       }
     };
     half(std::integral_constant<int, 0>{});
-    if (!grid_barrier(word, error)) return;
+    if (!grid_barrier(c.meet, error)) return;
+    if (last) leave_barrier(c.meet);
     half(std::integral_constant<int, 1>{});
-    if (!last && !grid_barrier(word, error)) return;
+    if (!last && !grid_barrier(c.meet, error)) return;
   }
 }
 
@@ -400,7 +401,7 @@ TabLayout table_layout(const GridDev& d, int per, int es) {
 }
 
 template <class P, bool DISP, int MASK, bool CX>
-cudaError_t launch_one(const Plan& p, int nsteps, int st0, cudaStream_t s) {
+cudaError_t launch_one(const Plan& p, const Meeting& meet, int nsteps, int st0, cudaStream_t s) {
   const GridDev& d = p.re;
   auto* kernel = k_persist<P, DISP, MASK, CX>;
   int per_sm = 0;
@@ -422,7 +423,7 @@ cudaError_t launch_one(const Plan& p, int nsteps, int st0, cudaStream_t s) {
   tile_div_of((uint32_t)d.n[2], c.m_row, c.s_row);
   tile_div_of((uint32_t)(d.n[1] * d.n[2]), c.m_plane, c.s_plane);
   c.nsteps = nsteps;
-  c.word = p.word;
+  c.meet = meet;
   c.st0 = st0;
   c.tab = table_layout(d, per, (int)sizeof(typename P::T));
   GridDev re = p.re, im = p.im;
@@ -433,25 +434,25 @@ cudaError_t launch_one(const Plan& p, int nsteps, int st0, cudaStream_t s) {
 }
 
 template <class P, bool DISP, bool CX>
-cudaError_t launch_mask(const Plan& p, int nsteps, int st0, cudaStream_t s) {
+cudaError_t launch_mask(const Plan& p, const Meeting& meet, int nsteps, int st0, cudaStream_t s) {
   constexpr int kTMz = 1 << GMES_EZ | 1 << GMES_HX | 1 << GMES_HY;
   constexpr int kTEz = 1 << GMES_EX | 1 << GMES_EY | 1 << GMES_HZ;
   switch (p.re.active) {
     case kTMz:
-      return launch_one<P, DISP, kTMz, CX>(p, nsteps, st0, s);
+      return launch_one<P, DISP, kTMz, CX>(p, meet, nsteps, st0, s);
     case kTEz:
-      return launch_one<P, DISP, kTEz, CX>(p, nsteps, st0, s);
+      return launch_one<P, DISP, kTEz, CX>(p, meet, nsteps, st0, s);
     case 63:
-      return launch_one<P, DISP, 63, CX>(p, nsteps, st0, s);
+      return launch_one<P, DISP, 63, CX>(p, meet, nsteps, st0, s);
     default:
-      return launch_one<P, DISP, 0, CX>(p, nsteps, st0, s);
+      return launch_one<P, DISP, 0, CX>(p, meet, nsteps, st0, s);
   }
 }
 
 template <class P, bool CX = false>
-cudaError_t launch_disp(const Plan& p, int nsteps, int st0, cudaStream_t s) {
-  return p.disp ? launch_mask<P, true, CX>(p, nsteps, st0, s)
-                : launch_mask<P, false, CX>(p, nsteps, st0, s);
+cudaError_t launch_disp(const Plan& p, const Meeting& meet, int nsteps, int st0, cudaStream_t s) {
+  return p.disp ? launch_mask<P, true, CX>(p, meet, nsteps, st0, s)
+                : launch_mask<P, false, CX>(p, meet, nsteps, st0, s);
 }
 
 }  // namespace
@@ -491,15 +492,15 @@ bool persist_takes(const Plan& p, int nsteps) {
   return (int64_t)d.n[0] * d.n[1] * d.n[2] <= most;
 }
 
-cudaError_t launch_persist(const Plan& p, int nsteps, int st0, cudaStream_t s) {
-  if (p.cplx) return launch_disp<PolF64, true>(p, nsteps, st0, s);
+cudaError_t launch_persist(const Plan& p, const Meeting& meet, int nsteps, int st0, cudaStream_t s) {
+  if (p.cplx) return launch_disp<PolF64, true>(p, meet, nsteps, st0, s);
   switch (p.precision) {
     case GMES_FP64:
-      return launch_disp<PolF64>(p, nsteps, st0, s);
+      return launch_disp<PolF64>(p, meet, nsteps, st0, s);
     case GMES_FP32:
-      return launch_disp<PolF32>(p, nsteps, st0, s);
+      return launch_disp<PolF32>(p, meet, nsteps, st0, s);
     case GMES_DF64:
-      return launch_disp<PolDF>(p, nsteps, st0, s);
+      return launch_disp<PolDF>(p, meet, nsteps, st0, s);
     default:
       return cudaErrorInvalidValue;
   }

@@ -583,7 +583,7 @@ cudaError_t run_steps(const Plan& p, int nsteps, int side_mask, int st0, cudaStr
 // A complex grid runs every per-plane kernel on its real and imaginary
 // planes; only the ghost copy couples them.
 template <class P, bool STRICT>
-void run_half(const Plan& p, int side, int st, bool early, cudaStream_t s) {
+void run_half(const Plan& p, int side, int st, bool early, bool last, cudaStream_t s) {
   using T = typename P::T;
   const GridDev& d = p.re;
   int64_t maxplane = 1;
@@ -631,8 +631,10 @@ void run_half(const Plan& p, int side, int st, bool early, cudaStream_t s) {
       launch_after(true, k_probes<P>, dim3((v.nprobe + 127) / 128), 128, 0, s, v, side, (int64_t)st);
   }
   if (side == 0 && p.incident != nullptr) {
-    if (p.incident->word >= 0 && persist_takes(*p.incident, 1))
-      launch_persist(*p.incident, 1, st, s);
+    Meeting meet = p.incident->meet;
+    if (!last) meet.done = nullptr;  // the call's last launch answers for all
+    if (meet.slot >= 0 && persist_takes(*p.incident, 1))
+      launch_persist(*p.incident, meet, 1, st, s);
     else
       run_steps<P, STRICT>(*p.incident, 1, 3, st, s);
   }
@@ -641,8 +643,11 @@ void run_half(const Plan& p, int side, int st, bool early, cudaStream_t s) {
 template <class P, bool STRICT>
 cudaError_t run_steps(const Plan& p, int nsteps, int side_mask, int st0, cudaStream_t s) {
   for (int st = 0; st < nsteps; ++st) {
-    if (side_mask & 1) run_half<P, STRICT>(p, 0, st0 + st, st > 0, s);
-    if (side_mask & 2) run_half<P, STRICT>(p, 1, st0 + st, (st > 0 || (side_mask & 1)) && p.incident == nullptr, s);
+    const bool last = st + 1 == nsteps;
+    if (side_mask & 1) run_half<P, STRICT>(p, 0, st0 + st, st > 0, last, s);
+    if (side_mask & 2)
+      run_half<P, STRICT>(p, 1, st0 + st, (st > 0 || (side_mask & 1)) && p.incident == nullptr,
+                          last, s);
   }
   return cudaGetLastError();
 }
@@ -770,7 +775,8 @@ cudaError_t launch_nonfinite(const gmes_grid_desc& g, const GridDev& d, int32_t*
 }
 
 cudaError_t launch_step(const gmes_grid_desc& g, const Plan& p, int nsteps, cudaStream_t s) {
-  if (p.word >= 0 && persist_takes(p, nsteps)) return launch_persist(p, nsteps, 0, s);
+  if (p.meet.slot >= 0 && persist_takes(p, nsteps))
+    return launch_persist(p, p.meet, nsteps, 0, s);
   return dispatch_precision(g, p, nsteps, 3, 0, s);
 }
 

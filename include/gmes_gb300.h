@@ -309,7 +309,9 @@ gmes_status gmes_step(const gmes_grid_desc* g, int32_t nsteps, void* stream);
 
 /*
  * The kernels that gmes_step(g, nsteps) launches, in *launches: a small grid's
- * steps run as one launch, the others' as a few per half-step.
+ * steps run as one launch, the others' as a few per half-step.  (A one-launch
+ * grid takes the launches per half-step while 1024 streams have such launches in
+ * flight or 4096 captured ones exist.)
  */
 gmes_status gmes_step_launches(const gmes_grid_desc* g, int32_t nsteps, int64_t* launches);
 
