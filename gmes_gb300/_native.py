@@ -36,6 +36,7 @@ EXPORTS = [
     "gmes_tmz_sizes", "gmes_tmz_check", "gmes_tmz_set_design", "gmes_tmz_reset",
     "gmes_tmz_forward", "gmes_tmz_objective", "gmes_tmz_adjoint", "gmes_points_update",
     "gmes_copy_async", "gmes_nonfinite", "gmes_step_launches", "gmes_tmz_launches",
+    "gmes_wait_status", "gmes_wait_check",
 ]
 NOALLOC_MAX_GRIDS = 64
 
@@ -164,6 +165,9 @@ def load():
     lib.gmes_reset.argtypes = [P(GridDescC), C.c_void_p]
     lib.gmes_step.argtypes = [P(GridDescC), C.c_int32, C.c_void_p]
     lib.gmes_step_launches.argtypes = [P(GridDescC), C.c_int32, P(C.c_int64)]
+    lib.gmes_wait_status.argtypes = [C.c_int32]
+    lib.gmes_wait_check.argtypes = [C.c_int32, C.c_int32, C.c_int32, C.c_void_p, C.c_int64,
+                                    C.c_void_p]
     lib.gmes_half_step.argtypes = [P(GridDescC), C.c_int32, C.c_int32, C.c_void_p]
     lib.gmes_read_field.argtypes = [P(GridDescC), C.c_int32, P(C.c_double), C.c_void_p]
     lib.gmes_write_field.argtypes = [P(GridDescC), C.c_int32, P(C.c_double), C.c_void_p]
@@ -212,3 +216,15 @@ def check(status):
         return
     msg = load().gmes_last_error().decode(errors="replace")
     raise _STATUS_EXC.get(status, RuntimeError)(msg)
+
+
+def check_waits():
+    """Raise when a one-launch step of the current device gave up waiting (ask
+    after a synchronisation)."""
+    check(load().gmes_wait_status(0))
+
+
+def clear_waits():
+    """Wait for the current device and make its one-launch steps usable after
+    such an error."""
+    check(load().gmes_wait_status(1))

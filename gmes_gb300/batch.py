@@ -236,6 +236,7 @@ class Batch:
 
     def synchronize(self):
         self.stream.synchronize()
+        N.check_waits()
         torch = _torch()
         for e in self.engines:
             e.torch_stream.wait_stream(self.stream)

@@ -685,17 +685,26 @@ __global__ void __launch_bounds__(kChunkThreads, 2)
     k_tmz_chunk_fwd(const __grid_constant__ GridDev g, const __grid_constant__ TmzDev t,
                     const LatDiv d, const __grid_constant__ Meeting meet, int step0, int nsteps, int flags, 
                     int* error) {
+  auto met = [&] {
+    if (grid_barrier(meet, error)) return true;
+    const int64_t es = sizeof(typename P::T), nd = (int64_t)t.dn[0] * t.dn[1];
+    for (int q = 0; q < 3; ++q) spoil(t.f[q], t.nb * t.plane * es);
+    if (flags & GMES_TMZ_RECORD_HIST) spoil(t.hist, (int64_t)t.hist_steps * t.nb * nd * es);
+    if (flags & GMES_TMZ_RECORD_MONITOR)
+      spoil(t.mon, (int64_t)t.nb * t.total_steps * t.mn[0] * t.mn[1] * 8);
+    return false;
+  };
   for (int k = 0; k < nsteps; ++k) {
     const int n = step0 + k + 1;
     for_points(t, d, [&](const Lat& p) {
       point_fe<P>(g, t, p, n, (flags & GMES_TMZ_RECORD_HIST) ? k : -1);
     });
-    if (!grid_barrier(meet, error)) return;
+    if (!met()) return;
     if (k + 1 == nsteps) leave_barrier(meet);
     for_points(t, d, [&](const Lat& p) {
       point_fh<P>(g, t, p, n, (flags & GMES_TMZ_RECORD_MONITOR) ? n - 1 : -1);
     });
-    if (k + 1 < nsteps && !grid_barrier(meet, error)) return;
+    if (k + 1 < nsteps && !met()) return;
   }
 }
 
@@ -704,13 +713,18 @@ template <class P>
 __global__ void __launch_bounds__(kChunkThreads, 2)
     k_tmz_chunk_adj(const __grid_constant__ GridDev g, const __grid_constant__ TmzDev t,
                     const LatDiv d, const __grid_constant__ Meeting meet, int step0, int nsteps, int* error) {
+  auto met = [&] {
+    if (grid_barrier(meet, error)) return true;
+    spoil(t.grad, (int64_t)t.nb * t.dn[0] * t.dn[1] * 8);
+    return false;
+  };
   for (int k = nsteps - 1; k >= 0; --k) {
     const int n = step0 + k + 1, rb = n & 1, wb = rb ^ 1;
     for_points(t, d, [&](const Lat& p) { point_ah<P>(g, t, p, n, rb, wb); });
-    if (!grid_barrier(meet, error)) return;
+    if (!met()) return;
     if (k == 0) leave_barrier(meet);
     for_points(t, d, [&](const Lat& p) { point_ae<P>(g, t, p, k, rb, wb); });
-    if (k > 0 && !grid_barrier(meet, error)) return;
+    if (k > 0 && !met()) return;
   }
 }
 
@@ -2220,7 +2234,7 @@ cudaError_t forward(const GridDev& g, const TmzDev& t, const Meeting& meet, int 
                     int flags, cudaStream_t s) {
   if (nsteps <= 0) return cudaSuccess;
   map_sources(t, s);
-  if (meet.slot >= 0) {
+  if (meet.at != nullptr) {
     LatDiv d;
     int blocks = 0;
     const cudaError_t e = chunk_shape(k_tmz_chunk_fwd<P>, t, d, blocks);
@@ -2249,7 +2263,7 @@ cudaError_t adjoint(const GridDev& g, const TmzDev& t, const Meeting& meet, int 
                     cudaStream_t s) {
   if (nsteps <= 0) return cudaSuccess;
   map_sources(t, s);
-  if (meet.slot >= 0) {
+  if (meet.at != nullptr) {
     LatDiv d;
     int blocks = 0;
     const cudaError_t e = chunk_shape(k_tmz_chunk_adj<P>, t, d, blocks);

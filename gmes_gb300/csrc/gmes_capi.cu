@@ -50,20 +50,30 @@ int elem_size(int32_t precision) {
 // What kernels tell the host of their grid-wide barriers: pinned, allocated
 // once per process outside any stream capture (gmes_build_coefficients) and
 // kept, as the pool of slots is (graphs may give theirs back at exit).
+constexpr int kMaxDevices = 64;
 struct BarrierHost {
-  int error;                    // a wait ran past its limit
+  int error[kMaxDevices];       // a wait ran past its limit, per device
   uint32_t done[kStreamSlots];  // number of the last launch that left a slot
 };
 std::atomic<BarrierHost*> g_barriers{nullptr};
 SlotPool* g_slots = nullptr;  // set before g_barriers
+std::atomic<Slot*> g_slots_at[kMaxDevices];  // per device
 
 cudaError_t ensure_barriers() {
   static std::mutex m;
   std::lock_guard<std::mutex> lock(m);
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < kMaxDevices && g_slots_at[dev].load() == nullptr) {
+    Slot* at = nullptr;
+    e = slots_address(&at);
+    if (e != cudaSuccess) return e;
+    g_slots_at[dev].store(at);
+  }
   if (g_barriers.load() != nullptr) return cudaSuccess;
   void* p = nullptr;
-  const cudaError_t e =
-      cudaHostAlloc(&p, sizeof(BarrierHost), cudaHostAllocPortable | cudaHostAllocMapped);
+  e = cudaHostAlloc(&p, sizeof(BarrierHost), cudaHostAllocPortable | cudaHostAllocMapped);
   if (e != cudaSuccess) return e;
   std::memset(p, 0, sizeof(BarrierHost));
   BarrierHost* b = static_cast<BarrierHost*>(p);
@@ -72,12 +82,12 @@ cudaError_t ensure_barriers() {
   return cudaSuccess;
 }
 
-// GMES_ERR_CUDA once a kernel has given up waiting.
+// GMES_ERR_CUDA once a kernel of this device has given up waiting.
 gmes_status check_wait_error() {
   const int* w = wait_error_word();
   if (w != nullptr && *static_cast<const volatile int*>(w) != 0)
     return fail(GMES_ERR_CUDA, "a step kernel gave up waiting for its other blocks: the fields "
-                               "it was stepping are not valid");
+                               "it was stepping are not valid (gmes_wait_status)");
   return GMES_OK;
 }
 
@@ -156,7 +166,11 @@ gmes_status check_aux(const gmes_grid_desc* g) {
 
 int* wait_error_word() {
   BarrierHost* b = g_barriers.load();
-  return b == nullptr ? nullptr : &b->error;
+  int dev = 0;
+  if (b == nullptr || cudaGetDevice(&dev) != cudaSuccess || dev >= kMaxDevices ||
+      g_slots_at[dev].load() == nullptr)
+    return nullptr;
+  return b->error + dev;
 }
 
 int sm_count() {
@@ -287,8 +301,9 @@ void give_graph_slot(void* slot) { g_slots->give_graph((int)(intptr_t)slot); }
 
 Meeting meeting(cudaStream_t s) {
   Meeting m;
-  BarrierHost* const b = g_barriers.load();
-  if (b == nullptr) return m;
+  int dev = 0;
+  if (wait_error_word() == nullptr || cudaGetDevice(&dev) != cudaSuccess) return m;
+  Slot* const slots = g_slots_at[dev].load();
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   cudaGraph_t graph = nullptr;
   if (cudaStreamGetCaptureInfo(s, &st, nullptr, &graph, nullptr, nullptr, nullptr) != cudaSuccess)
@@ -296,8 +311,10 @@ Meeting meeting(cudaStream_t s) {
   if (st == cudaStreamCaptureStatusNone) {
     unsigned long long id = 0;
     if (cudaStreamGetId(s, &id) != cudaSuccess) return m;
-    m.slot = g_slots->enter(id, &m.number);
-    if (m.slot >= 0) m.done = b->done + m.slot;
+    const int slot = g_slots->enter(id, &m.number);
+    if (slot < 0) return m;
+    m.at = slots + slot;
+    m.done = g_barriers.load()->done + slot;
     return m;
   }
   if (st != cudaStreamCaptureStatusActive) return m;
@@ -313,7 +330,7 @@ Meeting meeting(cudaStream_t s) {
     cudaUserObjectRelease(keep, 1);  // gives the slot back
     return m;
   }
-  m.slot = slot;
+  m.at = slots + slot;
   return m;
 }
 
@@ -647,6 +664,39 @@ gmes_status gmes_step_launches(const gmes_grid_desc* g, int32_t nsteps, int64_t*
     *launches = (int64_t)nsteps * (2 * per_half(p) + (p.incident == nullptr ? 0
                                                       : persist_takes(inc, 1) ? 1
                                                                             : 2 * per_half(inc)));
+  return GMES_OK;
+}
+
+gmes_status gmes_wait_status(int32_t reset) {
+  if (reset == 0) return check_wait_error();
+  int* const error = wait_error_word();
+  if (error == nullptr) return GMES_OK;
+  cudaError_t e = cudaDeviceSynchronize();
+  if (e == cudaSuccess) e = clear_slots();
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  if (e != cudaSuccess) return cuda_fail(e, "making the barriers usable again");
+  *static_cast<volatile int*>(error) = 0;
+  return GMES_OK;
+}
+
+gmes_status gmes_wait_check(int32_t blocks, int32_t absent, int32_t polls, void* out,
+                            int64_t bytes, void* stream) {
+  if (blocks < 1 || blocks > sm_count() || absent < -1 || absent >= blocks)
+    return fail(GMES_ERR_VALUE, "blocks = %d outside [1, %d] or absent = %d outside [-1, %d)",
+                blocks, sm_count(), absent, blocks);
+  if (polls < 1 || polls > Meeting().polls)
+    return fail(GMES_ERR_VALUE, "polls = %d outside [1, %d]", polls, Meeting().polls);
+  if (bytes < 0 || (bytes > 0 && out == nullptr))
+    return fail(GMES_ERR_VALUE, "%lld bytes at %p", (long long)bytes, out);
+  gmes_status st = check_wait_error();
+  if (st != GMES_OK) return st;
+  cudaError_t e = ensure_barriers();
+  if (e != cudaSuccess) return cuda_fail(e, "allocating the barriers' host words");
+  Meeting m = meeting(static_cast<cudaStream_t>(stream));
+  if (m.at == nullptr) return fail(GMES_ERR_RUNTIME, "no barrier slot to be had");
+  m.polls = polls;
+  e = launch_wait_check(m, blocks, absent, out, bytes, static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return cuda_fail(e, "launching the barrier check");
   return GMES_OK;
 }
 
@@ -1274,7 +1324,6 @@ __global__ void k_noalloc_fill(char* dst, const __grid_constant__ TableChunk c) 
     out[w] = c.data[w];
 }
 
-constexpr int kMaxDevices = 64;
 std::mutex g_noalloc_mutex;
 void* g_noalloc_addr[kMaxDevices] = {};          // per device, looked up on first use
 alignas(256) char g_noalloc_image[kNoAllocBytes];  // host image, guarded by the mutex

@@ -234,11 +234,20 @@ void launch_after(bool early, void (*kernel)(K...), dim3 grid, dim3 threads, siz
   cudaLaunchKernelEx(&c, kernel, K(args)...);
 }
 
+// A barrier slot: the blocks' arrivals (zero low bits after every barrier),
+// whether a block has given up here, and the blocks that have left the launch's
+// last barrier.
+struct alignas(32) Slot {
+  unsigned word, failed, left;
+};
+
 // Where the blocks of a cooperative launch meet (gmes_barrier.cuh,
-// gmes_slots.h): slot -1 is none; done: where the launch's last block to leave
-// writes the launch's number, NULL for nowhere.
+// gmes_slots.h), NULL: nowhere to be had; done: where the launch's last block to
+// leave writes the launch's number, NULL for nowhere; polls: of one barrier
+// before a block gives up (some seconds).
 struct Meeting {
-  int32_t slot = -1;
+  Slot* at = nullptr;
+  int32_t polls = 1 << 22;
   uint32_t number = 0;
   uint32_t* done = nullptr;
 };
@@ -520,8 +529,8 @@ cudaError_t launch_points(const gmes_points& g, void* inplace, const void* in1, 
 
 // Host-side helpers implemented in gmes_capi.cu.
 GridDev make_grid_dev(const gmes_grid_desc& g);
-// Pinned word that a kernel sets when a wait ran past its limit (NULL until
-// the first gmes_build_coefficients), and the SMs of the current device.
+// Pinned word of the current device that a kernel sets when a wait ran past its
+// limit (NULL until the first gmes_build_coefficients), and the device's SMs.
 int* wait_error_word();
 int sm_count();
 
@@ -530,6 +539,14 @@ int sm_count();
 // of captured ones.
 constexpr int kStreamSlots = 1024, kGraphSlots = 4096;
 bool persist_takes(const Plan& p, int nsteps);
+// The current device's slots, and every one of them made fit for use again (the
+// device is idle).
+cudaError_t slots_address(Slot** at);
+cudaError_t clear_slots();
+// One barrier of `blocks` blocks of which `absent` (-1: none) stays away; the
+// results (bytes at out) are spoiled where a block gave up.
+cudaError_t launch_wait_check(const Meeting& meet, int blocks, int absent, void* out,
+                              int64_t bytes, cudaStream_t s);
 cudaError_t launch_persist(const Plan& p, const Meeting& meet, int nsteps, int st0,
                            cudaStream_t s);
 

@@ -244,6 +244,13 @@ __global__ void __launch_bounds__(kPersistThreads, GMES_PERSIST_BLOCKS)
   // barrier waits for the slowest SM.  Group v of the block is group
   // blockIdx.x + v gridDim.x of the grid; warp w takes v = w, w + 16, ...
   constexpr int kWarps = kPersistThreads / 32;
+  auto meet = [&] {
+    if (grid_barrier(c.meet, error)) return true;
+    for (int comp = 0; comp < 6; ++comp)
+      if ((g.active >> comp) & 1)
+        spoil(g.f[comp], g.npts[comp] * (CX ? 2 : 1) * (int64_t)sizeof(typename P::T));
+    return false;
+  };
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int groups = (c.cells + 31) / 32;
   const int mine = (groups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
@@ -322,7 +329,7 @@ __global__ void __launch_bounds__(kPersistThreads, GMES_PERSIST_BLOCKS)
     cell_of(t, i, j, k);
     ghost_cell<P, 1, MASK, CX>(g, gi, i, j, k, c.nsteps == 1);
   }
-  if (!grid_barrier(c.meet, error)) return;
+  if (!meet()) return;
   for (int st = 0; st < c.nsteps; ++st) {
     const bool last = st + 1 == c.nsteps;
     auto half = [&](auto tag) {
@@ -367,10 +374,10 @@ __global__ void __launch_bounds__(kPersistThreads, GMES_PERSIST_BLOCKS)
       }
     };
     half(std::integral_constant<int, 0>{});
-    if (!grid_barrier(c.meet, error)) return;
+    if (!meet()) return;
     if (last) leave_barrier(c.meet);
     half(std::integral_constant<int, 1>{});
-    if (!last && !grid_barrier(c.meet, error)) return;
+    if (!last && !meet()) return;
   }
 }
 
@@ -490,6 +497,40 @@ bool persist_takes(const Plan& p, int nsteps) {
   const int64_t most =
       nsteps == 1 ? kPersistCellsOneStep : (p.cplx ? kPersistCellsComplex : kPersistCells);
   return (int64_t)d.n[0] * d.n[1] * d.n[2] <= most;
+}
+
+__device__ Slot barrier_slots[kStreamSlots + kGraphSlots];
+
+cudaError_t slots_address(Slot** at) {
+  return cudaGetSymbolAddress(reinterpret_cast<void**>(at), barrier_slots);
+}
+
+__global__ void k_clear_slots() {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < kStreamSlots + kGraphSlots) barrier_slots[k] = Slot{0, 0, 0};
+}
+
+cudaError_t clear_slots() {
+  k_clear_slots<<<(kStreamSlots + kGraphSlots + 255) / 256, 256>>>();
+  return cudaGetLastError();
+}
+
+__global__ void k_wait_check(const Meeting m, int absent, void* out, int64_t bytes, int* error) {
+  if ((int)blockIdx.x == absent) return;
+  if (!grid_barrier(m, error)) {
+    spoil(out, bytes);
+    return;
+  }
+  leave_barrier(m);
+}
+
+cudaError_t launch_wait_check(const Meeting& meet, int blocks, int absent, void* out,
+                              int64_t bytes, cudaStream_t s) {
+  Meeting m = meet;
+  int* error = wait_error_word();
+  void* args[] = {&m, &absent, &out, &bytes, &error};
+  return cudaLaunchCooperativeKernel((const void*)k_wait_check, dim3((unsigned)blocks), dim3(32),
+                                     args, 0, s);
 }
 
 cudaError_t launch_persist(const Plan& p, const Meeting& meet, int nsteps, int st0, cudaStream_t s) {

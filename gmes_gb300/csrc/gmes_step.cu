@@ -633,7 +633,7 @@ void run_half(const Plan& p, int side, int st, bool early, bool last, cudaStream
   if (side == 0 && p.incident != nullptr) {
     Meeting meet = p.incident->meet;
     if (!last) meet.done = nullptr;  // the call's last launch answers for all
-    if (meet.slot >= 0 && persist_takes(*p.incident, 1))
+    if (meet.at != nullptr && persist_takes(*p.incident, 1))
       launch_persist(*p.incident, meet, 1, st, s);
     else
       run_steps<P, STRICT>(*p.incident, 1, 3, st, s);
@@ -775,7 +775,7 @@ cudaError_t launch_nonfinite(const gmes_grid_desc& g, const GridDev& d, int32_t*
 }
 
 cudaError_t launch_step(const gmes_grid_desc& g, const Plan& p, int nsteps, cudaStream_t s) {
-  if (p.meet.slot >= 0 && persist_takes(p, nsteps))
+  if (p.meet.at != nullptr && persist_takes(p, nsteps))
     return launch_persist(p, p.meet, nsteps, 0, s);
   return dispatch_precision(g, p, nsteps, 3, 0, s);
 }

@@ -314,7 +314,7 @@ class GridEngine:
 
     def probe_values(self, k):
         """(k, nprobe) float64 numpy: the probes of the last k recorded steps of a chunk."""
-        self._stream.synchronize()
+        self.synchronize()
         if self.cmplx:
             v = self.probe_val[:, :k].cpu().numpy()
             return v[0] + 1j * v[1]
@@ -424,13 +424,20 @@ class GridEngine:
         t = self.fields[c]
         if self.cmplx:
             a = t.cpu().numpy()
-            return a[0] + 1j * a[1]
-        if self.prec == N.DF64:
-            return (t[..., 0].double() + t[..., 1].double()).cpu().numpy()
-        return t.double().cpu().numpy()
+            a = a[0] + 1j * a[1]
+        elif self.prec == N.DF64:
+            a = (t[..., 0].double() + t[..., 1].double()).cpu().numpy()
+        else:
+            a = t.double().cpu().numpy()
+        N.check_waits()
+        return a
 
     def read_tensor(self, c):
-        """Component ``c`` as a float64 (complex128) device tensor."""
+        """Component ``c`` as a float64 (complex128) device tensor.
+
+        Not synchronised: a step that gave up waiting shows as NaN here, and
+        as an error at the next call that waits or steps.
+        """
         t = self.fields[c]
         if self.cmplx:
             return _torch().complex(t[0], t[1])
@@ -497,3 +504,4 @@ class GridEngine:
 
     def synchronize(self):
         self._stream.synchronize()
+        N.check_waits()

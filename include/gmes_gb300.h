@@ -316,6 +316,26 @@ gmes_status gmes_step(const gmes_grid_desc* g, int32_t nsteps, void* stream);
 gmes_status gmes_step_launches(const gmes_grid_desc* g, int32_t nsteps, int64_t* launches);
 
 /*
+ * One-launch steps and differentiation calls meet at grid-wide barriers.  A
+ * block that waits there for some seconds gives up: the launch ends, its results
+ * (the fields; the state, history and monitor; the gradient) read as NaN, and
+ * every call that steps on the device fails with GMES_ERR_CUDA.
+ * gmes_wait_status(0) says whether that has happened on the current device (ask
+ * after a synchronisation); gmes_wait_status(1) waits for the device, makes the
+ * barriers usable and clears the error.
+ */
+gmes_status gmes_wait_status(int32_t reset);
+
+/*
+ * One such barrier of `blocks` blocks (at most the device's SMs), of which block
+ * `absent` stays away (-1: none) and which the others leave after `polls` polls
+ * at most, spoiling `bytes` bytes of device memory at `out`: what a caller's
+ * handling of the error can be tried with.
+ */
+gmes_status gmes_wait_check(int32_t blocks, int32_t absent, int32_t polls, void* out,
+                            int64_t bytes, void* stream);
+
+/*
  * One half of step `step` (0-based index into src_val, < src_steps when
  * there are sources): side 0 = H ghost copy, E update, E sources; side 1 =
  * E ghost copy, H update, H sources.  gmes_step(g, n) is n pairs of these.
