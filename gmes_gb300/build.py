@@ -21,6 +21,8 @@ LIB = PKG / "libgmes_gb300.so"
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
+          # a launch's dropped status (a [[nodiscard]] result) does not build
+          "-Xcompiler", "-Werror=unused-result",
           f"-I{ROOT / 'include'}"]
 # Per-file flags: the coefficient builder and the rasteriser reproduce the
 # reference's FP64 operation order, so multiply-add contraction is disabled;

@@ -2237,15 +2237,17 @@ cudaError_t forward(const GridDev& g, const TmzDev& t, const Meeting& meet, int 
   if (meet.at != nullptr) {
     LatDiv d;
     int blocks = 0;
-    const cudaError_t e = chunk_shape(k_tmz_chunk_fwd<P>, t, d, blocks);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = chunk_shape(k_tmz_chunk_fwd<P>, t, d, blocks);
     GridDev gg = g;
     TmzDev tt = t;
     Meeting m = meet;
     int* error = wait_error_word();
     void* args[] = {&gg, &tt, &d, &m, &step0, &nsteps, &flags, &error};
-    return cudaLaunchCooperativeKernel((const void*)k_tmz_chunk_fwd<P>, dim3((unsigned)blocks),
-                                       dim3(kChunkThreads), args, 0, s);
+    if (e == cudaSuccess)
+      e = cudaLaunchCooperativeKernel((const void*)k_tmz_chunk_fwd<P>, dim3((unsigned)blocks),
+                                      dim3(kChunkThreads), args, 0, s);
+    if (!no_room(e)) return e;
+    (void)cudaGetLastError();
   }
   const dim3 grid = lattice_grid(t), block(kBX, kBY);
   for (int k = 0; k < nsteps; ++k) {
@@ -2266,15 +2268,17 @@ cudaError_t adjoint(const GridDev& g, const TmzDev& t, const Meeting& meet, int 
   if (meet.at != nullptr) {
     LatDiv d;
     int blocks = 0;
-    const cudaError_t e = chunk_shape(k_tmz_chunk_adj<P>, t, d, blocks);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = chunk_shape(k_tmz_chunk_adj<P>, t, d, blocks);
     GridDev gg = g;
     TmzDev tt = t;
     Meeting m = meet;
     int* error = wait_error_word();
     void* args[] = {&gg, &tt, &d, &m, &step0, &nsteps, &error};
-    return cudaLaunchCooperativeKernel((const void*)k_tmz_chunk_adj<P>, dim3((unsigned)blocks),
-                                       dim3(kChunkThreads), args, 0, s);
+    if (e == cudaSuccess)
+      e = cudaLaunchCooperativeKernel((const void*)k_tmz_chunk_adj<P>, dim3((unsigned)blocks),
+                                      dim3(kChunkThreads), args, 0, s);
+    if (!no_room(e)) return e;
+    (void)cudaGetLastError();
   }
   const dim3 grid = lattice_grid(t), block(kBX, kBY);
   for (int k = nsteps - 1; k >= 0; --k) {

@@ -509,19 +509,19 @@ constexpr int kTmzPmlE = 16, kTmzPmlX = 18, kTmzPmlY = 20, kTmzPlace = 22;  // b
 constexpr int kTmzPlaces = 511;
 static_assert(GMES_MAX_PML <= 4, "2-bit profile-set fields");
 
-cudaError_t launch_tmz_design(int precision, const GridDev& g, const TmzDev& t,
+[[nodiscard]] cudaError_t launch_tmz_design(int precision, const GridDev& g, const TmzDev& t,
                               const double* eps, cudaStream_t s);
-cudaError_t launch_tmz_forward(int precision, const GridDev& g, const TmzDev& t,
+[[nodiscard]] cudaError_t launch_tmz_forward(int precision, const GridDev& g, const TmzDev& t,
                                const Meeting& meet, int step0, int nsteps, int flags,
                                int block_steps, cudaStream_t s);
-cudaError_t launch_tmz_adjoint(int precision, const GridDev& g, const TmzDev& t,
+[[nodiscard]] cudaError_t launch_tmz_adjoint(int precision, const GridDev& g, const TmzDev& t,
                                const Meeting& meet, int step0, int nsteps, int block_steps,
                                cudaStream_t s);
 // Whether a call's steps run as one cooperative launch (given a barrier slot).
 bool tmz_chunked(int precision, const TmzDev& t, int block_steps);
 // Launches of one forward or adjoint call.
 int64_t tmz_launches(int precision, const TmzDev& t, int block_steps, int nsteps, bool adj);
-cudaError_t launch_tmz_objective(const GridDev& g, const TmzDev& t, int nsteps, double* J,
+[[nodiscard]] cudaError_t launch_tmz_objective(const GridDev& g, const TmzDev& t, int nsteps, double* J,
                                  cudaStream_t s);
 
 cudaError_t launch_points(const gmes_points& g, void* inplace, const void* in1, const void* in2,
@@ -547,12 +547,18 @@ cudaError_t clear_slots();
 // results (bytes at out) are spoiled where a block gave up.
 cudaError_t launch_wait_check(const Meeting& meet, int blocks, int absent, void* out,
                               int64_t bytes, cudaStream_t s);
-cudaError_t launch_persist(const Plan& p, const Meeting& meet, int nsteps, int st0,
-                           cudaStream_t s);
+// [[nodiscard]] here and below: a dropped status does not build (build.py).
+[[nodiscard]] cudaError_t launch_persist(const Plan& p, const Meeting& meet, int nsteps, int st0,
+                                         cudaStream_t s);
+// Whether a cooperative launch failed because its blocks do not fit together (a
+// context with fewer SMs than the device): the launches per half-step then do.
+inline bool no_room(cudaError_t e) {
+  return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources;
+}
 
 // Launchers implemented per precision in gmes_step.cu.
-cudaError_t launch_step(const gmes_grid_desc& g, const Plan& p, int nsteps, cudaStream_t s);
-cudaError_t launch_half(const gmes_grid_desc& g, const Plan& p, int side, int step,
+[[nodiscard]] cudaError_t launch_step(const gmes_grid_desc& g, const Plan& p, int nsteps, cudaStream_t s);
+[[nodiscard]] cudaError_t launch_half(const gmes_grid_desc& g, const Plan& p, int side, int step,
                         cudaStream_t s);
 // The descriptors of a batch of at most kParamJobs grids, passed by value
 // to the multi-grid cell kernel (kernel arguments are limited to 32764
@@ -566,14 +572,14 @@ static_assert(sizeof(BatchDescs) + 512 <= 32764, "batch descriptors exceed the a
 
 // host_jobs: host copies of the batch's descriptors (v.jobs), or NULL; with
 // them a batch of at most kParamJobs grids may take the argument-bank kernel.
-cudaError_t launch_batch(const BatchView& v, const GridDev* host_jobs, int precision, bool disp,
+[[nodiscard]] cudaError_t launch_batch(const BatchView& v, const GridDev* host_jobs, int precision, bool disp,
                          int nsteps, int blocks, cudaStream_t s);
-cudaError_t launch_raster(const gmes_grid_desc& gd, const GridDev& d, int c,
+[[nodiscard]] cudaError_t launch_raster(const gmes_grid_desc& gd, const GridDev& d, int c,
                           const gmes_shape* shapes, int nshapes, const uint8_t* lut,
                           cudaStream_t s);
-cudaError_t launch_build_coefficients(const gmes_grid_desc& g, const GridDev& d,
+[[nodiscard]] cudaError_t launch_build_coefficients(const gmes_grid_desc& g, const GridDev& d,
                                       cudaStream_t s);
-cudaError_t launch_nonfinite(const gmes_grid_desc& g, const GridDev& d, int32_t* flag,
+[[nodiscard]] cudaError_t launch_nonfinite(const gmes_grid_desc& g, const GridDev& d, int32_t* flag,
                              cudaStream_t s);
 
 }  // namespace gmes

@@ -574,7 +574,8 @@ __global__ void k_multi_sources(const BatchView v, int side, int s) {
 }
 
 template <class P, bool STRICT>
-cudaError_t run_steps(const Plan& p, int nsteps, int side_mask, int st0, cudaStream_t s);
+[[nodiscard]] cudaError_t run_steps(const Plan& p, int nsteps, int side_mask, int st0,
+                                    cudaStream_t s);
 
 // One half-step: ghost copy of the other half's components, the fused
 // update of this half's components, this half's point sources, TFSF
@@ -583,7 +584,7 @@ cudaError_t run_steps(const Plan& p, int nsteps, int side_mask, int st0, cudaStr
 // A complex grid runs every per-plane kernel on its real and imaginary
 // planes; only the ghost copy couples them.
 template <class P, bool STRICT>
-void run_half(const Plan& p, int side, int st, bool early, bool last, cudaStream_t s) {
+[[nodiscard]] cudaError_t run_half(const Plan& p, int side, int st, bool early, bool last, cudaStream_t s) {
   using T = typename P::T;
   const GridDev& d = p.re;
   int64_t maxplane = 1;
@@ -633,21 +634,26 @@ void run_half(const Plan& p, int side, int st, bool early, bool last, cudaStream
   if (side == 0 && p.incident != nullptr) {
     Meeting meet = p.incident->meet;
     if (!last) meet.done = nullptr;  // the call's last launch answers for all
-    if (meet.at != nullptr && persist_takes(*p.incident, 1))
-      launch_persist(*p.incident, meet, 1, st, s);
-    else
-      run_steps<P, STRICT>(*p.incident, 1, 3, st, s);
+    if (meet.at != nullptr && persist_takes(*p.incident, 1)) {
+      const cudaError_t e = launch_persist(*p.incident, meet, 1, st, s);
+      if (!no_room(e)) return e;
+      (void)cudaGetLastError();
+    }
+    return run_steps<P, STRICT>(*p.incident, 1, 3, st, s);
   }
+  return cudaSuccess;
 }
 
 template <class P, bool STRICT>
 cudaError_t run_steps(const Plan& p, int nsteps, int side_mask, int st0, cudaStream_t s) {
   for (int st = 0; st < nsteps; ++st) {
     const bool last = st + 1 == nsteps;
-    if (side_mask & 1) run_half<P, STRICT>(p, 0, st0 + st, st > 0, last, s);
-    if (side_mask & 2)
-      run_half<P, STRICT>(p, 1, st0 + st, (st > 0 || (side_mask & 1)) && p.incident == nullptr,
-                          last, s);
+    for (int side = 0; side < 2; ++side) {
+      if (!((side_mask >> side) & 1)) continue;
+      const bool early = side == 0 ? st > 0 : (st > 0 || (side_mask & 1)) && p.incident == nullptr;
+      const cudaError_t e = run_half<P, STRICT>(p, side, st0 + st, early, last, s);
+      if (e != cudaSuccess) return e;
+    }
   }
   return cudaGetLastError();
 }
@@ -775,8 +781,11 @@ cudaError_t launch_nonfinite(const gmes_grid_desc& g, const GridDev& d, int32_t*
 }
 
 cudaError_t launch_step(const gmes_grid_desc& g, const Plan& p, int nsteps, cudaStream_t s) {
-  if (p.meet.at != nullptr && persist_takes(p, nsteps))
-    return launch_persist(p, p.meet, nsteps, 0, s);
+  if (p.meet.at != nullptr && persist_takes(p, nsteps)) {
+    const cudaError_t e = launch_persist(p, p.meet, nsteps, 0, s);
+    if (!no_room(e)) return e;
+    (void)cudaGetLastError();
+  }
   return dispatch_precision(g, p, nsteps, 3, 0, s);
 }
 
