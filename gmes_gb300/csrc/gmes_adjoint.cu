@@ -665,7 +665,126 @@ __global__ void __launch_bounds__(kBX* kBY)
   if (lattice_point(t, p)) point_ae<P>(g, t, p, slot, rb, wb);
 }
 
+// Lattice points of all designs up to which a call's steps run as one
+// cooperative launch.  Measured on GB300, 60 steps forward / adjoint ms, two
+// launches per step -> one launch (with the sources in kernels of their own,
+// four launches per step, in brackets):
+//   FP64  128x123 x 1    (1.28 / 1.24)   0.74 / 0.75  -> 0.53 / 0.51
+//         256x251 x 4    (1.82 / 2.19)   1.33 / 1.74  -> 0.87 / 1.21
+//         400x395 x 24   (6.39 / 12.0)   5.80 / 11.6  -> 5.47 / 10.5
+//         512x507 x 64   (20.3 / 40.8)   19.4 / 40.5  -> 23.2 / 46.8
+//   df64  128x123 x 8    (1.39 / 1.27)   0.96 / 0.86  -> 0.63 / 0.60
+//         256x251 x 16   (2.20 / 2.61)   1.70 / 2.12  -> 1.53 / 2.25
+//         512x507 x 64   (19.7 / 29.6)   16.8 / 27.9  -> 22.0 / 43.3
+// A small lattice's half-step is bound by its launch; a large one by the FP64
+// pipe or L2, for which the one-launch kernel has fewer warps (62 registers).
+constexpr int64_t kChunkPoints = 1 << 22, kChunkPointsDf = 1 << 20;
+
 constexpr int kChunkThreads = 512;
+
+// A long list of point sources, walked entry by entry (per design): the kernels
+// that take it have t.nsrc = 0, so that their bodies look nothing up.
+struct SourceList {
+  const gmes_point_source* src;
+  const double* src_val;
+  int n;
+};
+// An entry of the list at point `at` of all designs' lattices.
+struct ListSource {
+  int comp, mode;  // comp -1: names no lattice point
+  int64_t at;
+};
+__device__ __forceinline__ ListSource list_source(const TmzDev& t, const SourceList& l, int b,
+                                                  int k) {
+  const gmes_point_source s = l.src[k];
+  const bool on = s.comp >= 2 && s.comp <= 4 && s.offset >= 0 && s.offset < t.plane;
+  return {on ? s.comp : -1, s.mode, (int64_t)b * t.plane + s.offset};
+}
+// Its action (entry k) in half `side` of step n of the forward, and in the
+// adjoint, where a hard source zeroes the adjoint of the value it overwrites.
+template <class P>
+__device__ __forceinline__ void source_fwd(const TmzDev& t, const SourceList& l, int side, int n,
+                                           const ListSource& s, int k) {
+  if (s.comp < 0 || (s.comp == 2) != (side == 0)) return;
+  typename P::T* f = static_cast<typename P::T*>(t.f[s.comp - 2]) + s.at;
+  const typename P::R was = P::ldw(f);  // issued with the value
+  const typename P::R v =
+      P::from_double(__ldg(l.src_val + ((int64_t)(n - 1) * 2 + side) * l.n + k));
+  P::st(f, s.mode == 0 ? v : was - v);
+}
+template <class P>
+__device__ __forceinline__ void source_adj(const TmzDev& t, int side, const ListSource& s) {
+  if (s.comp < 0 || s.mode != 0 || (s.comp == 2) != (side == 0)) return;
+  P::st(static_cast<typename P::T*>(t.l[s.comp - 2]) + s.at, P::zero());
+}
+template <class P>
+__global__ void k_tmz_src(const TmzDev t, const SourceList l, int side, int n) {
+  after_launch();
+  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= (int64_t)l.n * t.nb) return;
+  const int b = (int)(q / l.n), k = (int)(q - (int64_t)b * l.n);
+  source_fwd<P>(t, l, side, n, list_source(t, l, b, k), k);
+}
+template <class P>
+__global__ void k_tmz_adj_src(const TmzDev t, const SourceList l, int side) {
+  after_launch();
+  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= (int64_t)l.n * t.nb) return;
+  const int b = (int)(q / l.n), k = (int)(q - (int64_t)b * l.n);
+  source_adj<P>(t, side, list_source(t, l, b, k));
+}
+
+// The entries of a list that sit on this block's points (for_points), one-launch
+// kernels: found once per launch (the adjoint's: hard ones alone); a block with
+// more of them than fit walks the whole list.
+constexpr int kOwnSources = 1024;
+struct OwnSources {
+  int count;
+  unsigned at[kOwnSources];  // point | (comp - 2) << 24 | hard << 26
+  int entry[kOwnSources];
+};
+static_assert(kChunkPoints <= 1 << 24, "a point's place in 24 bits");
+// f(entry, number) for this block's share of the list.
+template <bool HARD, class F>
+__device__ __forceinline__ void walk_list(const TmzDev& t, const SourceList& l, F f) {
+  const unsigned all = (unsigned)l.n * (unsigned)t.nb;
+  for (unsigned q = threadIdx.x; q < all; q += kChunkThreads) {
+    const unsigned b = q / (unsigned)l.n, k = q - b * (unsigned)l.n;
+    const ListSource s = list_source(t, l, (int)b, (int)k);
+    if (s.comp >= 0 && !(HARD && s.mode != 0) &&
+        ((unsigned)s.at >> 5) % gridDim.x == blockIdx.x)
+      f(s, (int)k);
+  }
+}
+template <bool HARD>
+__device__ __forceinline__ void find_sources(const TmzDev& t, const SourceList& l, OwnSources& own) {
+  if (l.n == 0) return;
+  if (threadIdx.x == 0) own.count = 0;
+  __syncthreads();
+  walk_list<HARD>(t, l, [&](const ListSource& s, int k) {
+    const int q = atomicAdd(&own.count, 1);
+    if (q >= kOwnSources) return;
+    own.at[q] = (unsigned)s.at | (unsigned)(s.comp - 2) << 24 | (s.mode == 0 ? 1u << 26 : 0u);
+    own.entry[q] = k;
+  });
+  __syncthreads();
+}
+// f for each of them, after the block's points.
+template <bool HARD, class F>
+__device__ __forceinline__ void for_sources(const TmzDev& t, const SourceList& l,
+                                            const OwnSources& own, F f) {
+  if (l.n == 0 || own.count == 0) return;
+  __syncthreads();
+  if (own.count > kOwnSources) {
+    walk_list<HARD>(t, l, f);
+    return;
+  }
+  for (int q = threadIdx.x; q < own.count; q += kChunkThreads) {
+    const unsigned a = own.at[q];
+    f(ListSource{(int)(a >> 24 & 3) + 2, (int)(~a >> 26 & 1), (int64_t)(a & 0xffffffu)},
+      own.entry[q]);
+  }
+}
 
 // Groups of 32 points go round the blocks in turn, so that every SM gets its
 // share of the absorbing layer, the design and the sources.
@@ -683,8 +802,10 @@ __device__ __forceinline__ void for_points(const TmzDev& t, const LatDiv& d, F f
 template <class P>
 __global__ void __launch_bounds__(kChunkThreads, 2)
     k_tmz_chunk_fwd(const __grid_constant__ GridDev g, const __grid_constant__ TmzDev t,
-                    const LatDiv d, const __grid_constant__ Meeting meet, int step0, int nsteps, int flags, 
-                    int* error) {
+                    const LatDiv d, const SourceList l, const __grid_constant__ Meeting meet,
+                    int step0, int nsteps, int flags, int* error) {
+  __shared__ OwnSources own;
+  find_sources<false>(t, l, own);
   auto met = [&] {
     if (grid_barrier(meet, error)) return true;
     const int64_t es = sizeof(typename P::T), nd = (int64_t)t.dn[0] * t.dn[1];
@@ -699,10 +820,16 @@ __global__ void __launch_bounds__(kChunkThreads, 2)
     for_points(t, d, [&](const Lat& p) {
       point_fe<P>(g, t, p, n, (flags & GMES_TMZ_RECORD_HIST) ? k : -1);
     });
+    for_sources<false>(t, l, own, [&](const ListSource& s, int q) {
+      source_fwd<P>(t, l, 0, n, s, q);
+    });
     if (!met()) return;
     if (k + 1 == nsteps) leave_barrier(meet);
     for_points(t, d, [&](const Lat& p) {
       point_fh<P>(g, t, p, n, (flags & GMES_TMZ_RECORD_MONITOR) ? n - 1 : -1);
+    });
+    for_sources<false>(t, l, own, [&](const ListSource& s, int q) {
+      source_fwd<P>(t, l, 1, n, s, q);
     });
     if (k + 1 < nsteps && !met()) return;
   }
@@ -712,18 +839,28 @@ __global__ void __launch_bounds__(kChunkThreads, 2)
 template <class P>
 __global__ void __launch_bounds__(kChunkThreads, 2)
     k_tmz_chunk_adj(const __grid_constant__ GridDev g, const __grid_constant__ TmzDev t,
-                    const LatDiv d, const __grid_constant__ Meeting meet, int step0, int nsteps, int* error) {
+                    const LatDiv d, const SourceList l, const __grid_constant__ Meeting meet,
+                    int step0, int nsteps, int* error) {
+  __shared__ OwnSources own;
+  find_sources<true>(t, l, own);
   auto met = [&] {
     if (grid_barrier(meet, error)) return true;
     spoil(t.grad, (int64_t)t.nb * t.dn[0] * t.dn[1] * 8);
     return false;
   };
+  if (l.n > 0) {  // the H sources of the first step
+    for_sources<true>(t, l, own, [&](const ListSource& s, int) { source_adj<P>(t, 1, s); });
+    if (!met()) return;
+  }
   for (int k = nsteps - 1; k >= 0; --k) {
     const int n = step0 + k + 1, rb = n & 1, wb = rb ^ 1;
     for_points(t, d, [&](const Lat& p) { point_ah<P>(g, t, p, n, rb, wb); });
+    for_sources<true>(t, l, own, [&](const ListSource& s, int) { source_adj<P>(t, 0, s); });
     if (!met()) return;
     if (k == 0) leave_barrier(meet);
     for_points(t, d, [&](const Lat& p) { point_ae<P>(g, t, p, k, rb, wb); });
+    if (k > 0)
+      for_sources<true>(t, l, own, [&](const ListSource& s, int) { source_adj<P>(t, 1, s); });
     if (k > 0 && !met()) return;
   }
 }
@@ -2223,39 +2360,53 @@ cudaError_t chunk_shape(K* kernel, const TmzDev& t, LatDiv& d, int& blocks) {
   return cudaSuccess;
 }
 
-// Names the points of the sources as they are now: a caller may have set
-// others since the design.
-void map_sources(const TmzDev& t, cudaStream_t s) {
-  if (t.nsrc > 0) k_tmz_map_sources<<<(t.nsrc + 127) / 128, 128, 0, s>>>(t);
+// A call's sources: looked up in the bodies (u.nsrc > 0; their points are named
+// as they are now: a caller may have set others since the design), or a list.
+SourceList one_step_sources(TmzDev& u, cudaStream_t s) {
+  SourceList l = {u.src, u.src_val, 0};
+  if (u.nsrc > kTmzLookUp) {
+    l.n = u.nsrc;
+    u.nsrc = 0;
+  } else if (u.nsrc > 0) {
+    k_tmz_map_sources<<<(u.nsrc + 127) / 128, 128, 0, s>>>(u);
+  }
+  return l;
+}
+
+template <class K, class... A>
+cudaError_t launch_chunk(K* kernel, const GridDev& g, const TmzDev& t, const SourceList& l,
+                         const Meeting& meet, cudaStream_t s, A... steps) {
+  LatDiv d;
+  int blocks = 0;
+  const cudaError_t e = chunk_shape(kernel, t, d, blocks);
+  if (e != cudaSuccess) return e;
+  int* error = wait_error_word();
+  void* args[] = {(void*)&g, (void*)&t, &d, (void*)&l, (void*)&meet, &steps..., &error};
+  return cudaLaunchCooperativeKernel((const void*)kernel, dim3((unsigned)blocks),
+                                     dim3(kChunkThreads), args, 0, s);
 }
 
 template <class P>
 cudaError_t forward(const GridDev& g, const TmzDev& t, const Meeting& meet, int step0, int nsteps,
                     int flags, cudaStream_t s) {
   if (nsteps <= 0) return cudaSuccess;
-  map_sources(t, s);
+  TmzDev u = t;
+  const SourceList l = one_step_sources(u, s);
   if (meet.at != nullptr) {
-    LatDiv d;
-    int blocks = 0;
-    cudaError_t e = chunk_shape(k_tmz_chunk_fwd<P>, t, d, blocks);
-    GridDev gg = g;
-    TmzDev tt = t;
-    Meeting m = meet;
-    int* error = wait_error_word();
-    void* args[] = {&gg, &tt, &d, &m, &step0, &nsteps, &flags, &error};
-    if (e == cudaSuccess)
-      e = cudaLaunchCooperativeKernel((const void*)k_tmz_chunk_fwd<P>, dim3((unsigned)blocks),
-                                      dim3(kChunkThreads), args, 0, s);
+    const cudaError_t e = launch_chunk(k_tmz_chunk_fwd<P>, g, u, l, meet, s, step0, nsteps, flags);
     if (!no_room(e)) return e;
     (void)cudaGetLastError();
   }
   const dim3 grid = lattice_grid(t), block(kBX, kBY);
+  const dim3 entries((unsigned)(((int64_t)l.n * t.nb + 127) / 128));
   for (int k = 0; k < nsteps; ++k) {
     const int n = step0 + k + 1;
-    launch_after(k > 0, k_tmz_fe<P>, grid, block, 0, s, g, t, n,
+    launch_after(k > 0, k_tmz_fe<P>, grid, block, 0, s, g, u, n,
                  (flags & GMES_TMZ_RECORD_HIST) ? k : -1);
-    launch_after(true, k_tmz_fh<P>, grid, block, 0, s, g, t, n,
+    if (l.n > 0) launch_after(true, k_tmz_src<P>, entries, 128, 0, s, u, l, 0, n);
+    launch_after(true, k_tmz_fh<P>, grid, block, 0, s, g, u, n,
                  (flags & GMES_TMZ_RECORD_MONITOR) ? n - 1 : -1);
+    if (l.n > 0) launch_after(true, k_tmz_src<P>, entries, 128, 0, s, u, l, 1, n);
   }
   return cudaGetLastError();
 }
@@ -2264,28 +2415,24 @@ template <class P>
 cudaError_t adjoint(const GridDev& g, const TmzDev& t, const Meeting& meet, int step0, int nsteps,
                     cudaStream_t s) {
   if (nsteps <= 0) return cudaSuccess;
-  map_sources(t, s);
+  TmzDev u = t;
+  const SourceList l = one_step_sources(u, s);
   if (meet.at != nullptr) {
-    LatDiv d;
-    int blocks = 0;
-    cudaError_t e = chunk_shape(k_tmz_chunk_adj<P>, t, d, blocks);
-    GridDev gg = g;
-    TmzDev tt = t;
-    Meeting m = meet;
-    int* error = wait_error_word();
-    void* args[] = {&gg, &tt, &d, &m, &step0, &nsteps, &error};
-    if (e == cudaSuccess)
-      e = cudaLaunchCooperativeKernel((const void*)k_tmz_chunk_adj<P>, dim3((unsigned)blocks),
-                                      dim3(kChunkThreads), args, 0, s);
+    const cudaError_t e = launch_chunk(k_tmz_chunk_adj<P>, g, u, l, meet, s, step0, nsteps);
     if (!no_room(e)) return e;
     (void)cudaGetLastError();
   }
   const dim3 grid = lattice_grid(t), block(kBX, kBY);
+  const dim3 entries((unsigned)(((int64_t)l.n * t.nb + 127) / 128));
+  bool early = false;
   for (int k = nsteps - 1; k >= 0; --k) {
     const int n = step0 + k + 1;
     const int rb = n & 1, wb = rb ^ 1;
-    launch_after(k + 1 < nsteps, k_tmz_ah<P>, grid, block, 0, s, g, t, n, rb, wb);
-    launch_after(true, k_tmz_ae<P>, grid, block, 0, s, g, t, k, rb, wb);
+    if (l.n > 0) launch_after(early, k_tmz_adj_src<P>, entries, 128, 0, s, u, l, 1);
+    launch_after(early || l.n > 0, k_tmz_ah<P>, grid, block, 0, s, g, u, n, rb, wb);
+    if (l.n > 0) launch_after(true, k_tmz_adj_src<P>, entries, 128, 0, s, u, l, 0);
+    launch_after(true, k_tmz_ae<P>, grid, block, 0, s, g, u, k, rb, wb);
+    early = true;
   }
   return cudaGetLastError();
 }
@@ -2429,23 +2576,9 @@ cudaError_t launch_tmz_design(int precision, const GridDev& g, const TmzDev& t,
   return cudaGetLastError();
 }
 
-// Lattice points of all designs up to which a call's steps run as one
-// cooperative launch.  Measured on GB300, 60 steps forward / adjoint ms, two
-// launches per step -> one launch (with the sources in kernels of their own,
-// four launches per step, in brackets):
-//   FP64  128x123 x 1    (1.28 / 1.24)   0.74 / 0.75  -> 0.53 / 0.51
-//         256x251 x 4    (1.82 / 2.19)   1.33 / 1.74  -> 0.87 / 1.21
-//         400x395 x 24   (6.39 / 12.0)   5.80 / 11.6  -> 5.47 / 10.5
-//         512x507 x 64   (20.3 / 40.8)   19.4 / 40.5  -> 23.2 / 46.8
-//   df64  128x123 x 8    (1.39 / 1.27)   0.96 / 0.86  -> 0.63 / 0.60
-//         256x251 x 16   (2.20 / 2.61)   1.70 / 2.12  -> 1.53 / 2.25
-//         512x507 x 64   (19.7 / 29.6)   16.8 / 27.9  -> 22.0 / 43.3
-// A small lattice's half-step is bound by its launch; a large one by the FP64
-// pipe or L2, for which the one-launch kernel has fewer warps (62 registers).
-constexpr int64_t kChunkPoints = 1 << 22, kChunkPointsDf = 1 << 20;
-
 bool tmz_chunked(int precision, const TmzDev& t, int block_steps) {
   return steps_per_launch(precision, t, block_steps) == 1 && wait_error_word() != nullptr &&
+         (int64_t)t.nsrc * t.nb < (int64_t(1) << 31) &&
          t.plane * t.nb <= (precision == GMES_DF64 ? kChunkPointsDf : kChunkPoints);
 }
 
@@ -2453,7 +2586,9 @@ int64_t tmz_launches(int precision, const TmzDev& t, int block_steps, int nsteps
   const int per = steps_per_launch(precision, t, block_steps);
   if (nsteps <= 0) return 0;
   if (per > 1) return adj ? adj_launches(nsteps, per) : (nsteps + per - 1) / per;
-  return (t.nsrc > 0) + (tmz_chunked(precision, t, block_steps) ? 1 : 2 * (int64_t)nsteps);
+  const bool list = t.nsrc > kTmzLookUp, named = t.nsrc > 0 && !list;
+  if (tmz_chunked(precision, t, block_steps)) return named + 1;
+  return named + (list ? 4 : 2) * (int64_t)nsteps;
 }
 
 cudaError_t launch_tmz_forward(int precision, const GridDev& g, const TmzDev& t,

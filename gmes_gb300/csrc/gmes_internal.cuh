@@ -507,6 +507,18 @@ enum : uint32_t {
 };
 constexpr int kTmzPmlE = 16, kTmzPmlX = 18, kTmzPmlY = 20, kTmzPlace = 22;  // bit offsets
 constexpr int kTmzPlaces = 511;
+// The one-step kernels' bodies look their points' sources up (a point of both an
+// E and an H source searches back through the list) in lists of at most this
+// many entries; longer lists are walked entry by entry.  Measured on GB300 (FP64
+// 300x243, 60 steps forward / adjoint ms): in kernels of their own, four plain
+// launches per step; looked up; walked
+//   13 Ez                             1.41 / 1.28   0.61 / 0.64   -
+//   60 Ez + 60 Hy on the same points  1.48 / 1.28   1.43 / 2.07   0.62 / 0.64
+//   250 Ez + 250 Hy                   1.46 / 1.40   4.62 / 7.39   0.62 / 0.64
+//   5000 Ez                           1.57 / 1.42   15.7 / 16.1   0.78 / 0.67
+// (a short list: no walk, no list in shared memory; 163 Ez, each alone on its
+// point, looked up / walked in FP32 x 6 designs: 0.78 / 0.82 forward)
+constexpr int kTmzLookUp = 32;
 static_assert(GMES_MAX_PML <= 4, "2-bit profile-set fields");
 
 [[nodiscard]] cudaError_t launch_tmz_design(int precision, const GridDev& g, const TmzDev& t,
