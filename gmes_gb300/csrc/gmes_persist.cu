@@ -382,12 +382,24 @@ __global__ void __launch_bounds__(kPersistThreads, GMES_PERSIST_BLOCKS)
 }
 
 // Shared memory of the tables: at most kTabMost, so that two blocks stay
-// resident on an SM; a grid that needs more does without them.
+// resident on an SM; a grid that needs more does without them, and so does a call
+// too short to earn what building them takes.  Measured on GB300, us per step of
+// calls of 1 / 2 / 4 / 20 steps, six launches per step | tables | none:
+//   64^2   FP64  18.9 16.4 15.9 15.2 | 16.7 10.9  8.3  6.1 | 14.5 10.6  8.8  7.2
+//   600^2  FP32  29.0 27.2 26.3 25.8 | 27.0 17.7 13.9 10.7 | 22.5 16.6 14.4 12.6
+//   900^2  FP64  76.2 73.9 72.8 72.5 | 49.8 36.0 28.3 22.3 | 37.3 28.9 26.5 24.6
+//   24^3   df64  20.8 19.6 18.5 17.8 | 22.1 14.5 10.8  7.7 | 16.8 12.4 10.1  8.4
+//   32^3   FP32  20.7 18.8 18.1 17.6 | 20.9 13.5  9.9  7.2 | 15.3 11.5  9.3  7.6
+// Beyond the tables' reach (every component's axes and cells in kTabMost), calls
+// of 20 steps, six launches | none: 1024^2 FP64 88.9 | 43.0, 4096^2 FP64 1266 | 749,
+// FP32 766 | 609, df64 950 | 862, 6000x6500 FP32 1761 | 968.
 constexpr int kTabMost = 100 * 1024;
+constexpr int kTabSteps = 4;
 
-TabLayout table_layout(const GridDev& d, int per, int es) {
+TabLayout table_layout(const GridDev& d, int per, int es, int nsteps) {
   TabLayout L;
   std::memset(&L, 0, sizeof(L));
+  if (nsteps < kTabSteps) return L;
   int64_t off = 0;
   for (int c = 0; c < 6; ++c) {
     if (!((d.active >> c) & 1)) continue;
@@ -432,7 +444,7 @@ cudaError_t launch_one(const Plan& p, const Meeting& meet, int nsteps, int st0, 
   c.nsteps = nsteps;
   c.meet = meet;
   c.st0 = st0;
-  c.tab = table_layout(d, per, (int)sizeof(typename P::T));
+  c.tab = table_layout(d, per, (int)sizeof(typename P::T), nsteps);
   GridDev re = p.re, im = p.im;
   int* error = wait_error_word();
   void* args[] = {&re, &im, &c, &error};
@@ -471,21 +483,21 @@ cudaError_t launch_disp(const Plan& p, const Meeting& meet, int nsteps, int st0,
 //               df64 132 -> 67, 2000^2 FP64 313 -> 127 FP32 189 -> 91
 // Grids of at most three components gain at every size (only their active
 // components' points are visited, with the inactive curl terms left out), from
-// the first step on (64^2 FP64 19.1 -> 17.1, 301x277 20.9 -> 20.4).  3-D grids
+// the first step on (64^2 FP64 18.9 -> 14.5, 300^2 21.0 -> 16.5).  3-D grids
 // gain while their launches weigh more than the one-plane kernel's shared
-// neighbour loads, and in calls long enough for the tables; with the launches
-// overlapped, a call of 1 / 2 / 4 / 20 steps:
-//   48x40x44 FP64   26.9 -> 30.9   25.8 -> 23.4   25.4 -> 19.3   25.0 -> 15.9
-//            FP32   21.2 -> 25.1   18.7 -> 16.5   17.2 -> 12.9   16.7 ->  9.8
-//            df64   22.5 -> 26.9   20.0 -> 19.2   19.0 -> 14.9   18.5 -> 11.8
-//   24^3     FP64   26.3 -> 22.0   22.3 -> 14.8   21.1 -> 10.9   21.0 ->  7.6
-//   32^3     FP32   21.5 -> 21.1   18.0 -> 13.5   16.0 -> 10.0   15.7 ->  7.0
-//   64^3     FP64   38.7 -> 54.0   36.3 -> 45.6   34.7 -> 41.0   33.8 -> 37.0
-//            FP32   25.0 -> 36.0   22.1 -> 26.9   20.0 -> 22.3   18.9 -> 18.6
+// neighbour loads; with the launches overlapped, a call of 1 / 2 / 4 / 20 steps
+// (in brackets: with the tables that short calls no longer build):
+//   48x40x44 FP64   26.9 -> (30.9)   23.7 -> 17.6   23.2 -> 19.1   22.3 -> 16.0
+//            FP32   21.2 -> (25.1)   19.6 -> 14.6   18.5 -> 13.4   17.8 -> 10.4
+//            df64   22.5 -> (26.9)   20.6 -> 16.5   19.2 -> 15.0   18.9 -> 12.1
+//   24^3     FP64   24.9 -> 16.7     22.7 -> 12.5   22.5 -> 10.4   21.5 ->  7.6
+//   32^3     FP32   20.7 -> 15.4     18.8 -> 11.5   18.1 -> 10.3   17.6 ->  7.3
+//   64^3     FP64   38.7 -> (54.0)   36.3 -> (45.6)   34.7 -> 41.0   33.8 -> 37.0
+//            FP32   25.0 -> (36.0)   22.1 -> (26.9)   20.0 -> 22.3   18.9 -> 18.6
 //   63x45x37 Drude / Lorentz / DCP + UPML
-//            FP64   42.8 -> 37.5   40.5 -> 30.9   38.6 -> 27.1   37.7 -> 24.0
-//   complex 32x32x30 28.6 -> 20.9  25.6 -> 14.7   24.7 -> 11.9   27.1 ->  9.4
-//   complex 64x64x48 41.5 -> 41.5  39.8 -> 35.0   38.5 -> 32.3   37.5 -> 29.4
+//            FP64   42.8 -> (37.5)   40.5 -> (30.9)   38.6 -> 27.1   37.7 -> 24.0
+//   complex 32x31x30  27.0 -> 20.6   25.8 -> 15.5   25.2 -> 11.8   24.5 ->  9.6
+//   complex 64x64x48  41.5 -> (41.5)   39.8 -> (35.0)   38.5 -> 32.3   37.5 -> 29.4
 constexpr int64_t kPersistCells = 1 << 17, kPersistCellsComplex = 1 << 18;
 constexpr int64_t kPersistCellsOneStep = 1 << 15;
 
