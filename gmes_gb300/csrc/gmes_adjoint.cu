@@ -277,6 +277,11 @@ __device__ __forceinline__ void adje_cpml(const GridDev& g, unsigned fl, typenam
   }
 }
 
+// dJ/dE_n of a monitor value e of a design of weight w.
+__device__ __forceinline__ double seed_value(const GridDev& g, double w, double e) {
+  return 2.0 * g.dt * w * e;
+}
+
 // Objective seed of lattice point (i, j) of design b at reverse step n:
 // dJ/dE_n = 2 dt w_b E_n on monitor points (*has), nothing elsewhere.
 __device__ __forceinline__ double seed_of(const GridDev& g, const TmzDev& t, int b, int i, int j,
@@ -287,7 +292,7 @@ __device__ __forceinline__ double seed_of(const GridDev& g, const TmzDev& t, int
   const int64_t nm = (int64_t)t.mn[0] * t.mn[1];
   const double w = t.weight != nullptr ? t.weight[b] : 1.0;
   const double e = t.mon[((int64_t)b * t.total_steps + (n - 1)) * nm + m];
-  return 2.0 * g.dt * w * e;
+  return seed_value(g, w, e);
 }
 
 // ---------------------------------------------------------------------------
@@ -1401,9 +1406,11 @@ struct TbSpecial {
   using T = typename P::T;
   using G = TbGeom<P, Q>;
   unsigned row[Q];
+  unsigned mine;   // the lane's points, bit 2 q + h: on the monitor; 8 above: its own pixels
   uint16_t* map;   // Ez sources
   double* acc;     // gradient of the launch, then -1 / eps, per region point
   R v[Q][2];       // source values (forward) or design increments (adjoint)
+  R seeds[Q][2];   // adjoint
   __device__ __forceinline__ void init(unsigned char* smem) {
     acc = reinterpret_cast<double*>(smem + G::kHead * sizeof(R));
     map = reinterpret_cast<uint16_t*>(acc + 2 * G::NP);
@@ -1427,9 +1434,17 @@ struct TbSpecial {
   }
   __device__ __forceinline__ void load(const TmzDev& t, const TbPlace<P, Q>& p,
                                        const TbTile<R>& tile) {
+    mine = 0;
 #pragma unroll
-    for (int q = 0; q < Q; ++q)
-      row[q] = __reduce_or_sync(0xffffffffu, flags(t, p, q, 0) | flags(t, p, q, 1));
+    for (int q = 0; q < Q; ++q) {
+      const unsigned f[2] = {flags(t, p, q, 0), flags(t, p, q, 1)};
+      row[q] = __reduce_or_sync(0xffffffffu, f[0] | f[1]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (f[h] & kTmzMonitor) mine |= 1u << (2 * q + h);
+        if ((f[h] & kTmzDesign) && owned(t, p, q, h)) mine |= 256u << (2 * q + h);
+      }
+    }
     if (tile.any & kTmzSrcE) tb_source_map<P, Q>(t, p.ri0, p.rj0, map);
   }
   // forward: the sources' values of step n, fetched a step ahead
@@ -1462,17 +1477,33 @@ struct TbSpecial {
         t.mon[((int64_t)p.b * t.total_steps + (n - 1)) * t.mn[0] * t.mn[1] +
               monitor_index(t, p.li[q], h ? p.j1 : p.j0)] = to_double(e[h]);
   }
-  // adjoint: the objective's seed, hard sources, and the design gradient,
-  // which accumulates in shared memory over the launch
-  __device__ __forceinline__ void seed(const GridDev& g, const TmzDev& t, const TbPlace<P, Q>& p,
-                                       int q, int n, R e[2]) const {
-    if (!(row[q] & kTmzMonitor)) return;
+  // adjoint: the objective's seeds of step n and the design increments of slot,
+  // fetched together and a step ahead (one after another in the rows, with the
+  // flags read again, the tiles of a 200x200 design took 16.5 us per launch, the
+  // slowest 31; now 14 and 24); hard sources; and the design gradient, which
+  // accumulates in shared memory over the launch
+  __device__ __forceinline__ void seed_fetch(const GridDev& g, const TmzDev& t,
+                                             const TbPlace<P, Q>& p, int n) {
+    if ((mine & 255u) == 0) return;
+    const double w = t.weight != nullptr ? t.weight[p.b] : 1.0;
+    const double* at =
+        t.mon + ((int64_t)p.b * t.total_steps + (n - 1)) * t.mn[0] * t.mn[1];
+    double m[Q][2];
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        m[q][h] = (mine >> (2 * q + h)) & 1
+                      ? at[monitor_index(t, p.li[q], h ? p.j1 : p.j0)] : 0.0;
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) seeds[q][h] = P::from_double(seed_value(g, w, m[q][h]));
+  }
+  __device__ __forceinline__ void seed(int q, R e[2]) const {
 #pragma unroll
     for (int h = 0; h < 2; ++h)
-      if (flags(t, p, q, h) & kTmzMonitor) {
-        bool has;
-        e[h] = e[h] + P::from_double(seed_of(g, t, p.b, p.li[q], h ? p.j1 : p.j0, n, &has));
-      }
+      if ((mine >> (2 * q + h)) & 1) e[h] = e[h] + seeds[q][h];
   }
   __device__ __forceinline__ void zero(const TbPlace<P, Q>& p, int q, R e[2]) const {
     if (!(row[q] & kTmzSrcE)) return;
@@ -1486,7 +1517,7 @@ struct TbSpecial {
       if (row[q] & kTmzDesign) {
 #pragma unroll
         for (int h = 0; h < 2; ++h)
-          if ((flags(t, p, q, h) & kTmzDesign) && owned(t, p, q, h)) f(q, h, pixel(t, p, q, h));
+          if ((mine >> (8 + 2 * q + h)) & 1) f(q, h, pixel(t, p, q, h));
       }
   }
   __device__ __forceinline__ void grad_load(const TmzDev& t, const TbPlace<P, Q>& p) {
@@ -1502,12 +1533,10 @@ struct TbSpecial {
       v[q][h] = P::ldw(static_cast<const T*>(t.hist) + b + dp);
     });
   }
-  __device__ __forceinline__ void grad_add(const TmzDev& t, const TbPlace<P, Q>& p, int q,
-                                           const R e[2]) {
-    if (!(row[q] & kTmzDesign)) return;
+  __device__ __forceinline__ void grad_add(const TbPlace<P, Q>& p, int q, const R e[2]) {
 #pragma unroll
     for (int h = 0; h < 2; ++h)
-      if ((flags(t, p, q, h) & kTmzDesign) && owned(t, p, q, h)) {
+      if ((mine >> (8 + 2 * q + h)) & 1) {
         const int k = at(p, q, h);
         acc[k] += to_double(e[h]) * to_double(v[q][h]) * acc[G::NP + k];
       }
@@ -1755,10 +1784,15 @@ __device__ void tb_general_adj(const GridDev& g, const TmzDev& t, int n0, int ns
   unsigned fl[Q];
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
-    const int a = ty + kRowsAtOnce * q, k = a * RJ + c;
+    const int a = ty + kRowsAtOnce * q;
     li[q] = wrap_index(ri0 + a, t.nx);
     fl[q] = tb_point<P>(t, b, li[q], j, pt[q]);
     if (jtile && a >= H && a < H + TI && ri0 + a < t.nx) fl[q] |= 1u << 31;  // tile point
+  }
+  after_previous();
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const int k = (ty + kRowsAtOnce * q) * RJ + c;
     const int64_t lin = base + (int64_t)li[q] * t.ny + j;
     sLE[k] = static_cast<const T*>(t.l[0])[lin];
     sLX[k] = static_cast<const T*>(t.l[1])[lin];
@@ -2054,10 +2088,15 @@ __global__ void __launch_bounds__(kTbThreads, 2)
 // point and the gradient, lambda_X / lambda_Y gathering those.  The weights of
 // the neighbour along j come by a shuffle, those along i from the lane or the
 // next warp's row (w2 of its last row, v1 of its first).
+//
+// What no kernel of the chain writes is read before the wait for the launch
+// before: the tile's record and, in special and general tiles, the map and the
+// first step's seeds and increments.  Adjoint of 200x200 x 3, 100 steps, ms: all
+// after the wait 0.59, so 0.52.
 template <class P, int Q>
 __global__ void __launch_bounds__(kTbThreads, 2)
     k_tmz_tb_adj(const GridDev g, const TmzDev t, int n0, int nsub, int step0, int rb) {
-  after_launch();
+  release_next();
   using R = typename P::R;
   using G = TbGeom<P, Q>;
   using Two = Row2<R>;
@@ -2077,12 +2116,16 @@ __global__ void __launch_bounds__(kTbThreads, 2)
   const TbPlace<P, Q> p(t);
   const int lane = p.lane, w = p.warp;
   R e[Q][2], x[Q][2], y[Q][2];
+  auto load = [&] {
+    after_previous();
 #pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    p.load(t, t.l[0], q, e[q]);
-    p.load(t, t.l[1], q, x[q]);
-    p.load(t, t.l[2], q, y[q]);
-  }
+    for (int q = 0; q < Q; ++q) {
+      p.load(t, t.l[0], q, e[q]);
+      p.load(t, t.l[1], q, x[q]);
+      p.load(t, t.l[2], q, y[q]);
+    }
+  };
+  if (!tile.fancy) load();  // a special tile has more to do first
   if (w == 0) sU[lane] = Two{P::zero(), P::zero()};
   if (w == kTbWarps - 1) sD[kTbWarps * 32 + lane] = Two{P::zero(), P::zero()};
   constexpr unsigned kAll = 0xffffffffu;
@@ -2099,6 +2142,17 @@ __global__ void __launch_bounds__(kTbThreads, 2)
     if constexpr (SP) {
       sp.init(tb_smem);
       sp.load(t, p, tile);
+    }
+    // the seeds and increments of step n, fetched a step ahead
+    auto fetch = [&](int n) {
+      if constexpr (SP) {
+        if (design) sp.grad_fetch(t, p, n - step0 - 1);
+        if (mon) sp.seed_fetch(g, t, p, n);
+      }
+    };
+    fetch(n0 + nsub);
+    if constexpr (SP) {
+      load();
       if (design) sp.grad_load(t, p);
     }
     if constexpr (LAYER) {
@@ -2125,8 +2179,6 @@ __global__ void __launch_bounds__(kTbThreads, 2)
     __syncthreads();
     for (int s = nsub - 1; s >= 0; --s) {
       const int n = n0 + s + 1;
-      if constexpr (SP)
-        if (design) sp.grad_fetch(t, p, n - step0 - 1);
       const Two up = sU[w * 32 + lane];
       R u[2] = {up.a, up.b};
       R v1[Q][2], v2[Q][2];
@@ -2142,7 +2194,7 @@ __global__ void __launch_bounds__(kTbThreads, 2)
         }
         const R wl = __shfl_up_sync(kAll, wx[1], 1);
         if constexpr (SP)
-          if (mon) sp.seed(g, t, p, q, n, e[q]);
+          if (mon) sp.seed(q, e[q]);
         e[q][0] = e[q][0] + ((wl - wx[0]) + (u[0] - ya[q][0]));
         e[q][1] = e[q][1] + ((wx[0] - wx[1]) + (u[1] - ya[q][1]));
         u[0] = ya[q][0];
@@ -2161,8 +2213,9 @@ __global__ void __launch_bounds__(kTbThreads, 2)
           }
         }
         if constexpr (SP)
-          if (design) sp.grad_add(t, p, q, e[q]);
+          if (design) sp.grad_add(p, q, e[q]);
       }
+      if (s > 0) fetch(n - 1);
       sD[w * 32 + lane] = Two{v1[0][0], v1[0][1]};
       __syncthreads();
       const Two dn = sD[(w + 1) * 32 + lane];
@@ -2471,15 +2524,30 @@ cudaError_t copy_state(void* const* dst, void* const* src, int n, int64_t bytes,
 // threads at 128 registers, 4 rows 15.9 / 18.0, 6 rows 17.2 / 30.0.
 constexpr int kTbQ = 2;
 
+// Shared memory of a launch of `blocks` blocks that need `bytes` each, at most
+// kTbSmemMost.  A launch that one block per SM holds asks for more than half an
+// SM: with the next launch's blocks coming up beside it, the SMs left over would
+// otherwise take two of its blocks, and the slowest tile sets its time.  Measured
+// on GB300, 100 steps forward / adjoint ms (plain launches of the kernels before |
+// overlapped | overlapped, one block per SM):
+//   100x100 x 12   0.724 / 0.541   0.739 / 0.595   0.636 / 0.447
+//   128x123 x 8    0.732 / 0.513   0.653 / 0.568   0.580 / 0.433
+//   200x200 x 3    0.675 / 0.566   0.578 / 0.517   0.563 / 0.462
+constexpr size_t kTbSmemMost = 116 * 1024;
+size_t launch_smem(size_t bytes, unsigned blocks) {
+  return blocks <= (unsigned)sm_count() ? kTbSmemMost : bytes;
+}
+
 template <class P, int Q>
 cudaError_t forward_blocked(const GridDev& g, const TmzDev& t, int step0, int nsteps, int flags,
                             int per_launch, cudaStream_t s) {
-  constexpr size_t smem = TbGeom<P, Q>::fwd_bytes;
+  const unsigned grid = tb_tiles<P, Q>(t) * (unsigned)t.nb;
+  static_assert(TbGeom<P, Q>::fwd_bytes <= kTbSmemMost, "the attribute below");
+  const size_t smem = launch_smem(TbGeom<P, Q>::fwd_bytes, grid);
   cudaError_t e = cudaFuncSetAttribute(k_tmz_tb_fwd<P, Q>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTbSmemMost);
   if (e != cudaSuccess) return e;
   if (t.tmp[0] == nullptr) return cudaErrorInvalidValue;
-  const unsigned grid = tb_tiles<P, Q>(t) * (unsigned)t.nb;
   const int launches = (nsteps + per_launch - 1) / per_launch;
   TmzDev u = t;
   if (launches % 2 == 1) {
@@ -2514,13 +2582,14 @@ int adj_launches(int nsteps, int per_launch) {
 template <class P, int Q>
 cudaError_t adjoint_blocked(const GridDev& g, const TmzDev& t, int step0, int nsteps,
                             int per_launch, cudaStream_t s) {
-  constexpr size_t smem = TbGeom<P, Q>::adj_bytes;
+  const unsigned grid = tb_tiles<P, Q>(t) * (unsigned)t.nb;
+  static_assert(TbGeom<P, Q>::adj_bytes <= kTbSmemMost, "the attribute below");
+  const size_t smem = launch_smem(TbGeom<P, Q>::adj_bytes, grid);
   cudaError_t e = cudaFuncSetAttribute(k_tmz_tb_adj<P, Q>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTbSmemMost);
   if (e != cudaSuccess) return e;
   if (t.tmp[0] == nullptr) return cudaErrorInvalidValue;
   if (nsteps <= 0) return cudaSuccess;
-  const unsigned grid = tb_tiles<P, Q>(t) * (unsigned)t.nb;
   const int launches = adj_launches(nsteps, per_launch);
   TmzDev u = t;
   if (launches % 2 == 1) {
