@@ -158,10 +158,14 @@ class Batch:
             return 0
         return 2 * (int(self.b.ghosts > 0) + 1 + int(self.b.srcs > 0))
 
-    def _solo_launches_per_step(self, i):
-        """Launches of one single-grid step: per half-step the ghost copy, the
-        cell update and the sources (when the grid has any)."""
-        return 2 * (2 + int(self.engines[i].desc.nsrc > 0))
+    def _solo_launches(self, i, k):
+        """Launches of k single-grid steps: one call's (a small grid takes one),
+        per half-step otherwise the ghost copy, the cell update and the sources
+        (when the grid has any)."""
+        e = self.engines[i]
+        if hasattr(e, "step_launches"):
+            return e.step_launches(k)
+        return 2 * k * (2 + int(e.desc.nsrc > 0))
 
     def _one_launch(self, i, k):
         """Whether grid i's chunk of k steps is a single launch."""
@@ -170,8 +174,8 @@ class Batch:
 
     @property
     def launches_per_step(self):
-        """Kernel launches of one step of every grid of the batch."""
-        return self._multi_launches_per_step() + sum(self._solo_launches_per_step(i)
+        """Kernel launches of a run of one step of every grid of the batch."""
+        return self._multi_launches_per_step() + sum(self._solo_launches(i, 1)
                                                      for i in self.solo)
 
     def run(self, steps, n0s=None):
@@ -228,8 +232,7 @@ class Batch:
                 N.check(self.lib.gmes_graph_launch(C.c_void_p(e._graph(s)), sst))
             else:
                 N.check(self.lib.gmes_step(C.byref(e.desc), s, sst))
-            launched += (e.step_launches(s) if hasattr(e, "step_launches")
-                         else s * self._solo_launches_per_step(i))
+            launched += self._solo_launches(i, s)
         for ss in side:
             self.stream.wait_stream(ss)
         return launched

@@ -2342,7 +2342,6 @@ __global__ void __launch_bounds__(kTbThreads) k_tmz_tiles(const TmzDev t) {
     o.pm = (int)pm;
     for (int k = 0; k < 4; ++k) o.c[k] = c[k];
     for (int k = 0; k < 3; ++k) o.d[k] = c[4 + k];
-    o.e = P::zero();
     static_cast<TbTile<R>*>(t.tiles)[blockIdx.x] = o;
   }
 }

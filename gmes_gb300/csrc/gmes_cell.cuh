@@ -618,32 +618,31 @@ __device__ __forceinline__ uint8_t ldc(const GridDev& g, I off) {
   return __ldg(g.cls[C] + off);
 }
 
-template <class P, int MASK, int C, bool STRICT, bool DISP>
+template <class P, int C, bool STRICT, bool DISP>
 __device__ __forceinline__ void upd(const GridDev& g, int64_t lin, const int x[3],
                                     typename P::R p1, typename P::R p2, typename P::R F,
                                     uint8_t id, Pre<P> pre) {
-  if (!is_active<MASK, C>(g)) return;
+  if (!is_active<0, C>(g)) return;
   if constexpr (STRICT)
     update_strict<C, DISP>(g, lin, x, p1, p2, F, id);
   else
     update_fast<P, C, DISP>(g, lin, x, p1, p2, F, id, pre);
 }
 
-template <class P, int MASK, int C, bool STRICT>
+template <class P, int C, bool STRICT>
 __device__ __forceinline__ Pre<P> pre_of(const GridDev& g, int64_t lin, const int x[3],
                                          uint8_t id) {
   if constexpr (STRICT) {
     return Pre<P>{P::zero(), P::zero()};
   } else {
-    if (!is_active<MASK, C>(g)) return Pre<P>{P::zero(), P::zero()};
+    if (!is_active<0, C>(g)) return Pre<P>{P::zero(), P::zero()};
     return prefetch_state<P, C>(g, lin, x, id);
   }
 }
 
-// MASK: the active-component mask when known at compile time, 0 when read
-// from the grid; I: offset type (int32_t for grids whose components hold
+// I: offset type (int32_t for grids whose components hold
 // fewer than 2^31 points, int64_t otherwise).
-template <class P, int SIDE, bool STRICT, bool DISP, int MASK, class I>
+template <class P, int SIDE, bool STRICT, bool DISP, class I>
 __device__ __forceinline__ void cell_body(const GridDev& g, int i, int j, int k) {
   using R = typename P::R;
   const I s00 = (I)g.st[0][0], s01 = (I)g.st[0][1], s10 = (I)g.st[1][0], s11 = (I)g.st[1][1];
@@ -656,53 +655,53 @@ __device__ __forceinline__ void cell_body(const GridDev& g, int i, int j, int k)
     const I lx = ii * s00 + jj * s01 + kk;
     const I ly = ii * s10 + jj * s11 + kk;
     const I lz = ii * s20 + jj * s21 + kk;
-    const uint8_t idx = ldc<MASK, 0>(g, lx), idy = ldc<MASK, 1>(g, ly), idz = ldc<MASK, 2>(g, lz);
-    const R ex = ldf<P, MASK, 0>(g, lx), ey = ldf<P, MASK, 1>(g, ly), ez = ldf<P, MASK, 2>(g, lz);
+    const uint8_t idx = ldc<0, 0>(g, lx), idy = ldc<0, 1>(g, ly), idz = ldc<0, 2>(g, lz);
+    const R ex = ldf<P, 0, 0>(g, lx), ey = ldf<P, 0, 1>(g, ly), ez = ldf<P, 0, 2>(g, lz);
     // neighbour H values
     const I hx = ii * s30 + jj * s31 + kk;         // Hx[i, j, k]
     const I hy = (ii + 1) * s40 + jj * s41 + kk;   // Hy[i+1, j, k]
     const I hz = (ii + 1) * s50 + jj * s51 + kk;   // Hz[i+1, j, k]
-    const R hz_a = ldf<P, MASK, 5>(g, hz + s51);          // Hz[i+1, j+1, k]
-    const R hz_b = ldf<P, MASK, 5>(g, hz);                // Hz[i+1, j,   k]
-    const R hz_c = ldf<P, MASK, 5>(g, hz + s51 - s50);    // Hz[i,   j+1, k]
-    const R hy_a = ldf<P, MASK, 4>(g, hy + 1);            // Hy[i+1, j, k+1]
-    const R hy_b = ldf<P, MASK, 4>(g, hy);                // Hy[i+1, j, k]
-    const R hy_c = ldf<P, MASK, 4>(g, hy + 1 - s40);      // Hy[i,   j, k+1]
-    const R hx_a = ldf<P, MASK, 3>(g, hx + s31 + 1);      // Hx[i, j+1, k+1]
-    const R hx_b = ldf<P, MASK, 3>(g, hx + s31);          // Hx[i, j+1, k]
-    const R hx_c = ldf<P, MASK, 3>(g, hx + 1);            // Hx[i, j,   k+1]
-    const Pre<P> px = pre_of<P, MASK, 0, STRICT>(g, lx, xc, idx);
-    const Pre<P> py = pre_of<P, MASK, 1, STRICT>(g, ly, xc, idy);
-    const Pre<P> pz = pre_of<P, MASK, 2, STRICT>(g, lz, xc, idz);
-    upd<P, MASK, 0, STRICT, DISP>(g, lx, xc, hz_a - hz_b, hy_a - hy_b, ex, idx, px);
-    upd<P, MASK, 1, STRICT, DISP>(g, ly, xc, hx_a - hx_b, hz_a - hz_c, ey, idy, py);
-    upd<P, MASK, 2, STRICT, DISP>(g, lz, xc, hy_a - hy_c, hx_a - hx_c, ez, idz, pz);
+    const R hz_a = ldf<P, 0, 5>(g, hz + s51);          // Hz[i+1, j+1, k]
+    const R hz_b = ldf<P, 0, 5>(g, hz);                // Hz[i+1, j,   k]
+    const R hz_c = ldf<P, 0, 5>(g, hz + s51 - s50);    // Hz[i,   j+1, k]
+    const R hy_a = ldf<P, 0, 4>(g, hy + 1);            // Hy[i+1, j, k+1]
+    const R hy_b = ldf<P, 0, 4>(g, hy);                // Hy[i+1, j, k]
+    const R hy_c = ldf<P, 0, 4>(g, hy + 1 - s40);      // Hy[i,   j, k+1]
+    const R hx_a = ldf<P, 0, 3>(g, hx + s31 + 1);      // Hx[i, j+1, k+1]
+    const R hx_b = ldf<P, 0, 3>(g, hx + s31);          // Hx[i, j+1, k]
+    const R hx_c = ldf<P, 0, 3>(g, hx + 1);            // Hx[i, j,   k+1]
+    const Pre<P> px = pre_of<P, 0, STRICT>(g, lx, xc, idx);
+    const Pre<P> py = pre_of<P, 1, STRICT>(g, ly, xc, idy);
+    const Pre<P> pz = pre_of<P, 2, STRICT>(g, lz, xc, idz);
+    upd<P, 0, STRICT, DISP>(g, lx, xc, hz_a - hz_b, hy_a - hy_b, ex, idx, px);
+    upd<P, 1, STRICT, DISP>(g, ly, xc, hx_a - hx_b, hz_a - hz_c, ey, idy, py);
+    upd<P, 2, STRICT, DISP>(g, lz, xc, hy_a - hy_c, hx_a - hx_c, ez, idz, pz);
   } else {
     // own points: Hx[i, j+1, k+1], Hy[i+1, j, k+1], Hz[i+1, j+1, k]
     const I lx = ii * s30 + (jj + 1) * s31 + kk + 1;
     const I ly = (ii + 1) * s40 + jj * s41 + kk + 1;
     const I lz = (ii + 1) * s50 + (jj + 1) * s51 + kk;
-    const uint8_t idx = ldc<MASK, 3>(g, lx), idy = ldc<MASK, 4>(g, ly), idz = ldc<MASK, 5>(g, lz);
-    const R hx = ldf<P, MASK, 3>(g, lx), hy = ldf<P, MASK, 4>(g, ly), hz = ldf<P, MASK, 5>(g, lz);
+    const uint8_t idx = ldc<0, 3>(g, lx), idy = ldc<0, 4>(g, ly), idz = ldc<0, 5>(g, lz);
+    const R hx = ldf<P, 0, 3>(g, lx), hy = ldf<P, 0, 4>(g, ly), hz = ldf<P, 0, 5>(g, lz);
     const I ex = ii * s00 + jj * s01 + kk;
     const I ey = ii * s10 + jj * s11 + kk;
     const I ez = ii * s20 + jj * s21 + kk;
-    const R ez_0 = ldf<P, MASK, 2>(g, ez);           // Ez[i, j, k]
-    const R ez_j = ldf<P, MASK, 2>(g, ez + s21);     // Ez[i, j+1, k]
-    const R ez_i = ldf<P, MASK, 2>(g, ez + s20);     // Ez[i+1, j, k]
-    const R ey_0 = ldf<P, MASK, 1>(g, ey);           // Ey[i, j, k]
-    const R ey_k = ldf<P, MASK, 1>(g, ey + 1);       // Ey[i, j, k+1]
-    const R ey_i = ldf<P, MASK, 1>(g, ey + s10);     // Ey[i+1, j, k]
-    const R ex_0 = ldf<P, MASK, 0>(g, ex);           // Ex[i, j, k]
-    const R ex_k = ldf<P, MASK, 0>(g, ex + 1);       // Ex[i, j, k+1]
-    const R ex_j = ldf<P, MASK, 0>(g, ex + s01);     // Ex[i, j+1, k]
+    const R ez_0 = ldf<P, 0, 2>(g, ez);           // Ez[i, j, k]
+    const R ez_j = ldf<P, 0, 2>(g, ez + s21);     // Ez[i, j+1, k]
+    const R ez_i = ldf<P, 0, 2>(g, ez + s20);     // Ez[i+1, j, k]
+    const R ey_0 = ldf<P, 0, 1>(g, ey);           // Ey[i, j, k]
+    const R ey_k = ldf<P, 0, 1>(g, ey + 1);       // Ey[i, j, k+1]
+    const R ey_i = ldf<P, 0, 1>(g, ey + s10);     // Ey[i+1, j, k]
+    const R ex_0 = ldf<P, 0, 0>(g, ex);           // Ex[i, j, k]
+    const R ex_k = ldf<P, 0, 0>(g, ex + 1);       // Ex[i, j, k+1]
+    const R ex_j = ldf<P, 0, 0>(g, ex + s01);     // Ex[i, j+1, k]
     const int x3[3] = {i, j + 1, k + 1}, x4[3] = {i + 1, j, k + 1}, x5[3] = {i + 1, j + 1, k};
-    const Pre<P> px = pre_of<P, MASK, 3, STRICT>(g, lx, x3, idx);
-    const Pre<P> py = pre_of<P, MASK, 4, STRICT>(g, ly, x4, idy);
-    const Pre<P> pz = pre_of<P, MASK, 5, STRICT>(g, lz, x5, idz);
-    upd<P, MASK, 3, STRICT, DISP>(g, lx, x3, ez_j - ez_0, ey_k - ey_0, hx, idx, px);
-    upd<P, MASK, 4, STRICT, DISP>(g, ly, x4, ex_k - ex_0, ez_i - ez_0, hy, idy, py);
-    upd<P, MASK, 5, STRICT, DISP>(g, lz, x5, ey_i - ey_0, ex_j - ex_0, hz, idz, pz);
+    const Pre<P> px = pre_of<P, 3, STRICT>(g, lx, x3, idx);
+    const Pre<P> py = pre_of<P, 4, STRICT>(g, ly, x4, idy);
+    const Pre<P> pz = pre_of<P, 5, STRICT>(g, lz, x5, idz);
+    upd<P, 3, STRICT, DISP>(g, lx, x3, ez_j - ez_0, ey_k - ey_0, hx, idx, px);
+    upd<P, 4, STRICT, DISP>(g, ly, x4, ex_k - ex_0, ez_i - ez_0, hy, idy, py);
+    upd<P, 5, STRICT, DISP>(g, lz, x5, ey_i - ey_0, ex_j - ex_0, hz, idz, pz);
   }
 }
 
@@ -788,7 +787,7 @@ struct EarlyCoef {
 // 42.54 -> 30.1 / 29.7 / 34.3 / 31.1 Gcell/s at 6 / 7 / 8 / 10 blocks per SM
 // (64 registers at 8), dispersive FP32 25.42 -> 22.35; df64 (5, 6 blocks)
 // 26.74 -> 17.5 / 20.7, FP64 (6 blocks) 19.25 -> 16.99.
-template <class P, int SIDE, bool DISP, int MASK, class I>
+template <class P, int SIDE, bool DISP, class I>
 __device__ __forceinline__ void cell_body_fast(const GridDev& g, int i, int j, int k) {
   using R = typename P::R;
   using T = typename P::T;
@@ -804,38 +803,38 @@ __device__ __forceinline__ void cell_body_fast(const GridDev& g, int i, int j, i
   const I l0 = SIDE == 0 ? oX : oX + X1 + 1;
   const I l1 = SIDE == 0 ? oY : oY + Y0 + 1;
   const I l2 = SIDE == 0 ? oZ : oZ + Z0 + Z1;
-  const R f0 = ldf<P, MASK, c0>(g, l0), f1 = ldf<P, MASK, c0 + 1>(g, l1),
-          f2 = ldf<P, MASK, c0 + 2>(g, l2);
+  const R f0 = ldf<P, 0, c0>(g, l0), f1 = ldf<P, 0, c0 + 1>(g, l1),
+          f2 = ldf<P, 0, c0 + 2>(g, l2);
   R d01, d02, d11, d12, d21, d22;  // (D1, D2) of each component
   if constexpr (SIDE == 0) {
-    const R hz_a = ldf<P, MASK, 5>(g, oZ + Z0 + Z1);  // Hz[i+1, j+1, k]
-    const R hz_b = ldf<P, MASK, 5>(g, oZ + Z0);       // Hz[i+1, j,   k]
-    const R hz_c = ldf<P, MASK, 5>(g, oZ + Z1);       // Hz[i,   j+1, k]
-    const R hy_a = ldf<P, MASK, 4>(g, oY + Y0 + 1);   // Hy[i+1, j, k+1]
-    const R hy_b = ldf<P, MASK, 4>(g, oY + Y0);       // Hy[i+1, j, k]
-    const R hy_c = ldf<P, MASK, 4>(g, oY + 1);        // Hy[i,   j, k+1]
-    const R hx_a = ldf<P, MASK, 3>(g, oX + X1 + 1);   // Hx[i, j+1, k+1]
-    const R hx_b = ldf<P, MASK, 3>(g, oX + X1);       // Hx[i, j+1, k]
-    const R hx_c = ldf<P, MASK, 3>(g, oX + 1);        // Hx[i, j,   k+1]
+    const R hz_a = ldf<P, 0, 5>(g, oZ + Z0 + Z1);  // Hz[i+1, j+1, k]
+    const R hz_b = ldf<P, 0, 5>(g, oZ + Z0);       // Hz[i+1, j,   k]
+    const R hz_c = ldf<P, 0, 5>(g, oZ + Z1);       // Hz[i,   j+1, k]
+    const R hy_a = ldf<P, 0, 4>(g, oY + Y0 + 1);   // Hy[i+1, j, k+1]
+    const R hy_b = ldf<P, 0, 4>(g, oY + Y0);       // Hy[i+1, j, k]
+    const R hy_c = ldf<P, 0, 4>(g, oY + 1);        // Hy[i,   j, k+1]
+    const R hx_a = ldf<P, 0, 3>(g, oX + X1 + 1);   // Hx[i, j+1, k+1]
+    const R hx_b = ldf<P, 0, 3>(g, oX + X1);       // Hx[i, j+1, k]
+    const R hx_c = ldf<P, 0, 3>(g, oX + 1);        // Hx[i, j,   k+1]
     d01 = curl_diff(hz_a, hz_b); d02 = curl_diff(hy_a, hy_b);
     d11 = curl_diff(hx_a, hx_b); d12 = curl_diff(hz_a, hz_c);
     d21 = curl_diff(hy_a, hy_c); d22 = curl_diff(hx_a, hx_c);
   } else {
-    const R ez_0 = ldf<P, MASK, 2>(g, oZ);       // Ez[i, j, k]
-    const R ez_j = ldf<P, MASK, 2>(g, oZ + Z1);  // Ez[i, j+1, k]
-    const R ez_i = ldf<P, MASK, 2>(g, oZ + Z0);  // Ez[i+1, j, k]
-    const R ey_0 = ldf<P, MASK, 1>(g, oY);       // Ey[i, j, k]
-    const R ey_k = ldf<P, MASK, 1>(g, oY + 1);   // Ey[i, j, k+1]
-    const R ey_i = ldf<P, MASK, 1>(g, oY + Y0);  // Ey[i+1, j, k]
-    const R ex_0 = ldf<P, MASK, 0>(g, oX);       // Ex[i, j, k]
-    const R ex_k = ldf<P, MASK, 0>(g, oX + 1);   // Ex[i, j, k+1]
-    const R ex_j = ldf<P, MASK, 0>(g, oX + X1);  // Ex[i, j+1, k]
+    const R ez_0 = ldf<P, 0, 2>(g, oZ);       // Ez[i, j, k]
+    const R ez_j = ldf<P, 0, 2>(g, oZ + Z1);  // Ez[i, j+1, k]
+    const R ez_i = ldf<P, 0, 2>(g, oZ + Z0);  // Ez[i+1, j, k]
+    const R ey_0 = ldf<P, 0, 1>(g, oY);       // Ey[i, j, k]
+    const R ey_k = ldf<P, 0, 1>(g, oY + 1);   // Ey[i, j, k+1]
+    const R ey_i = ldf<P, 0, 1>(g, oY + Y0);  // Ey[i+1, j, k]
+    const R ex_0 = ldf<P, 0, 0>(g, oX);       // Ex[i, j, k]
+    const R ex_k = ldf<P, 0, 0>(g, oX + 1);   // Ex[i, j, k+1]
+    const R ex_j = ldf<P, 0, 0>(g, oX + X1);  // Ex[i, j+1, k]
     d01 = curl_diff(ez_j, ez_0); d02 = curl_diff(ey_k, ey_0);
     d11 = curl_diff(ex_k, ex_0); d12 = curl_diff(ez_i, ez_0);
     d21 = curl_diff(ey_i, ey_0); d22 = curl_diff(ex_j, ex_0);
   }
-  const uint8_t id0 = ldc<MASK, c0>(g, l0), id1 = ldc<MASK, c0 + 1>(g, l1),
-                id2 = ldc<MASK, c0 + 2>(g, l2);
+  const uint8_t id0 = ldc<0, c0>(g, l0), id1 = ldc<0, c0 + 1>(g, l1),
+                id2 = ldc<0, c0 + 2>(g, l2);
   const uint32_t t = (uint32_t)id0 | (uint32_t)id1 << 8 | (uint32_t)id2 << 16;
   int same = 0;
   __match_all_sync(__activemask(), t, &same);
@@ -850,17 +849,17 @@ __device__ __forceinline__ void cell_body_fast(const GridDev& g, int i, int j, i
     cc2 = P::zero();
   if constexpr (UniformCpml<P, SIDE>::value) {
     if (uniform) {
-      if (is_active<MASK, c0>(g)) {
+      if (is_active<0, c0>(g)) {
         const ClassCoef& q = g.tab[c0][id0];
         ka = q.kind;
         if (EarlyCoef<P>::value) ca1 = P::cfg(&q.c1), ca2 = P::cfg(&q.c2);
       }
-      if (is_active<MASK, c0 + 1>(g)) {
+      if (is_active<0, c0 + 1>(g)) {
         const ClassCoef& q = g.tab[c0 + 1][id1];
         kb = q.kind;
         if (EarlyCoef<P>::value) cb1 = P::cfg(&q.c1), cb2 = P::cfg(&q.c2);
       }
-      if (is_active<MASK, c0 + 2>(g)) {
+      if (is_active<0, c0 + 2>(g)) {
         const ClassCoef& q = g.tab[c0 + 2][id2];
         kc = q.kind;
         if (EarlyCoef<P>::value) cc1 = P::cfg(&q.c1), cc2 = P::cfg(&q.c2);
@@ -870,9 +869,9 @@ __device__ __forceinline__ void cell_body_fast(const GridDev& g, int i, int j, i
            kc == GMES_KIND_DIELECTRIC;
   } else {
     fast = uniform &&
-           (!is_active<MASK, c0>(g) || g.tab[c0][id0].kind == GMES_KIND_DIELECTRIC) &&
-           (!is_active<MASK, c0 + 1>(g) || g.tab[c0 + 1][id1].kind == GMES_KIND_DIELECTRIC) &&
-           (!is_active<MASK, c0 + 2>(g) || g.tab[c0 + 2][id2].kind == GMES_KIND_DIELECTRIC);
+           (!is_active<0, c0>(g) || g.tab[c0][id0].kind == GMES_KIND_DIELECTRIC) &&
+           (!is_active<0, c0 + 1>(g) || g.tab[c0 + 1][id1].kind == GMES_KIND_DIELECTRIC) &&
+           (!is_active<0, c0 + 2>(g) || g.tab[c0 + 2][id2].kind == GMES_KIND_DIELECTRIC);
   }
   constexpr bool E = SIDE == 0;
   if (fast) {  // warp-uniform
@@ -880,23 +879,23 @@ __device__ __forceinline__ void cell_body_fast(const GridDev& g, int i, int j, i
     const ClassCoef& qb = g.tab[c0 + 1][id1];
     const ClassCoef& qc = g.tab[c0 + 2][id2];
     if (UniformCpml<P, SIDE>::value && EarlyCoef<P>::value) {
-      if (is_active<MASK, c0>(g))
-        P::st(static_cast<T*>(g.f[c0]) + l0, plain_mask<MASK, c0>(f0, ca1, ca2, d01, d02));
-      if (is_active<MASK, c0 + 1>(g))
-        P::st(static_cast<T*>(g.f[c0 + 1]) + l1, plain_mask<MASK, c0 + 1>(f1, cb1, cb2, d11, d12));
-      if (is_active<MASK, c0 + 2>(g))
-        P::st(static_cast<T*>(g.f[c0 + 2]) + l2, plain_mask<MASK, c0 + 2>(f2, cc1, cc2, d21, d22));
+      if (is_active<0, c0>(g))
+        P::st(static_cast<T*>(g.f[c0]) + l0, plain_upd<E>(f0, ca1, ca2, d01, d02));
+      if (is_active<0, c0 + 1>(g))
+        P::st(static_cast<T*>(g.f[c0 + 1]) + l1, plain_upd<E>(f1, cb1, cb2, d11, d12));
+      if (is_active<0, c0 + 2>(g))
+        P::st(static_cast<T*>(g.f[c0 + 2]) + l2, plain_upd<E>(f2, cc1, cc2, d21, d22));
       return;
     }
-    if (is_active<MASK, c0>(g))
+    if (is_active<0, c0>(g))
       P::st(static_cast<T*>(g.f[c0]) + l0,
-            plain_mask<MASK, c0>(f0, P::cfg(&qa.c1), P::cfg(&qa.c2), d01, d02));
-    if (is_active<MASK, c0 + 1>(g))
+            plain_upd<E>(f0, P::cfg(&qa.c1), P::cfg(&qa.c2), d01, d02));
+    if (is_active<0, c0 + 1>(g))
       P::st(static_cast<T*>(g.f[c0 + 1]) + l1,
-            plain_mask<MASK, c0 + 1>(f1, P::cfg(&qb.c1), P::cfg(&qb.c2), d11, d12));
-    if (is_active<MASK, c0 + 2>(g))
+            plain_upd<E>(f1, P::cfg(&qb.c1), P::cfg(&qb.c2), d11, d12));
+    if (is_active<0, c0 + 2>(g))
       P::st(static_cast<T*>(g.f[c0 + 2]) + l2,
-            plain_mask<MASK, c0 + 2>(f2, P::cfg(&qc.c1), P::cfg(&qc.c2), d21, d22));
+            plain_upd<E>(f2, P::cfg(&qc.c1), P::cfg(&qc.c2), d21, d22));
     return;
   }
   if constexpr (UniformCpml<P, SIDE>::value) {
@@ -919,17 +918,17 @@ __device__ __forceinline__ void cell_body_fast(const GridDev& g, int i, int j, i
       const ClassCoef& qc = g.tab[c0 + 2][id2];
       if (ka == GMES_KIND_CPML)
         cpml_separate<P, c0>(g, l0, xa, d01, d02, f0, qa, pa);
-      else if (is_active<MASK, c0>(g))
+      else if (is_active<0, c0>(g))
         P::st(static_cast<T*>(g.f[c0]) + l0,
               plain_upd<E>(f0, P::cfg(&qa.c1), P::cfg(&qa.c2), d01, d02));
       if (kb == GMES_KIND_CPML)
         cpml_separate<P, c0 + 1>(g, l1, xb, d11, d12, f1, qb, pb);
-      else if (is_active<MASK, c0 + 1>(g))
+      else if (is_active<0, c0 + 1>(g))
         P::st(static_cast<T*>(g.f[c0 + 1]) + l1,
               plain_upd<E>(f1, P::cfg(&qb.c1), P::cfg(&qb.c2), d11, d12));
       if (kc == GMES_KIND_CPML)
         cpml_separate<P, c0 + 2>(g, l2, xq, d21, d22, f2, qc, pc);
-      else if (is_active<MASK, c0 + 2>(g))
+      else if (is_active<0, c0 + 2>(g))
         P::st(static_cast<T*>(g.f[c0 + 2]) + l2,
               plain_upd<E>(f2, P::cfg(&qc.c1), P::cfg(&qc.c2), d21, d22));
       return;
@@ -937,20 +936,20 @@ __device__ __forceinline__ void cell_body_fast(const GridDev& g, int i, int j, i
   }
   if constexpr (SIDE == 0) {
     const int xc[3] = {i, j, k};
-    const Pre<P> pa = pre_of<P, MASK, 0, false>(g, l0, xc, id0);
-    const Pre<P> pb = pre_of<P, MASK, 1, false>(g, l1, xc, id1);
-    const Pre<P> pc = pre_of<P, MASK, 2, false>(g, l2, xc, id2);
-    upd<P, MASK, 0, false, DISP>(g, l0, xc, d01, d02, f0, id0, pa);
-    upd<P, MASK, 1, false, DISP>(g, l1, xc, d11, d12, f1, id1, pb);
-    upd<P, MASK, 2, false, DISP>(g, l2, xc, d21, d22, f2, id2, pc);
+    const Pre<P> pa = pre_of<P, 0, false>(g, l0, xc, id0);
+    const Pre<P> pb = pre_of<P, 1, false>(g, l1, xc, id1);
+    const Pre<P> pc = pre_of<P, 2, false>(g, l2, xc, id2);
+    upd<P, 0, false, DISP>(g, l0, xc, d01, d02, f0, id0, pa);
+    upd<P, 1, false, DISP>(g, l1, xc, d11, d12, f1, id1, pb);
+    upd<P, 2, false, DISP>(g, l2, xc, d21, d22, f2, id2, pc);
   } else {
     const int x3[3] = {i, j + 1, k + 1}, x4[3] = {i + 1, j, k + 1}, x5[3] = {i + 1, j + 1, k};
-    const Pre<P> pa = pre_of<P, MASK, 3, false>(g, l0, x3, id0);
-    const Pre<P> pb = pre_of<P, MASK, 4, false>(g, l1, x4, id1);
-    const Pre<P> pc = pre_of<P, MASK, 5, false>(g, l2, x5, id2);
-    upd<P, MASK, 3, false, false>(g, l0, x3, d01, d02, f0, id0, pa);
-    upd<P, MASK, 4, false, false>(g, l1, x4, d11, d12, f1, id1, pb);
-    upd<P, MASK, 5, false, false>(g, l2, x5, d21, d22, f2, id2, pc);
+    const Pre<P> pa = pre_of<P, 3, false>(g, l0, x3, id0);
+    const Pre<P> pb = pre_of<P, 4, false>(g, l1, x4, id1);
+    const Pre<P> pc = pre_of<P, 5, false>(g, l2, x5, id2);
+    upd<P, 3, false, false>(g, l0, x3, d01, d02, f0, id0, pa);
+    upd<P, 4, false, false>(g, l1, x4, d11, d12, f1, id1, pb);
+    upd<P, 5, false, false>(g, l2, x5, d21, d22, f2, id2, pc);
   }
 }
 

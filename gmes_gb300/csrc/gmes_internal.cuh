@@ -494,7 +494,7 @@ template <class R>
 struct TbTile {
   uint32_t any;
   int32_t kind, pm, fancy;
-  R c[4], d[3], e;
+  R c[4], d[3];
 };
 
 // Flags of the resolved lattice map.  "Plain": the update is

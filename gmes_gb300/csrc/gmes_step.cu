@@ -184,7 +184,7 @@ struct ArgDescs<PolDF> {
   static constexpr bool value = GMES_MULTI_ARG_DF != 0;
 };
 
-template <class P, int SIDE, bool STRICT, bool DISP, int MASK, class I>
+template <class P, int SIDE, bool STRICT, bool DISP, class I>
 __global__ void __launch_bounds__(kCellThreads, CellMinBlocks<P, SIDE, DISP>::value)
     k_cell(const GridDev g, int bx_log2, int i0) {
   after_launch();
@@ -196,9 +196,9 @@ __global__ void __launch_bounds__(kCellThreads, CellMinBlocks<P, SIDE, DISP>::va
   const int i = i0 + (int)blockIdx.z;
   if (k >= g.n[2] || j >= g.n[1] || i >= g.n[0]) return;
   if constexpr (STRICT)
-    cell_body<P, SIDE, STRICT, DISP, MASK, I>(g, i, j, k);
+    cell_body<P, SIDE, STRICT, DISP, I>(g, i, j, k);
   else
-    cell_body_fast<P, SIDE, DISP, MASK, I>(g, i, j, k);
+    cell_body_fast<P, SIDE, DISP, I>(g, i, j, k);
 }
 
 // Cells per block row along k (log2): a warp covers 16 cells of two rows
@@ -217,17 +217,17 @@ __global__ void __launch_bounds__(kCellThreads, CellMinBlocks<P, SIDE, DISP>::va
 // what a warp-level count of the slabs predicts for both shapes.)  The row
 // length is kRowLog2 (cell_tiling).
 
-template <class P, bool STRICT, int MASK, class I>
+template <class P, bool STRICT, class I>
 void launch_cell(const GridDev& d, int side, bool disp, dim3 grid, int bx_log2, int i0,
                  cudaStream_t s) {
   auto go = [&](auto kernel) { launch_after(true, kernel, grid, kCellThreads, 0, s, d, bx_log2, i0); };
   if (side == 0) {
     if (disp)
-      go(k_cell<P, 0, STRICT, true, MASK, I>);
+      go(k_cell<P, 0, STRICT, true, I>);
     else
-      go(k_cell<P, 0, STRICT, false, MASK, I>);
+      go(k_cell<P, 0, STRICT, false, I>);
   } else {
-    go(k_cell<P, 1, STRICT, false, MASK, I>);
+    go(k_cell<P, 1, STRICT, false, I>);
   }
 }
 
@@ -509,9 +509,9 @@ __global__ void __launch_bounds__(kBatchThreads, MultiMinBlocks<P, SIDE, DISP>::
     // the batch is prepared)
     if (k < g.n[2] && j < g.n[1]) {
       if constexpr (STRICT)
-        cell_body<P, SIDE, STRICT, DISP, 0, int32_t>(g, i, j, k);
+        cell_body<P, SIDE, STRICT, DISP, int32_t>(g, i, j, k);
       else
-        cell_body_fast<P, SIDE, DISP, 0, int32_t>(g, i, j, k);
+        cell_body_fast<P, SIDE, DISP, int32_t>(g, i, j, k);
     }
   }
 }
@@ -542,9 +542,9 @@ __global__ void __launch_bounds__(kBatchThreads, MultiMinBlocks<P, SIDE, DISP>::
     const int j = jb * by + (threadIdx.x >> bxl);
     if (k < g.n[2] && j < g.n[1]) {
       if constexpr (STRICT)
-        cell_body<P, SIDE, STRICT, DISP, 0, int32_t>(g, i, j, k);
+        cell_body<P, SIDE, STRICT, DISP, int32_t>(g, i, j, k);
       else
-        cell_body_fast<P, SIDE, DISP, 0, int32_t>(g, i, j, k);
+        cell_body_fast<P, SIDE, DISP, int32_t>(g, i, j, k);
     }
   }
 }
@@ -616,9 +616,9 @@ template <class P, bool STRICT>
       // takes them; a compile-time active mask (all six components) ran ~35%
       // slower, so the mask stays a runtime value.
       if (offsets_fit_i32(d))
-        launch_cell<P, STRICT, 0, int32_t>(v, side, p.disp, grid, bx_log2, i0, s);
+        launch_cell<P, STRICT, int32_t>(v, side, p.disp, grid, bx_log2, i0, s);
       else
-        launch_cell<P, STRICT, 0, int64_t>(v, side, p.disp, grid, bx_log2, i0, s);
+        launch_cell<P, STRICT, int64_t>(v, side, p.disp, grid, bx_log2, i0, s);
     }
   }
   for (int part = 0; part < nplanes; ++part) {

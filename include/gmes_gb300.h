@@ -509,7 +509,10 @@ typedef struct {
   int32_t design_n[2];   /* design box extent */
   int32_t monitor_lo[2];
   int32_t monitor_n[2];
-  int32_t nsrc;          /* point sources: comp 2 (Ez), 3 (Hx), 4 (Hy); offset = i * ny + j */
+  int32_t nsrc;          /* point sources: comp 2 (Ez), 3 (Hx), 4 (Hy); offset = i * ny + j,
+                            one entry at most per component and point.  The blocked kernels
+                            find the tiles with sources at gmes_tmz_set_design: set the design
+                            again after sources have moved (their values may change freely). */
   int32_t total_steps;   /* rows of monitor and src_val */
   int32_t hist_steps;    /* capacity of hist in steps (one checkpoint segment) */
   int32_t block_steps;   /* FP32: steps per launch, 0 = GMES_TMZ_MAX_BLOCK_STEPS (temporally
