@@ -104,11 +104,11 @@ def test_long_lists_cost_about_what_short_ones_do(name, n):
     else:
         rows = [(c, 1, 60 * ny + q) for c in (2, 4) for q in range(n // 2)]
     eps = np.ones((1, 9, 8))
-    took = {}
-    for k in (13, n):
-        prob = _problem(nx, ny, 1, rows[:k], vals[:, :, :k], "fp64", steps, keep_history=True)
-        best = []
-        for _ in range(6):
+    probs = {k: _problem(nx, ny, 1, rows[:k], vals[:, :, :k], "fp64", steps, keep_history=True)
+             for k in (13, n)}
+    took = {k: [] for k in probs}
+    for _ in range(6):
+        for k, prob in probs.items():
             ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
             prob.forward(eps)
             ev[0].record()
@@ -116,6 +116,5 @@ def test_long_lists_cost_about_what_short_ones_do(name, n):
             prob.backward()
             ev[1].record()
             torch.cuda.synchronize()
-            best.append(ev[0].elapsed_time(ev[1]))
-        took[k] = min(best)
-    assert took[n] < 3 * took[13], took
+            took[k].append(ev[0].elapsed_time(ev[1]))
+    assert min(took[n]) < 3 * min(took[13]), took

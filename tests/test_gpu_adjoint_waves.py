@@ -41,12 +41,11 @@ def test_designs_do_not_depend_on_the_batch(batch):
 
 def test_one_wave_takes_its_slowest_tile():
     import torch
-    took = {}
-    for batch in (4, 12):
-        prob = _problem(100, 100, batch)
-        eps = np.ones((batch, 30, 30))
-        best = []
-        for _ in range(12):
+    probs = {b: _problem(100, 100, b) for b in (4, 12)}
+    took = {b: [] for b in probs}
+    for _ in range(16):  # in turn: the clocks are the same for both
+        for batch, prob in probs.items():
+            eps = np.ones((batch, 30, 30))
             ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
             prob.forward(eps)
             ev[0].record()
@@ -54,6 +53,5 @@ def test_one_wave_takes_its_slowest_tile():
             prob.backward()
             ev[1].record()
             torch.cuda.synchronize()
-            best.append(ev[0].elapsed_time(ev[1]))
-        took[batch] = sorted(best)[3]
-    assert took[12] < 1.1 * took[4], took
+            took[batch].append(ev[0].elapsed_time(ev[1]))
+    assert min(took[12]) < 1.1 * min(took[4]), took
