@@ -812,6 +812,8 @@ gmes_status gmes_batch_step(const gmes_batch* b, int32_t nsteps, int32_t blocks,
   if (nsteps < 0 || blocks < 0) return fail(GMES_ERR_VALUE, "negative nsteps or blocks");
   if (b->njobs < 1) return fail(GMES_ERR_VALUE, "empty batch");
   if (nsteps == 0) return GMES_OK;
+  const gmes_status st = check_wait_error();
+  if (st != GMES_OK) return st;
   const std::vector<GridDev> host =
       b->njobs <= kParamJobs ? recall_batch(b->workspace, b->njobs) : std::vector<GridDev>();
   cudaError_t e = launch_batch(batch_view(*b), host.empty() ? nullptr : host.data(),
@@ -1219,6 +1221,8 @@ gmes_status gmes_tmz_objective(const gmes_grid_desc* g, const gmes_tmz_batch* b,
   if (J == nullptr) return fail(GMES_ERR_VALUE, "J is NULL");
   if (nsteps < 0 || nsteps > b->total_steps)
     return fail(GMES_ERR_INDEX, "nsteps = %d outside [0, %d]", nsteps, b->total_steps);
+  st = check_wait_error();
+  if (st != GMES_OK) return st;
   cudaError_t e = launch_tmz_objective(make_grid_dev(*g), make_tmz_dev(*g, *b), nsteps, J,
                                        static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "launching the objective kernel");
@@ -1350,6 +1354,8 @@ extern "C" gmes_status gmes_batch_step_noalloc(const gmes_grid_desc* const* grid
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
   if (dev < 0 || dev >= kMaxDevices) return fail(GMES_ERR_RUNTIME, "device %d unsupported", dev);
+  const gmes_status waits = check_wait_error();
+  if (waits != GMES_OK) return waits;
   std::lock_guard<std::mutex> lock(g_noalloc_mutex);
   if (g_noalloc_addr[dev] == nullptr) {
     void* addr = nullptr;

@@ -89,6 +89,32 @@ def test_step_after_a_wait_that_ran_out():
         assert np.isfinite(want.read(c)).all()
 
 
+def test_batches_after_a_wait_that_ran_out():
+    import torch
+
+    from gmes_gb300.batch import Batch
+    grids = [_start(_scene(G.FDTD, (1.9, 1.7, 1.6), 10, "fp64")) for _ in range(3)]
+    alone = grids.pop()
+    batch = Batch(grids, use_graphs=False)
+    batch.run([2, 2], [0.0, 0.0])
+    batch.synchronize()
+    s = torch.cuda.Stream()
+    _check(s.cuda_stream, 0)
+    s.synchronize()
+    with pytest.raises(RuntimeError, match="gave up"):
+        batch.run([2, 2], [2.0, 2.0])
+    with pytest.raises(RuntimeError, match="gave up"):
+        batch.synchronize()
+    N.clear_waits()
+    batch.run([2, 2], [2.0, 2.0])
+    batch.synchronize()
+    alone.step(2)
+    alone.step(2, n0=2.0)
+    for e in grids:  # untouched by the other launch
+        for c in range(6):
+            assert np.array_equal(e.read(c), alone.read(c))
+
+
 @pytest.mark.parametrize("segment", [None, 8])
 def test_differentiation_after_a_wait_that_ran_out(segment):
     from gmes_gb300.adjoint import TMzAdjoint
